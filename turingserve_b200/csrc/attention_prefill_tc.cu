@@ -26,9 +26,6 @@
 // then, O is rescaled in tensor memory, after the product before it has finished.  Two blocks
 // share an SM.  Every barrier wait is bounded; a block that gives up records where, stops, and
 // frees its tensor memory.
-#include <utility>
-#include <vector>
-
 #include "common.cuh"
 #include "tc_utils.cuh"
 
@@ -65,18 +62,6 @@ constexpr float LOG2E_F = 1.4426950408889634f;
 
 __device__ int g_attn_status = 0;   // 0 = fine; otherwise the wait that ran out
 
-// Shared-memory descriptor for an MN-major operand ([k rows][64 elements = 128 B], 128-byte swizzle):
-// 8-row groups along K are 1024 B apart (SBO), the next 64 elements along MN are `lbo` bytes away.
-__device__ __forceinline__ uint64_t smem_desc_mn(uint32_t addr, uint32_t lbo) {
-  uint64_t d = 0;
-  d |= (uint64_t)((addr & 0x3FFFF) >> 4);
-  d |= (uint64_t)(lbo >> 4) << 16;
-  d |= (uint64_t)(1024 >> 4) << 32;
-  d |= (uint64_t)1 << 46;
-  d |= (uint64_t)2 << 61;
-  return d;
-}
-
 struct AttnArgs {
   bf16* out;
   const bf16* qkv;
@@ -90,44 +75,11 @@ struct AttnArgs {
   int* status;
 };
 
-// D[tmem] (+)= A[tmem] . B[smem]: the A operand (here P) is read from tensor memory.
-__device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
-      ::"r"(tmem_d), "r"(tmem_a), "l"(b), "r"(idesc), "r"(accumulate) : "memory");
-}
-
-// A 4-D box (64 columns, a page's rows, one kv head, `run` pages that follow one another in the pool).
-__device__ __forceinline__ void tma_load_run(void* dst, const CUtensorMap* map, int x, int kvh, int page0, uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
-      ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(0), "r"(kvh), "r"(page0) : "memory");
-}
-
-// 2^x by the special-function unit alone (2 ulp; the results are rounded to bfloat16), 0 for -inf.
-__device__ __forceinline__ float ex2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-
 // warps 0-7: two threads per query row; warp 8: product issue; warp 9: TMA loads of keys; warp 10: of values
 // (one thread each: with pages shorter than a tile in a shuffled pool a tile is up to 16 copies of keys and
 // 16 of values at about 100 cycles of issue each, more than one thread gets through in a tile's time)
 constexpr int ATT_THREADS = 2 * TQ + 96;
 constexpr int MMA_WARP = 2 * TQ / 32, TMA_WARP = MMA_WARP + 1, TMA_V_WARP = MMA_WARP + 2;
-
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&v)[16]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
-      ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]),
-        "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]) : "memory");
-}
 
 template <int TK, int HD>
 __global__ void __launch_bounds__(ATT_THREADS, TK == 64 ? 2 : 1)
@@ -534,38 +486,6 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap k_map, const __g
   if (warp == MMA_WARP) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
   }
-}
-
-// The cache [pages, KVH, page, 128] as a 4-D tensor: boxes of 64 columns x a page's rows x one kv head x
-// `run` pages (128-byte swizzle, zeros outside).  Encoded once per (cache, shape).
-bool run_map(CUtensorMap* out, const void* cache, int num_pages, int KVH, int page, int run, int HD) {
-  struct Key {
-    const void* p;
-    int n, k, g, r;
-    bool operator==(const Key& o) const { return p == o.p && n == o.n && k == o.k && g == o.g && r == o.r; }
-  };
-  static std::vector<std::pair<Key, CUtensorMap>> cache_;
-  static std::mutex mu;
-  std::lock_guard<std::mutex> lock(mu);
-  const Key key{cache, num_pages, KVH, page, run + 1024 * HD};
-  for (auto& e : cache_)
-    if (e.first == key) {
-      *out = e.second;
-      return true;
-    }
-  EncodeTiledFn fn = encode_fn();
-  if (fn == nullptr) return false;
-  cuuint64_t dims[4] = {(cuuint64_t)HD, (cuuint64_t)page, (cuuint64_t)KVH, (cuuint64_t)num_pages};
-  cuuint64_t strides[3] = {(cuuint64_t)HD * 2, (cuuint64_t)page * HD * 2, (cuuint64_t)KVH * page * HD * 2};
-  cuuint32_t box[4] = {64, (cuuint32_t)page, 1, (cuuint32_t)run};
-  cuuint32_t estr[4] = {1, 1, 1, 1};
-  if (fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(cache), dims, strides, box, estr,
-         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-    return false;
-  if (cache_.size() > 1024) cache_.clear();
-  cache_.emplace_back(key, *out);
-  return true;
 }
 
 int* attn_status_word() {

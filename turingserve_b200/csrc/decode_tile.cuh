@@ -36,10 +36,6 @@ __device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, i
       ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(c3) : "memory");
 }
 
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-
 // Query fragments of a group: rows 0..G-1, zero above.
 template <int D>
 __device__ __forceinline__ void load_q_fragments(unsigned (&qf)[D / 16][4], const bf16* qbase, int G, int lane) {

@@ -7,6 +7,8 @@
 
 #include <mutex>
 #include <unordered_map>
+#include <utility>
+#include <vector>
 
 #include "common.cuh"
 
@@ -64,10 +66,21 @@ __device__ __forceinline__ bool mbar_wait_spin(uint64_t* bar, uint32_t parity, i
   return false;
 }
 
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
       ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(y) : "memory");
+}
+
+// A 4-D box (64 columns, a page's rows, one kv head, `run` pages that follow one another in the pool).
+__device__ __forceinline__ void tma_load_run(void* dst, const CUtensorMap* map, int x, int kvh, int page0, uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
+      ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(0), "r"(kvh), "r"(page0) : "memory");
 }
 
 // Shared-memory matrix descriptor: K-major tile of [rows][64] bf16 written by TMA with the 128-byte
@@ -79,6 +92,18 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
   d |= (uint64_t)(1024 >> 4) << 32;                  // stride byte offset between 8-row groups
   d |= (uint64_t)1 << 46;                            // descriptor version of this architecture
   d |= (uint64_t)2 << 61;                            // 128-byte swizzle
+  return d;
+}
+
+// Shared-memory descriptor for an MN-major operand ([k rows][64 elements = 128 B], 128-byte swizzle):
+// 8-row groups along K are 1024 B apart (SBO), the next 64 elements along MN are `lbo` bytes away.
+__device__ __forceinline__ uint64_t smem_desc_mn(uint32_t addr, uint32_t lbo) {
+  uint64_t d = 0;
+  d |= (uint64_t)((addr & 0x3FFFF) >> 4);
+  d |= (uint64_t)(lbo >> 4) << 16;
+  d |= (uint64_t)(1024 >> 4) << 32;
+  d |= (uint64_t)1 << 46;
+  d |= (uint64_t)2 << 61;
   return d;
 }
 
@@ -94,6 +119,14 @@ __device__ __forceinline__ void umma(uint32_t tmem_d, uint64_t a, uint64_t b, ui
       " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
       ::"r"(tmem_d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate) : "memory");
 }
+// D[tmem] (+)= A[tmem] . B[smem]: the A operand (here P) is read from tensor memory.
+__device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
+      ::"r"(tmem_d), "r"(tmem_a), "l"(b), "r"(idesc), "r"(accumulate) : "memory");
+}
+
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
@@ -125,6 +158,20 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&v)[32
         "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]),
         "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31]) : "memory");
 }
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&v)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+      ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]),
+        "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]) : "memory");
+}
+
+// 2^x by the special-function unit alone (2 ulp; the results are rounded to bfloat16), 0 for -inf.
+__device__ __forceinline__ float ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
@@ -188,5 +235,36 @@ inline bool tensor_map(CUtensorMap* out, const void* ptr, int rows, int K, int b
   return true;
 }
 
+// A cache [pages, KVH, page, HD] as a 4-D tensor: boxes of 64 columns x a page's rows x one kv head x
+// `run` pages (128-byte swizzle, zeros outside).  Encoded once per (cache, shape).
+inline bool run_map(CUtensorMap* out, const void* cache, int num_pages, int KVH, int page, int run, int HD) {
+  struct Key {
+    const void* p;
+    int n, k, g, r;
+    bool operator==(const Key& o) const { return p == o.p && n == o.n && k == o.k && g == o.g && r == o.r; }
+  };
+  static std::vector<std::pair<Key, CUtensorMap>> cache_;
+  static std::mutex mu;
+  std::lock_guard<std::mutex> lock(mu);
+  const Key key{cache, num_pages, KVH, page, run + 1024 * HD};
+  for (auto& e : cache_)
+    if (e.first == key) {
+      *out = e.second;
+      return true;
+    }
+  EncodeTiledFn fn = encode_fn();
+  if (fn == nullptr) return false;
+  cuuint64_t dims[4] = {(cuuint64_t)HD, (cuuint64_t)page, (cuuint64_t)KVH, (cuuint64_t)num_pages};
+  cuuint64_t strides[3] = {(cuuint64_t)HD * 2, (cuuint64_t)page * HD * 2, (cuuint64_t)KVH * page * HD * 2};
+  cuuint32_t box[4] = {64, (cuuint32_t)page, 1, (cuuint32_t)run};
+  cuuint32_t estr[4] = {1, 1, 1, 1};
+  if (fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(cache), dims, strides, box, estr,
+         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+    return false;
+  if (cache_.size() > 1024) cache_.clear();
+  cache_.emplace_back(key, *out);
+  return true;
+}
 
 }  // namespace tc

@@ -68,7 +68,7 @@ class LazyProduct:
 class CudaOps:
     """ctypes front of ``libturingserve_b200.so``."""
 
-    ABI = 16
+    ABI = 17
     UNSUPPORTED = -4            # a kernel's refusal of a shape or layout another kernel takes
 
     def __init__(self, lib_path: str) -> None:
@@ -134,6 +134,7 @@ class CudaOps:
             "ts_head_gated_rmsnorm": [P, P, P, I, P, I, F, I, I, I, I, P],
             "ts_attention_biased": [P, I, I, P, I, I, P, P, P, P, P, I, I, I, I, I, I, I, I, F, F, P, I, I, P, P, I, I, P, I, P, P, I, P],
             "ts_attention_biased_mma": [P, I, I, P, I, I, P, P, P, P, P, I, I, I, I, I, I, I, I, F, F, P, I, I, P, P, I, I, P, I, P, P, I, P],
+            "ts_attention_biased_tc": [P, I, I, P, I, I, P, P, P, P, P, I, I, I, I, I, I, I, I, I, F, F, P, I, I, P, I, P, P, I, P],
             "ts_rope_headnorm_write": [P, I, I, I, P, P, I, I, F, P, P, P, I, I, I, I, I, I, I, P, I, P],
             "ts_rope_headnorm_write_supports_parts": [I, I, I, I],
             "ts_rms_rows": [P, P, I, I, I, P, F, I, I, P],
@@ -173,6 +174,8 @@ class CudaOps:
         self.lib.ts_set_delta_rows(int(os.environ.get("TURINGSERVE_B200_DELTA_ROWS", "0")))
         self.lib.ts_attention_biased_mma_supported.argtypes = [I, I, I, I, I, I]
         self.lib.ts_attention_biased_mma_supported.restype = c_int
+        self.lib.ts_attention_biased_tc_supported.argtypes = [I, I, I, I, I, I, I]
+        self.lib.ts_attention_biased_tc_supported.restype = c_int
         self.lib.ts_attention_biased_mma_chunk.argtypes = [I, I, I]
         self.lib.ts_attention_biased_mma_chunk.restype = c_int
         self.lib.ts_attention_biased_mma_scratch_floats.argtypes = [I, I, I, I, I, I]
@@ -833,6 +836,12 @@ class CudaOps:
         self._check(self.lib.ts_batched_linear(_ptr(out), out.stride(0), out.stride(1), _ptr(x), x.stride(0), x.stride(1),
                                                _ptr(w), T, H, N, K, _code(x.dtype), self._stream()), "batched_linear")
 
+    # portions of this attention that reach over at least this many keys go to the tcgen05 kernel.  It starts with more set-up
+    # (latent rows, one prompt: 64 tokens 24.5 against 18.4 us on mma.sync, 128 tokens 25 against 26.5, 256 tokens 31 against
+    # 41; rows of 128: 16 tokens 14.3 against 12.3, 64 tokens 14.3 against 14.3, 256 tokens 16 against 25) and then takes a
+    # third of the time a key (8 tokens behind 2,000: 92 against 238 and 39 against 121 us; 2 behind 500: 33 against 64 and 18
+    # against 39 us), whatever the number of rows.
+    biased_tc_keys = int(os.environ.get("TURINGSERVE_B200_BIASED_TC_KEYS", "128"))
     biased_decode_splits = int(os.environ.get("TURINGSERVE_B200_BIASED_DECODE_SPLITS", "0"))
 
     def attention_biased(self, out, q, k_cache, v_cache, block_tables, step, KVH: int, page_size: int, scale: float,
@@ -891,11 +900,27 @@ class CudaOps:
                     float(softcap), _ptr(slopes), w, n_splits, _ptr(scratch), _ptr(counters), spread_flag, c, _ptr(sinks),
                     keep, _ptr(out_freq), _ptr(gate), gate_ts, self._stream())
 
+            def portions(first: int, count: int) -> int:
+                """Requests whose keys are not cut: by tcgen05 from ``biased_tc_keys`` keys on."""
+                if (self.use_tc_attention and reach >= self.biased_tc_keys
+                        and self.lib.ts_attention_biased_tc_supported(H, KVH, Dk, Dv, v_in_k, page_size, _code(q.dtype))):
+                    rc = self.lib.ts_attention_biased_tc(
+                        _ptr(out), out.stride(0), out.stride(1), _ptr(q), q.stride(0), q.stride(1), _ptr(k_cache), _ptr(v_cache),
+                        block_tables.data_ptr() + 4 * first * width, step.q_start.data_ptr() + 4 * first,
+                        step.seq_lens.data_ptr() + 4 * first, count, width, step.max_q_len, H, KVH, Dk, Dv, page_size,
+                        k_cache.shape[0], float(scale), float(softcap), _ptr(slopes), w, c, _ptr(sinks), keep, _ptr(out_freq),
+                        _ptr(gate), gate_ts, self._stream())
+                    if rc != self.UNSUPPORTED:
+                        return rc
+                return launch(first, count, step.max_q_len, 1, 0)
+
             if spread:
                 rc = launch(0, nd, 1, ms, 1)
                 if rc == 0 and nd < B:
                     self.launches += 1
-                    rc = launch(nd, B - nd, step.max_q_len, 1, 0)
+                    rc = portions(nd, B - nd)
+            elif ms == 1:
+                rc = portions(0, B)
             else:
                 rc = launch(0, B, step.max_q_len, ms, 0)
             if rc != self.UNSUPPORTED:
