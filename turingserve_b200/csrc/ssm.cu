@@ -18,6 +18,7 @@
 //                    computed; afterwards one block of the request stores the filter's new last inputs
 #include "common.cuh"
 #include "mma_utils.cuh"
+#include "scan_rows.cuh"
 
 namespace {
 
@@ -112,9 +113,27 @@ ssm_prepare_kernel(float* __restrict__ ready, const T* __restrict__ proj, int pr
   }
 }
 
-// PLAN: an instance of its own for long portions (its per-thread copy plan costs 60 registers more, which would halve the
-// blocks an SM holds in single-token steps: 51 -> 59 us at 112 heads)
-template <typename T, bool PLAN>
+// The filter's new last inputs: the step's last taps - 1 raw rows, or, of a step shorter than that, the old ones moved up (a
+// thread reads all it needs of a channel before it writes that channel).
+template <int THREADS, typename T>
+__device__ __forceinline__ void store_last_inputs(float* tail, const T* proj, int proj_stride, int xbc_off, int t0, int n, int Cn, int taps) {
+  const int keep = taps - 1;
+  for (int c = threadIdx.x; c < Cn; c += THREADS > 0 ? THREADS : blockDim.x) {
+    float v[SS_MAX_TAPS];
+#pragma unroll
+    for (int r = 0; r < SS_MAX_TAPS - 1; ++r) {
+      if (r < keep) {
+        const int rel = n - keep + r;
+        v[r] = rel >= 0 ? to_f(proj[(size_t)(t0 + rel) * proj_stride + xbc_off + c]) : tail[(size_t)(rel + keep) * Cn + c];
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < SS_MAX_TAPS - 1; ++r)
+      if (r < keep) tail[(size_t)r * Cn + c] = v[r];
+  }
+}
+
+template <typename T>
 __global__ void __launch_bounds__(512)
 ssm_scan_kernel(float* __restrict__ out, const float* __restrict__ ready, const T* __restrict__ proj, int proj_stride,
                 int xbc_off, float* __restrict__ state, size_t state_stride, const float* __restrict__ skip,
@@ -147,47 +166,13 @@ ssm_scan_kernel(float* __restrict__ out, const float* __restrict__ ready, const 
   for (int i = threadIdx.x; i < 2 * stage; i += blockDim.x) smem[i] = 0.f;     // (what no copy writes stays zero)
   __syncthreads();
 
-  // Which pieces of a group a thread copies is the same for every group: with PLAN (long portions) it is worked out
-  // once (the divisions of the index by the pieces a row would otherwise cost more instructions a group than the copies
-  // themselves; for a single token the plan itself is what costs: 28.7 -> 36.9 us).  16-byte pieces: at most
-  // SS_MAX_COPIES a thread (16 rows of N / 2 + 4 pieces over 16 ceil(N / 8) threads).
-  constexpr int SS_MAX_COPIES = 8;
-  int cp_row[SS_MAX_COPIES], cp_src[SS_MAX_COPIES], cp_dst[SS_MAX_COPIES];
-  if (PLAN && vec4) {
-    const int nb = N / 4, nx = cols_here / 4, per_row = 2 * nb + nx;
-#pragma unroll
-    for (int k = 0; k < SS_MAX_COPIES; ++k) {
-      const int i = threadIdx.x + k * blockDim.x;
-      cp_row[k] = SS_GROUP;                                // (beyond every group: never copied)
-      cp_src[k] = cp_dst[k] = 0;
-      if (i < SS_GROUP * per_row) {
-        const int r = i / per_row, c = i % per_row;
-        cp_row[k] = r;
-        if (c < nb) {
-          cp_src[k] = r * W + inner + g * N + 4 * c;
-          cp_dst[k] = r * Np + 4 * c;
-        } else if (c < 2 * nb) {
-          cp_src[k] = r * W + inner + GN + g * N + 4 * (c - nb);
-          cp_dst[k] = SS_GROUP * Np + r * Np + 4 * (c - nb);
-        } else {
-          cp_src[k] = r * W + h * P + blockIdx.x * SS_COLS + 4 * (c - 2 * nb);
-          cp_dst[k] = 2 * SS_GROUP * Np + r * SS_COLS + 4 * (c - 2 * nb);
-        }
-      }
-    }
-  }
   auto fetch = [&](int g0, int buf) {
     const int gn = min(SS_GROUP, n - g0);
     float* Bs = smem + (size_t)buf * stage;
     float* Cs = Bs + SS_GROUP * Np;
     float* xs = Cs + SS_GROUP * Np;
     float* da = xs + SS_GROUP * SS_COLS;
-    if (PLAN && vec4) {
-      const float* first = ready + (size_t)(t0 + g0) * W;
-#pragma unroll
-      for (int k = 0; k < SS_MAX_COPIES; ++k)
-        if (cp_row[k] < gn) cp_async_16(Bs + cp_dst[k], first + cp_src[k], true);
-    } else if (vec4) {
+    if (vec4) {
       const int nb = N / 4, nx = cols_here / 4, per_row = 2 * nb + nx;
       for (int i = threadIdx.x; i < gn * per_row; i += blockDim.x) {
         const int r = i / per_row, c = i % per_row;
@@ -233,7 +218,8 @@ ssm_scan_kernel(float* __restrict__ out, const float* __restrict__ ready, const 
       const float kx = dt * xv;
       const float4* br = reinterpret_cast<const float4*>(Bs + r * Np + part * SS_ROWS);
       const float4* cr = reinterpret_cast<const float4*>(Cs + r * Np + part * SS_ROWS);
-      float o = 0.f, o2 = 0.f;                             // two chains of four instead of one of eight
+      // (two chains, the order of scan_rows.cuh; the skip term starts the first row's)
+      float o = part == 0 ? dskip * xv : 0.f, o2 = 0.f;
 #pragma unroll
       for (int i = 0; i < SS_ROWS / 4; ++i) {
         const float4 b4 = br[i], c4 = cr[i];
@@ -246,18 +232,14 @@ ssm_scan_kernel(float* __restrict__ out, const float* __restrict__ ready, const 
         s[4 * i + 3] = fmaf(a, s[4 * i + 3], b4.w * kx);
         o2 = fmaf(s[4 * i + 3], c4.w, o2);
       }
-      // (the skip term rides with part 0: the loop below reads nothing of the staged rows, which the next group's
-      // copies may already be writing over)
-      o_s[(r * parts + part) * SS_COLS + col] = o + o2 + (part == 0 ? dskip * xv : 0.f);
+      o_s[(r * parts + part) * SS_COLS + col] = o + o2;
     }
     __syncthreads();
     for (int i = threadIdx.x; i < gn * SS_COLS; i += blockDim.x) {
       const int r = i / SS_COLS, c = i % SS_COLS;
       const int jj = blockIdx.x * SS_COLS + c;
       if (jj >= P) continue;
-      float o = 0.f;
-      for (int p = 0; p < parts; ++p) o += o_s[(r * parts + p) * SS_COLS + c];
-      out[(size_t)(t0 + g0 + r) * inner + h * P + jj] = o;
+      out[(size_t)(t0 + g0 + r) * inner + h * P + jj] = scan::tree_of_parts(o_s + r * parts * SS_COLS + c, parts, SS_COLS);
     }
   }
   cp_async_wait<0>();
@@ -266,25 +248,169 @@ ssm_scan_kernel(float* __restrict__ out, const float* __restrict__ ready, const 
     const int d = part * SS_ROWS + i;
     if (live && d < N) S[(size_t)d * P + j] = s[i];
   }
-  // the filter's new last inputs: the step's last taps - 1 raw rows, or, of a step shorter than that, the old ones
-  // moved up (a thread reads all it needs of a channel before it writes that channel)
-  if (blockIdx.x == 0 && h == 0 && taps > 1) {
-    float* tail = base + (size_t)H * N * P;
-    const int keep = taps - 1;
-    for (int c = threadIdx.x; c < Cn; c += blockDim.x) {
-      float v[SS_MAX_TAPS];
+  if (blockIdx.x == 0 && h == 0 && taps > 1)
+    store_last_inputs<0>(base + (size_t)H * N * P, proj, proj_stride, xbc_off, t0, n, Cn, taps);
+}
+
+// ---- long portions: half a warp owns SL_OWN columns, a lane ROWS rows of them, in registers over all tokens; groups of 16
+// tokens arrive by cp.async, two groups ahead, issued by two warps of their own; eight tokens' outputs of the two columns are
+// summed over the lanes at once.  What bounds it: issue slots, about 60 instructions a token and warp, two warps a scheduler
+// on the SMs that hold two blocks.  2,048 tokens, 48 heads of 128 x 64: 391 -> 267 us (before: a thread a column and 8 rows, a
+// block-wide sum of its parts).
+constexpr int SL_WARPS = 4, SL_LOAD_WARPS = 2, SL_OWN = 2, SL_COLS = 2 * SL_OWN * SL_WARPS, SL_STAGES = 3;
+
+template <typename T, int ROWS>
+__global__ void __launch_bounds__((SL_WARPS + SL_LOAD_WARPS) * 32)
+ssm_scan_long_kernel(float* __restrict__ out, const float* __restrict__ ready, const T* __restrict__ proj, int proj_stride,
+                     int xbc_off, float* __restrict__ state, size_t state_stride, const float* __restrict__ skip,
+                     const int* __restrict__ q_start, const int* __restrict__ slots, int H, int G, int N, int P, int taps) {
+  using namespace scan;
+  constexpr int NP = 16 * ROWS, COLS = SL_COLS, TOK = 2 * NP + COLS + 4;
+  static_assert(SS_GROUP / 2 * SL_OWN == 16, "half a group's outputs of the columns are half a warp's lanes");
+  pdl_launch_dependents();
+  pdl_wait();
+  extern __shared__ __align__(16) float smem[];            // [SL_STAGES][SS_GROUP][NP B | NP C | COLS x | dt, a, 2 unused]
+  const int h = blockIdx.y, b = blockIdx.z;
+  const int t0 = q_start[b], n = q_start[b + 1] - t0;
+  if (n <= 0) return;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, p = lane & 15, col = SL_OWN * (2 * warp + (lane >> 4));
+  const int g = h / (H / G);
+  const int inner = H * P, GN = G * N, Cn = inner + 2 * GN, W = Cn + 2 * H;
+  const int j0 = blockIdx.x * COLS, j = j0 + col;
+  if (N < NP || j0 + COLS > P) {
+    for (int i = threadIdx.x; i < SL_STAGES * SS_GROUP * TOK / 4; i += blockDim.x)
+      reinterpret_cast<float4*>(smem)[i] = make_float4(0.f, 0.f, 0.f, 0.f);    // (rows beyond N, columns beyond P stay zero)
+    __syncthreads();
+  }
+  if (warp >= SL_WARPS) {
+    // Loading warp w brings tokens w, w + SL_LOAD_WARPS, ... of a group, a lane the pieces lane, lane + 32 of B and C; single
+    // lanes the rest.
+    const int w = warp - SL_WARPS;
+    const int nb = N / 4, nx = min(COLS, P - j0) / 4;
+    const float* src = ready + (size_t)(t0 + w) * W + inner + g * N + 4 * lane;
+    const float* x_src = ready + (size_t)(t0 + w) * W + (lane < 16 ? h * P + j0 + 4 * lane : Cn + (lane - 16) * H + h);
+    auto fetch = [&](int g0, int st) {
+      const int gn = n - g0;
+      const size_t first = (size_t)g0 * W;
+      float* dst = smem + (st * SS_GROUP + w) * TOK;
 #pragma unroll
-      for (int r = 0; r < SS_MAX_TAPS - 1; ++r) {
-        if (r < keep) {
-          const int rel = n - keep + r;
-          v[r] = rel >= 0 ? to_f(proj[(size_t)(t0 + rel) * proj_stride + xbc_off + c]) : tail[(size_t)(rel + keep) * Cn + c];
+      for (int rr = 0; rr < SS_GROUP / SL_LOAD_WARPS; ++rr) {
+        if (w + rr * SL_LOAD_WARPS >= gn) break;
+        const size_t off = first + (size_t)rr * SL_LOAD_WARPS * W;
+        float* d = dst + rr * SL_LOAD_WARPS * TOK;
+#pragma unroll
+        for (int c = 0; c < NP / 4; c += 32) {
+          if (lane + c < nb) {
+            const int at = 4 * piece_at<ROWS>(lane + c);
+            cp_async_16(d + at, src + off + 4 * c, true);
+            cp_async_16(d + NP + at, src + off + 4 * c + GN, true);
+          }
+        }
+        if (lane < nx) cp_async_16(d + 2 * NP + 4 * lane, x_src + off, true);
+        else if (lane == 16 || lane == 17) ss_cp_async_4(d + 2 * NP + COLS + lane - 16, x_src + off);
+      }
+    };
+#pragma unroll
+    for (int st = 0; st < SL_STAGES - 1; ++st) {
+      if (st * SS_GROUP < n) fetch(st * SS_GROUP, st);
+      cp_async_commit();
+    }
+    int st = 0;
+    for (int g0 = 0; g0 < n; g0 += SS_GROUP, st = st + 1 == SL_STAGES ? 0 : st + 1) {
+      cp_async_wait<SL_STAGES - 2>();
+      __syncthreads();                                     // group g0 is here, and the one before has been computed from
+      const int ahead = g0 + (SL_STAGES - 1) * SS_GROUP;
+      if (ahead < n) fetch(ahead, st == 0 ? SL_STAGES - 1 : st - 1);
+      cp_async_commit();
+    }
+    cp_async_wait<0>();
+    return;
+  }
+  const bool live = j < P;                                 // (P is a multiple of 4: both columns or none)
+  float* base = state + (size_t)slots[b] * state_stride;
+  float* S = base + (size_t)h * N * P + j;
+  f2 s[SL_OWN][ROWS / 2];
+#pragma unroll
+  for (int i = 0; i < ROWS / 2; ++i) {
+    const int d = p * ROWS + 2 * i;                        // (N is a multiple of 4: both rows or none)
+    const bool there = live && d < N;
+#pragma unroll
+    for (int c = 0; c < SL_OWN; ++c)
+      s[c][i] = pack2(there ? S[(size_t)d * P + c] : 0.f, there ? S[(size_t)(d + 1) * P + c] : 0.f);
+  }
+  const float dskip = skip != nullptr ? skip[h] : 0.f;
+  float x[16];                                             // this lane's share of eight tokens' outputs, token * 2 + column
+  struct Token {
+    f2 B[ROWS / 2], C[ROWS / 2];
+    float2 x, da;
+  };
+  const uint32_t ring = (uint32_t)__cvta_generic_to_shared(smem);
+  auto load = [&](Token& t, uint32_t at) {
+    load_rows<ROWS>(at, p, t.B);
+    load_rows<ROWS>(at + 4 * NP, p, t.C);
+    t.x = load_pair(at + 4 * (2 * NP + col));
+    t.da = load_pair(at + 4 * (2 * NP + COLS));
+  };
+  auto take = [&](const Token& t, int r, Token& next, uint32_t next_at, bool more) {
+    const f2 a2 = pack2(t.da.y, t.da.y);
+    f2 bx[SL_OWN][ROWS / 2];
+#pragma unroll
+    for (int c = 0; c < SL_OWN; ++c) {
+      const float kx = t.da.x * (c == 0 ? t.x.x : t.x.y);
+      const f2 k2 = pack2(kx, kx);
+#pragma unroll
+      for (int i = 0; i < ROWS / 2; ++i) bx[c][i] = mul2_first(t.B[i], k2);
+    }
+    if (more) load(next, next_at);
+#pragma unroll
+    for (int c = 0; c < SL_OWN; ++c) {
+#pragma unroll
+      for (int i = 0; i < ROWS / 2; ++i) s[c][i] = fma2(a2, s[c][i], bx[c][i]);
+      // (the skip term starts the first row's chain)
+      x[r * SL_OWN + c] = dot_rows<ROWS>(s[c], t.C, p == 0 ? dskip * (c == 0 ? t.x.x : t.x.y) : 0.f);
+    }
+  };
+  int st = 0;
+  for (int g0 = 0; g0 < n; g0 += SS_GROUP, st = st + 1 == SL_STAGES ? 0 : st + 1) {
+    __syncthreads();
+    const int gn = min(SS_GROUP, n - g0);
+#pragma unroll 1
+    for (int r0 = 0; r0 < gn; r0 += SS_GROUP / 2) {
+      const uint32_t grp = ring + 4 * (st * SS_GROUP + r0) * TOK;
+      Token tk[2];
+      if (r0 + SS_GROUP / 2 <= gn) {
+        load(tk[0], grp);
+#pragma unroll
+        for (int r = 0; r < SS_GROUP / 2; ++r) take(tk[r & 1], r, tk[(r + 1) & 1], grp + 4 * (r + 1) * TOK, r + 1 < SS_GROUP / 2);
+      } else {
+#pragma unroll
+        for (int r = 0; r < SS_GROUP / 2; ++r) {
+#pragma unroll
+          for (int c = 0; c < SL_OWN; ++c) x[r * SL_OWN + c] = 0.f;
+          if (r0 + r < gn) {
+            load(tk[0], grp + 4 * r * TOK);
+            take(tk[0], r, tk[1], 0, false);
+          }
         }
       }
-#pragma unroll
-      for (int r = 0; r < SS_MAX_TAPS - 1; ++r)
-        if (r < keep) tail[(size_t)r * Cn + c] = v[r];
+      const float o = sum_scatter(x, lane);
+      const int r = r0 + p / SL_OWN;
+      if (live && r < gn) out[(size_t)(t0 + g0 + r) * inner + h * P + j + p % SL_OWN] = o;
     }
   }
+#pragma unroll
+  for (int i = 0; i < ROWS / 2; ++i) {
+    const int d = p * ROWS + 2 * i;
+    if (!live || d >= N) continue;
+#pragma unroll
+    for (int c = 0; c < SL_OWN; ++c) {
+      const float2 v = unpack2(s[c][i]);
+      S[(size_t)d * P + c] = v.x;
+      S[(size_t)(d + 1) * P + c] = v.y;
+    }
+  }
+  if (blockIdx.x == 0 && h == 0 && taps > 1)
+    store_last_inputs<SL_WARPS * 32>(base + (size_t)H * N * P, proj, proj_stride, xbc_off, t0, n, Cn, taps);
 }
 
 }  // namespace
@@ -338,22 +464,46 @@ TS_API int ts_ssm_scan(float* out, const float* ready, const void* proj, int pro
   // 16-byte copies: every piece of a row (B, C, this block's x columns) on a 16-byte boundary
   const int vec4 = N % 4 == 0 && P % 4 == 0 && W % 4 == 0 && !((uintptr_t)ready & 15);
   const size_t smem = sizeof(float) * ((size_t)2 * SS_GROUP * (2 * parts * SS_ROWS + SS_COLS + 4) + (size_t)SS_GROUP * parts * SS_COLS);
+  if (longest >= SS_LATE_TOKENS && vec4) {
+#define TS_SL(TT, RR)                                                                                                   \
+  do {                                                                                                                  \
+    constexpr size_t bytes = sizeof(float) * SL_STAGES * SS_GROUP * (2 * 16 * RR + SL_COLS + 4);                        \
+    static bool configured = false;                                                                                     \
+    if (!configured) {                                                                                                  \
+      cudaError_t e = cudaFuncSetAttribute(ssm_scan_long_kernel<TT, RR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes); \
+      if (e != cudaSuccess) TS_REFUSE((int)e, "ts_ssm_scan: shared memory %zu: %s", bytes, cudaGetErrorString(e));      \
+      configured = true;                                                                                                \
+    }                                                                                                                   \
+    ts_launch_late(ssm_scan_long_kernel<TT, RR>, dim3(ceil_div(P, SL_COLS), H, B), dim3((SL_WARPS + SL_LOAD_WARPS) * 32), bytes, s, \
+                   out, ready, (const TT*)proj, proj_stride, xbc_off, state, (size_t)state_stride, skip, q_start, slots, H, G, N, P, \
+                   taps);                                                                                               \
+  } while (0)
+    if (dtype == TS_F32) {
+      if (N <= 128) TS_SL(float, 8);
+      else TS_SL(float, 16);
+    } else if (dtype == TS_BF16) {
+      if (N <= 128) TS_SL(bf16, 8);
+      else TS_SL(bf16, 16);
+    } else {
+      TS_REFUSE(TS_ERR_DTYPE, "ts_ssm_scan: dtype %d", dtype);
+    }
+#undef TS_SL
+    TS_LAUNCH_CHECK();
+  }
   dim3 grid(ceil_div(P, SS_COLS), H, B);
 #define TS_SC(TT)                                                                                                       \
   do {                                                                                                                  \
     static size_t configured = 0;                                                                                       \
     if (smem > 48 * 1024 && smem > configured) {                                                                        \
-      cudaError_t e = cudaFuncSetAttribute(ssm_scan_kernel<TT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-      if (e == cudaSuccess)                                                                                             \
-        e = cudaFuncSetAttribute(ssm_scan_kernel<TT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);    \
+      cudaError_t e = cudaFuncSetAttribute(ssm_scan_kernel<TT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
       if (e != cudaSuccess) TS_REFUSE((int)e, "ts_ssm_scan: shared memory %zu: %s", smem, cudaGetErrorString(e));       \
       configured = smem;                                                                                                \
     }                                                                                                                   \
     if (longest >= SS_LATE_TOKENS)                                                                                      \
-      ts_launch_late(ssm_scan_kernel<TT, true>, grid, dim3(parts * SS_COLS), smem, s, out, ready, (const TT*)proj, proj_stride, xbc_off, \
+      ts_launch_late(ssm_scan_kernel<TT>, grid, dim3(parts * SS_COLS), smem, s, out, ready, (const TT*)proj, proj_stride, xbc_off, \
                      state, (size_t)state_stride, skip, q_start, slots, H, G, N, P, taps, parts, vec4);                 \
     else                                                                                                                \
-      ts_launch(ssm_scan_kernel<TT, false>, grid, dim3(parts * SS_COLS), smem, s, out, ready, (const TT*)proj, proj_stride, xbc_off, \
+      ts_launch(ssm_scan_kernel<TT>, grid, dim3(parts * SS_COLS), smem, s, out, ready, (const TT*)proj, proj_stride, xbc_off, \
                 state, (size_t)state_stride, skip, q_start, slots, H, G, N, P, taps, parts, vec4);                      \
   } while (0)
   if (dtype == TS_F32) TS_SC(float);

@@ -68,7 +68,7 @@ class LazyProduct:
 class CudaOps:
     """ctypes front of ``libturingserve_b200.so``."""
 
-    ABI = 17
+    ABI = 18
     UNSUPPORTED = -4            # a kernel's refusal of a shape or layout another kernel takes
 
     def __init__(self, lib_path: str) -> None:
@@ -124,6 +124,8 @@ class CudaOps:
             "ts_ssm_prepare": [P, P, I, I, I, P, P, P, P, P, ctypes.c_longlong, ctypes.c_longlong, P, P, P, I, I, I, I, I, P],
             "ts_ssm_scan": [P, P, P, I, I, P, ctypes.c_longlong, P, P, P, I, I, I, I, I, I, I, I, P],
             "ts_lightning_ex": [P, P, I, P, P, P, P, I, I, I, I, I, I, P],
+            "ts_lightning_long": [P, P, I, P, P, P, P, P, I, I, I, I, I, I, I, P],
+            "ts_lightning_long_supported": [I, I, I, I, I],
             "ts_gated_group_rmsnorm": [P, I, P, P, I, P, F, I, I, I, I, I, F, I, P],
             "ts_gate_mul": [P, I, P, I, P, I, I, I, I, F, I, P],
             "ts_act_mul": [P, P, I, I, I, I, I, P],
@@ -646,9 +648,19 @@ class CudaOps:
         """out (float32 [T, H V]): per head o_t = S_t^T q_t with S_t = decay_h S_(t-1) + k_t v_t^T, where
         q, k, v = silu of the columns [0, HD), [HD, 2HD), [2HD, 2HD + HV) of ``proj``; ``state``
         (float32 [slots, H, D, V]) is read and left updated at each request's slot."""
+        longest = int(getattr(step, "max_q_len", 0) or 0)
+        if self.lib.ts_lightning_long_supported(D, V, proj.stride(0), longest, _code(proj.dtype)):
+            ready = torch.empty((proj.shape[0], H * (2 * D + V)), dtype=torch.float32, device=proj.device)
+            rc = self.lib.ts_lightning_long(_ptr(out), _ptr(proj), proj.stride(0), _ptr(ready), _ptr(state), _ptr(decay),
+                                            _ptr(step.q_start), _ptr(step.state_slots), step.num_requests, proj.shape[0], H, D, V,
+                                            longest, _code(proj.dtype), self._stream())
+            if rc != self.UNSUPPORTED:
+                self.launches += 1
+                self._check(rc, "lightning_long")
+                return
         self._check(self.lib.ts_lightning_ex(_ptr(out), _ptr(proj), proj.stride(0), _ptr(state), _ptr(decay),
                                              _ptr(step.q_start), _ptr(step.state_slots), step.num_requests, H, D, V,
-                                             int(getattr(step, "max_q_len", 0) or 0), _code(proj.dtype), self._stream()),
+                                             longest, _code(proj.dtype), self._stream()),
                     "lightning")
 
     # -- attention with two score maps a head --------------------------------------------------------------
