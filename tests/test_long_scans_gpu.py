@@ -126,3 +126,46 @@ def test_state_space_long_portions(ops, dtype, H, P, N, G, taps, skipped):
         at += n
     for r in results[1:]:
         assert torch.equal(r[0], results[0][0]) and torch.equal(r[1], results[0][1])
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("H,G,D,V,taps,pad", [(4, 2, 128, 128, 4, 2), (2, 1, 64, 40, 3, 3), (3, 3, 8, 4, 1, 3), (2, 1, 100, 20, 2, 3),
+                                             (2, 1, 128, 24, 8, 3), (2, 1, 64, 40, 3, 0)])
+def test_delta_rule_portions(ops, dtype, H, G, D, V, taps, pad):
+    """Rows on 16-byte boundaries (``pad``) go to the kernel of eight lanes a column, others do not; portions of any lengths
+    from two tokens give the same bits."""
+    lens, C = [150, 64, 9, 200], 2 * G * D + H * V
+    width = C + 2 * H + G
+    assert pad == 0 or (width + pad) % 4 == 0
+    g = torch.Generator(device=DEV).manual_seed(D + V)
+    rnd = lambda *s: torch.randn(*s, generator=g, device=DEV)
+    proj = rnd(sum(lens), C + H * V + 2 * H).to(dtype)
+    conv_w, a_log, dt = rnd(C, taps) * 0.5, rnd(H) * 0.3, rnd(H) - 2.0
+    first = rnd(9, H * D * V + (taps - 1) * C)
+    results = []
+    for cuts in ((), (63,), (2, 66), (64, 70, 90), (16, 32, 148)):
+        state, out, kept = first.clone(), torch.full((sum(lens), H * V), float("nan"), device=DEV), torch.empty(sum(lens), width, device=DEV)
+        for rows, step in steps(lens, cuts):
+            p = proj[rows].contiguous()
+            ready = torch.full((len(rows), width + pad), float("nan"), device=DEV)[:, :width]
+            ops.delta_prepare(ready, p, conv_w, a_log, dt, state, step, H, G, D, V, taps, 1e-6)
+            o = torch.empty(len(rows), H * V, device=DEV)
+            ops.delta_scan(o, ready, p, state, step, H, G, D, V, taps)
+            out[rows], kept[rows] = o, ready
+        results.append((out, state, kept))
+    r = results[0][2].double()
+    q, k = (r[:, i * G * D:(i + 1) * G * D].view(-1, G, D).repeat_interleave(H // G, 1) for i in (0, 1))
+    v, fade, w = r[:, 2 * G * D:C].view(-1, H, V), r[:, C:C + H], r[:, C + H:C + 2 * H]
+    at = 0
+    for i, n in enumerate(lens):
+        S, o = first[2 * i + 1, :H * D * V].view(H, D, V).double(), []
+        for t in range(at, at + n):
+            S = fade[t][:, None, None] * S
+            u = w[t][:, None] * (v[t] - torch.einsum("hdv,hd->hv", S, k[t]))
+            S = S + k[t][:, :, None] * u[:, None, :]
+            o.append(torch.einsum("hdv,hd->hv", S, q[t]).reshape(-1))
+        assert close(results[0][0][at:at + n], torch.stack(o)) and close(results[0][1][2 * i + 1, :H * D * V], S.reshape(-1))
+        assert torch.equal(results[0][1][2 * i], first[2 * i])
+        at += n
+    for r in results[1:]:
+        assert torch.equal(r[0], results[0][0]) and torch.equal(r[1], results[0][1])

@@ -9,8 +9,8 @@
 //   ts_delta_prepare      one block per (token, head): filter + SiLU, unit length per head, g, beta and k.q, as 32-bit
 //                         rows [q (G D) | k (G D) | v (H V) | g (H) | beta (H) | k.q (G)]; reads the slot's filter
 //                         inputs for the tokens before the step's first, writes nothing to the slot
-//   ts_delta_scan         the recurrence, token by token for portions and single tokens alike (cutting a prompt
-//                         changes no bit); afterwards the request's blocks store the filter's new last inputs
+//   ts_delta_scan         the recurrence, token by token for portions (cutting a prompt into portions changes no bit) and
+//                         single tokens; afterwards the request's blocks store the filter's new last inputs
 //   ts_head_gated_rmsnorm o / rms(o) per head, times a weight (shared by the heads or one a head), times silu(gate)
 //
 // The scan: one pass over the state per token.  With a = (g S)^T k and c = (g S)^T q, both sums over the old
@@ -20,6 +20,7 @@
 // arrive in groups of DR_GROUP rows by cp.async, three groups ahead of the one that is computed.
 #include "common.cuh"
 #include "mma_utils.cuh"
+#include "scan_rows.cuh"
 
 namespace {
 
@@ -35,7 +36,7 @@ __device__ __forceinline__ float softplus_f(float x) { return x > 20.f ? x : log
 
 template <typename T>
 __global__ void __launch_bounds__(128)
-delta_prepare_kernel(float* __restrict__ ready, const T* __restrict__ proj, int proj_stride,
+delta_prepare_kernel(float* __restrict__ ready, int W, const T* __restrict__ proj, int proj_stride,
                      const float* __restrict__ conv_w, const float* __restrict__ a_log,
                      const float* __restrict__ dt_bias, const float* __restrict__ state, size_t state_stride,
                      const int* __restrict__ token_request, const int* __restrict__ q_start,
@@ -47,7 +48,7 @@ delta_prepare_kernel(float* __restrict__ ready, const T* __restrict__ proj, int 
   const int t = blockIdx.x, unit = blockIdx.y;         // units: the G query/key heads, then the H value heads
   const int b = token_request[t];
   const int t0 = q_start[b], i = t - t0;
-  const int qk = G * D, hv = H * V, C = 2 * qk + hv, W = C + 2 * H + G;
+  const int qk = G * D, hv = H * V, C = 2 * qk + hv;
   const float* tail = state + (size_t)slots[b] * state_stride + (size_t)H * D * V;     // [taps - 1][C]
   float* out = ready + (size_t)t * W;
   auto filtered = [&](int c) {
@@ -93,10 +94,35 @@ delta_prepare_kernel(float* __restrict__ ready, const T* __restrict__ proj, int 
   if (threadIdx.x == 0) out[C + 2 * H + g] = dot * rq * rk;
 }
 
+// The filter's new last inputs: what the slot held, moved up by n, then this step's raw rows; every block of the request takes
+// a share of the channels.
+__device__ __forceinline__ void store_last_inputs(float* tail, const void* proj, int proj_is_bf16, int proj_stride, int t0, int n, int C,
+                                                  int taps, int first, int stride) {
+  for (int c = first; c < C; c += stride) {
+    float nv[7];
+#pragma unroll
+    for (int jt = 0; jt < 7; ++jt) {
+      const int rel = n - (taps - 1) + jt;
+      nv[jt] = 0.f;
+      if (jt < taps - 1) {
+        if (rel >= 0) {
+          const size_t at = (size_t)(t0 + rel) * proj_stride + c;
+          nv[jt] = proj_is_bf16 ? to_f(reinterpret_cast<const bf16*>(proj)[at]) : reinterpret_cast<const float*>(proj)[at];
+        } else {
+          nv[jt] = tail[(size_t)(rel + taps - 1) * C + c];
+        }
+      }
+    }
+#pragma unroll
+    for (int jt = 0; jt < 7; ++jt)
+      if (jt < taps - 1) tail[(size_t)jt * C + c] = nv[jt];
+  }
+}
+
 // R rows of a column a lane; P lanes a column; CW = 32 / P columns a warp.
 template <int R>
 __global__ void __launch_bounds__(256, 1)
-delta_scan_kernel(float* __restrict__ out, const float* __restrict__ ready, const void* __restrict__ proj,
+delta_scan_kernel(float* __restrict__ out, const float* __restrict__ ready, int W, const void* __restrict__ proj,
                   int proj_stride, int proj_is_bf16, float* __restrict__ state, size_t state_stride,
                   const int* __restrict__ q_start, const int* __restrict__ slots, int H, int G, int D, int V,
                   int taps, int P, int vec4, int group) {
@@ -107,7 +133,7 @@ delta_scan_kernel(float* __restrict__ out, const float* __restrict__ ready, cons
   const int t0 = q_start[b], n = q_start[b + 1] - t0;
   if (n <= 0) return;
   const int kvh = h / (H / G);
-  const int qk = G * D, hv = H * V, C = 2 * qk + hv, W = C + 2 * H + G;
+  const int qk = G * D, hv = H * V, C = 2 * qk + hv;
   const int CW = 32 / P;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   const int p = lane / CW, cw = lane % CW;
@@ -222,30 +248,188 @@ delta_scan_kernel(float* __restrict__ out, const float* __restrict__ ready, cons
     const int d = p * R + i;
     if (live && d < D) S[(size_t)d * V + j] = s[i];
   }
-  // the filter's new last inputs: what the slot held, moved up by n, then this step's raw rows
-  if (taps > 1) {
-    float* tail = base + (size_t)H * D * V;
-    const int first = (h * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x, stride = H * gridDim.x * blockDim.x;
-    for (int c = first; c < C; c += stride) {                  // every block of the request takes a share of the channels
-      float nv[7];
+  if (taps > 1)
+    store_last_inputs(base + (size_t)H * D * V, proj, proj_is_bf16, proj_stride, t0, n, C, taps,
+                      (h * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x, H * gridDim.x * blockDim.x);
+}
+
+// ---- portions of keys up to 128 wide: eight lanes of a warp own a column, a lane 16 rows of it, two 32-bit operations an
+// instruction.  A token's chain is the sum a over the eight lanes (three shuffles), u, and the update; the read-out's sum is
+// not on it: a lane keeps its share of eight tokens' outputs, and eight sums cross the lanes at once.  Tokens arrive in groups
+// of 16 by cp.async, two groups ahead, issued by two warps of their own; a token's operands are loaded while the one before is
+// computed.  What bounds it: that chain, about 280 cycles a token.  1,537 tokens, 12 heads of 128 x 128: 460 -> 230 us (before:
+// a lane 8 rows, four shuffles for each of two sums, rows fetched by 4-byte copies because they were 3,102 values apart; they
+// start on 16-byte boundaries now).  Single tokens stay with the kernel above: one trip through the chain, and half as many
+// threads to a column.
+constexpr int DL_WARPS = 4, DL_LOAD_WARPS = 2, DL_COLS = 4 * DL_WARPS, DL_STAGES = 3, DL_ROWS = 16, DL_KEYS = 8 * DL_ROWS;
+
+__global__ void __launch_bounds__((DL_WARPS + DL_LOAD_WARPS) * 32, 2)
+delta_scan_rows_kernel(float* __restrict__ out, const float* __restrict__ ready, int W, const void* __restrict__ proj,
+                       int proj_stride, int proj_is_bf16, float* __restrict__ state, size_t state_stride,
+                       const int* __restrict__ q_start, const int* __restrict__ slots, int H, int G, int D, int V, int taps) {
+  using namespace scan;
+  constexpr int TOK = 2 * DL_KEYS + DL_COLS + 4;           // q | k | v of the block's columns | g, beta, k.q, 1 unused
+  pdl_launch_dependents();
+  pdl_wait();
+  extern __shared__ __align__(16) float smem[];            // [DL_STAGES][DR_GROUP][TOK]
+  const int h = blockIdx.y, b = blockIdx.z;
+  const int t0 = q_start[b], n = q_start[b + 1] - t0;
+  if (n <= 0) return;
+  const int kvh = h / (H / G);
+  const int qk = G * D, hv = H * V, C = 2 * qk + hv;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, p = lane & 7, col = 4 * warp + (lane >> 3);
+  const int j0 = blockIdx.x * DL_COLS, j = j0 + col;
+  if (D < DL_KEYS || j0 + DL_COLS > V) {                   // what no copy writes stays zero
+    for (int i = threadIdx.x; i < DL_STAGES * DR_GROUP * TOK / 4; i += blockDim.x)
+      reinterpret_cast<float4*>(smem)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    __syncthreads();
+  }
+  if (warp >= DL_WARPS) {
+    // Loading warp w brings tokens w, w + DL_LOAD_WARPS, ... of a group, a lane piece `lane` (four rows) of q and k: lane p's
+    // k-th piece lies at piece k * 8 + p, so that a column's lanes read neighbouring pieces.
+    const int w = warp - DL_WARPS;
+    const int chunks = D / 4, v_chunks = min(DL_COLS, V - j0) / 4, at = 4 * ((lane & 3) * 8 + (lane >> 2));
+    const float* src = ready + (size_t)(t0 + w) * W + kvh * D + 4 * lane;
+    const float* v_src = ready + (size_t)(t0 + w) * W + 2 * qk + h * V + j0 + 4 * lane;
+    const float* s_src = ready + (size_t)(t0 + w) * W + C + (lane == 16 ? h : lane == 17 ? H + h : 2 * H + kvh);
+    auto fetch = [&](int g0, int st) {
+      const int gn = n - g0;
+      const size_t first = (size_t)g0 * W;
+      float* dst = smem + (st * DR_GROUP + w) * TOK;
 #pragma unroll
-      for (int jt = 0; jt < 7; ++jt) {
-        const int rel = n - (taps - 1) + jt;
-        nv[jt] = 0.f;
-        if (jt < taps - 1) {
-          if (rel >= 0) {
-            const size_t at = (size_t)(t0 + rel) * proj_stride + c;
-            nv[jt] = proj_is_bf16 ? to_f(reinterpret_cast<const bf16*>(proj)[at]) : reinterpret_cast<const float*>(proj)[at];
-          } else {
-            nv[jt] = tail[(size_t)(rel + taps - 1) * C + c];
+      for (int rr = 0; rr < DR_GROUP / DL_LOAD_WARPS; ++rr) {
+        if (w + rr * DL_LOAD_WARPS >= gn) break;
+        const size_t off = first + (size_t)rr * DL_LOAD_WARPS * W;
+        float* d = dst + rr * DL_LOAD_WARPS * TOK;
+        if (lane < chunks) {
+          cp_async_16(d + at, src + off, true);
+          cp_async_16(d + DL_KEYS + at, src + off + qk, true);
+        }
+        if (lane < v_chunks) cp_async_16(d + 2 * DL_KEYS + 4 * lane, v_src + off, true);
+        else if (lane >= 16 && lane < 19) cp_async_4(d + 2 * DL_KEYS + DL_COLS + lane - 16, s_src + off);
+      }
+    };
+#pragma unroll
+    for (int st = 0; st < DL_STAGES - 1; ++st) {
+      if (st * DR_GROUP < n) fetch(st * DR_GROUP, st);
+      cp_async_commit();
+    }
+    int st = 0;
+    for (int g0 = 0; g0 < n; g0 += DR_GROUP, st = st + 1 == DL_STAGES ? 0 : st + 1) {
+      cp_async_wait<DL_STAGES - 2>();
+      __syncthreads();                                     // group g0 is here, and the one before has been computed from
+      const int ahead = g0 + (DL_STAGES - 1) * DR_GROUP;
+      if (ahead < n) fetch(ahead, st == 0 ? DL_STAGES - 1 : st - 1);
+      cp_async_commit();
+    }
+    cp_async_wait<0>();
+    return;
+  }
+  const bool live = j < V;
+  float* base = state + (size_t)slots[b] * state_stride;
+  float* S = base + (size_t)h * D * V + j;
+  f2 s[DL_ROWS / 2];
+#pragma unroll
+  for (int i = 0; i < DL_ROWS / 2; ++i) {
+    const int d = p * DL_ROWS + 2 * i;                     // (D is a multiple of 4: both rows or none)
+    const bool there = live && d < D;
+    s[i] = pack2(there ? S[(size_t)d * V] : 0.f, there ? S[(size_t)(d + 1) * V] : 0.f);
+  }
+  struct Token {
+    f2 k[DL_ROWS / 2], q[DL_ROWS / 2];
+    float v, g, beta, kq;
+  };
+  const uint32_t ring = (uint32_t)__cvta_generic_to_shared(smem);
+  auto load = [&](Token& t, uint32_t at) {
+#pragma unroll
+    for (int k = 0; k < DL_ROWS / 4; ++k) {
+      asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(t.k[2 * k]), "=l"(t.k[2 * k + 1]) : "r"(at + 4 * DL_KEYS + 16 * (k * 8 + p)));
+      asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(t.q[2 * k]), "=l"(t.q[2 * k + 1]) : "r"(at + 16 * (k * 8 + p)));
+    }
+    t.v = load_f32(at + 4 * (2 * DL_KEYS + col));
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, _}, [%3];" : "=f"(t.g), "=f"(t.beta), "=f"(t.kq) : "r"(at + 4 * (2 * DL_KEYS + DL_COLS)));
+  };
+  float x[8];                                              // this lane's share of the column's eight outputs
+  auto take = [&](const Token& t, int r, Token& next, uint32_t next_at, bool more) {
+    // a = S^T k over the old state: two chains of four pairs a lane
+    f2 a0 = mul2_first(s[0], t.k[0]), a1 = mul2_first(s[4], t.k[4]);
+    if (more) load(next, next_at);
+#pragma unroll
+    for (int i = 1; i < 4; ++i) {
+      a0 = fma2(s[i], t.k[i], a0);
+      a1 = fma2(s[4 + i], t.k[4 + i], a1);
+    }
+    const float2 e0 = unpack2(a0), e1 = unpack2(a1);
+    float a = (e0.x + e0.y) + (e1.x + e1.y);
+    a += __shfl_xor_sync(0xffffffffu, a, 1);
+    // (beside the shuffles: the read-out of the old state, the faded state)
+    f2 c0 = pack2(0.f, 0.f), c1 = c0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      c0 = fma2(s[i], t.q[i], c0);
+      c1 = fma2(s[4 + i], t.q[4 + i], c1);
+    }
+    a += __shfl_xor_sync(0xffffffffu, a, 2);
+    const f2 g2 = pack2(t.g, t.g);
+    f2 gs[DL_ROWS / 2];
+#pragma unroll
+    for (int i = 0; i < DL_ROWS / 2; ++i) gs[i] = fma2(g2, s[i], pack2(0.f, 0.f));
+    a += __shfl_xor_sync(0xffffffffu, a, 4);
+    const float bg = t.beta * t.g, bv = t.beta * t.v;
+    const float2 d0 = unpack2(c0), d1 = unpack2(c1);
+    const float c = t.g * ((d0.x + d0.y) + (d1.x + d1.y));
+    const float u = fmaf(-bg, a, bv);
+    const f2 u2 = pack2(u, u);
+#pragma unroll
+    for (int i = 0; i < DL_ROWS / 2; ++i) s[i] = fma2(t.k[i], u2, gs[i]);
+    x[r] = p == 0 ? fmaf(t.kq, u, c) : c;
+  };
+  int st = 0;
+  for (int g0 = 0; g0 < n; g0 += DR_GROUP, st = st + 1 == DL_STAGES ? 0 : st + 1) {
+    __syncthreads();
+    const int gn = min(DR_GROUP, n - g0);
+#pragma unroll 1
+    for (int r0 = 0; r0 < gn; r0 += 8) {
+      const uint32_t grp = ring + 4 * (st * DR_GROUP + r0) * TOK;
+      Token tk[2];
+      if (r0 + 8 <= gn) {
+        load(tk[0], grp);
+#pragma unroll
+        for (int r = 0; r < 8; ++r) take(tk[r & 1], r, tk[(r + 1) & 1], grp + 4 * (r + 1) * TOK, r + 1 < 8);
+      } else {
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+          x[r] = 0.f;
+          if (r0 + r < gn) {
+            load(tk[0], grp + 4 * r * TOK);
+            take(tk[0], r, tk[1], 0, false);
           }
         }
       }
+      // x[i] of the eight lanes summed; lane p gets token r0 + p's
 #pragma unroll
-      for (int jt = 0; jt < 7; ++jt)
-        if (jt < taps - 1) tail[(size_t)jt * C + c] = nv[jt];
+      for (int m = 0; m < 3; ++m) {
+        const bool up = (lane >> m) & 1;
+#pragma unroll
+        for (int i = 0; i < (4 >> m); ++i) {
+          const float keep = up ? x[2 * i + 1] : x[2 * i], send = up ? x[2 * i] : x[2 * i + 1];
+          x[i] = keep + __shfl_xor_sync(0xffffffffu, send, 1 << m);
+        }
+      }
+      if (live && r0 + p < gn) out[(size_t)(t0 + g0 + r0 + p) * hv + h * V + j] = x[0];
     }
   }
+#pragma unroll
+  for (int i = 0; i < DL_ROWS / 2; ++i) {
+    const int d = p * DL_ROWS + 2 * i;
+    if (!live || d >= D) continue;
+    const float2 v = unpack2(s[i]);
+    S[(size_t)d * V] = v.x;
+    S[(size_t)(d + 1) * V] = v.y;
+  }
+  if (taps > 1)
+    store_last_inputs(base + (size_t)H * D * V, proj, proj_is_bf16, proj_stride, t0, n, C, taps,
+                      (h * gridDim.x + blockIdx.x) * DL_WARPS * 32 + threadIdx.x, H * gridDim.x * DL_WARPS * 32);
 }
 
 template <typename T>
@@ -278,15 +462,16 @@ int g_delta_rows = 0;
 // Rows of a state column a lane of the scan holds (8, 16 or 32; 0: by the key width).  For measurements.
 TS_API void ts_set_delta_rows(int rows) { g_delta_rows = rows; }
 
-// ready: [T, 2 G D + H V + 2 H + G] 32-bit.  proj: [T, proj_stride] rows holding q at column 0, k at G D, v at
+// ready: [T, 2 G D + H V + 2 H + G] 32-bit, rows ready_stride apart.  proj: [T, proj_stride] rows holding q at column 0, k at G D, v at
 // 2 G D, then the gate (H V), b (H) and a (H).  conv_w: [2 G D + H V, taps] 32-bit.  state: [slots, state_stride].
-TS_API int ts_delta_prepare(float* ready, const void* proj, int proj_stride, const float* conv_w, const float* a_log,
+TS_API int ts_delta_prepare(float* ready, int ready_stride, const void* proj, int proj_stride, const float* conv_w, const float* a_log,
                             const float* dt_bias, const float* state, long long state_stride, const int* token_request,
                             const int* q_start, const int* slots, int T, int H, int G, int D, int V, int taps,
                             float unit_eps, int dtype, void* stream) {
   if (T <= 0) return 0;
   if (H <= 0 || G <= 0 || H % G || D <= 0 || V <= 0) TS_REFUSE(TS_ERR_SHAPE, "ts_delta_prepare: %d heads over %d of %d x %d", H, G, D, V);
   if (taps < 1 || taps > 8) TS_REFUSE(TS_ERR_LIMIT, "ts_delta_prepare: %d taps (1 to 8)", taps);
+  if (ready_stride < 2 * G * D + H * V + 2 * H + G) TS_REFUSE(TS_ERR_SHAPE, "ts_delta_prepare: rows of %d", ready_stride);
   const size_t smem = sizeof(float) * (size_t)2 * D;
   if (smem > 200 * 1024) TS_REFUSE(TS_ERR_LIMIT, "ts_delta_prepare: keys of %d", D);
   if (G + H > 65535) TS_REFUSE(TS_ERR_LIMIT, "ts_delta_prepare: %d heads", G + H);
@@ -299,7 +484,7 @@ TS_API int ts_delta_prepare(float* ready, const void* proj, int proj_stride, con
       if (e != cudaSuccess) TS_REFUSE((int)e, "ts_delta_prepare: shared memory %zu: %s", smem, cudaGetErrorString(e));   \
       configured = smem;                                                                                                 \
     }                                                                                                                    \
-    ts_launch(delta_prepare_kernel<TT>, dim3(T, G + H), dim3(128), smem, s, ready, (const TT*)proj, proj_stride, conv_w, a_log, \
+    ts_launch(delta_prepare_kernel<TT>, dim3(T, G + H), dim3(128), smem, s, ready, ready_stride, (const TT*)proj, proj_stride, conv_w, a_log, \
               dt_bias, state, (size_t)state_stride, token_request, q_start, slots, H, G, D, V, taps, unit_eps);          \
   } while (0)
   if (dtype == TS_F32) TS_DP(float);
@@ -309,9 +494,12 @@ TS_API int ts_delta_prepare(float* ready, const void* proj, int proj_stride, con
   TS_LAUNCH_CHECK();
 }
 
+// (from here on launched after its predecessor has ended: see ts_launch_late)
+constexpr int DL_LATE_TOKENS = 64;
+
 // out: [T, H V] 32-bit.  proj: the raw projection rows (for the filter's new last inputs).  max_q_len: the most tokens a
 // request of the launch brings (0: unknown); it sizes the staging buffers.
-TS_API int ts_delta_scan(float* out, const float* ready, const void* proj, int proj_stride, float* state,
+TS_API int ts_delta_scan(float* out, const float* ready, int ready_stride, const void* proj, int proj_stride, float* state,
                          long long state_stride, const int* q_start, const int* slots, int B, int H, int G, int D, int V,
                          int taps, int max_q_len, int dtype, void* stream) {
   if (B <= 0) return 0;
@@ -319,6 +507,27 @@ TS_API int ts_delta_scan(float* out, const float* ready, const void* proj, int p
   if (taps < 1 || taps > 8) TS_REFUSE(TS_ERR_LIMIT, "ts_delta_scan: %d taps (1 to 8)", taps);
   if (dtype != TS_F32 && dtype != TS_BF16) TS_REFUSE(TS_ERR_DTYPE, "ts_delta_scan: dtype %d", dtype);
   if (B > 65535 || H > 65535) TS_REFUSE(TS_ERR_LIMIT, "ts_delta_scan: %d requests / %d heads per launch", B, H);
+  const int W = ready_stride;
+  if (W < 2 * G * D + H * V + 2 * H + G) TS_REFUSE(TS_ERR_SHAPE, "ts_delta_scan: rows of %d", W);
+  const int vec4 = D % 4 == 0 && W % 4 == 0 && (G * D) % 4 == 0 && !((uintptr_t)ready & 15);
+  cudaStream_t s = (cudaStream_t)stream;
+  if (max_q_len != 1 && vec4 && V % 4 == 0 && D <= DL_KEYS && g_delta_rows == 0) {
+    constexpr size_t bytes = sizeof(float) * DL_STAGES * DR_GROUP * (2 * DL_KEYS + DL_COLS + 4);
+    static bool ready_to_go = false;
+    if (!ready_to_go) {
+      cudaError_t e = cudaFuncSetAttribute(delta_scan_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+      if (e != cudaSuccess) TS_REFUSE((int)e, "ts_delta_scan: shared memory %zu: %s", bytes, cudaGetErrorString(e));
+      ready_to_go = true;
+    }
+    const dim3 rows_grid(ceil_div(V, DL_COLS), H, B), rows_block((DL_WARPS + DL_LOAD_WARPS) * 32);
+    if (max_q_len >= DL_LATE_TOKENS)
+      ts_launch_late(delta_scan_rows_kernel, rows_grid, rows_block, bytes, s, out, ready, W, proj, proj_stride, dtype == TS_BF16 ? 1 : 0, state,
+                     (size_t)state_stride, q_start, slots, H, G, D, V, taps);
+    else
+      ts_launch(delta_scan_rows_kernel, rows_grid, rows_block, bytes, s, out, ready, W, proj, proj_stride, dtype == TS_BF16 ? 1 : 0, state,
+                (size_t)state_stride, q_start, slots, H, G, D, V, taps);
+    TS_LAUNCH_CHECK();
+  }
   // rows of a column a lane holds: few rows mean more lanes a column, so more warps to hide one another's latencies
   // (one warp a scheduler waits out every dependent instruction), but a longer shuffle tree
   // tokens staged at a time: no request of the launch brings more than max_q_len (0: unknown)
@@ -335,11 +544,8 @@ TS_API int ts_delta_scan(float* out, const float* ready, const void* proj, int p
   // spread over the chip, and every block stages the same q and k rows out of L2
   const int nwarps = max(1, min(8, min(ceil_div(16, CW), ceil_div(V, CW))));
   const int cols_block = nwarps * CW;
-  const int W = 2 * G * D + H * V + 2 * H + G;
-  const int vec4 = D % 4 == 0 && W % 4 == 0 && (G * D) % 4 == 0 && !((uintptr_t)ready & 15);
   const size_t smem = sizeof(float) * DR_STAGES * group * ((size_t)2 * P * (R + DR_PAD) + ((cols_block + 3 + 3) & ~3));
   if (smem > 200 * 1024) TS_REFUSE(TS_ERR_LIMIT, "ts_delta_scan: shared memory %zu", smem);
-  cudaStream_t s = (cudaStream_t)stream;
   dim3 grid(ceil_div(V, cols_block), H, B);
 #define TS_DS(RR)                                                                                                        \
   do {                                                                                                                   \
@@ -349,7 +555,7 @@ TS_API int ts_delta_scan(float* out, const float* ready, const void* proj, int p
       if (e != cudaSuccess) TS_REFUSE((int)e, "ts_delta_scan: shared memory %zu: %s", smem, cudaGetErrorString(e));      \
       configured = smem;                                                                                                 \
     }                                                                                                                    \
-    ts_launch(delta_scan_kernel<RR>, dim3(grid), dim3(nwarps * 32), smem, s, out, ready, proj, proj_stride,              \
+    ts_launch(delta_scan_kernel<RR>, dim3(grid), dim3(nwarps * 32), smem, s, out, ready, W, proj, proj_stride,           \
               dtype == TS_BF16 ? 1 : 0, state, (size_t)state_stride, q_start, slots, H, G, D, V, taps, P, vec4, group);  \
   } while (0)
   if (R == 32) TS_DS(32);

@@ -178,7 +178,7 @@ lightning_activate_kernel(float* __restrict__ ready, const T* __restrict__ proj,
 // two groups ahead, issued by two warps of their own (the copies of a group cost a computing warp a quarter of its time); a
 // column's 16 outputs of a group are summed over the lanes at once.  What bounds it: a warp alone on its scheduler (portions of
 // one request have 768 columns for 592 schedulers), about 35 instructions and 125 cycles a token.  2,048 tokens, 6 heads of
-// 128 x 128, activation included: 350 -> 198 us (before: a thread a column and 8 rows, a block-wide sum of its parts, the
+// 128 x 128, activation included: 350 -> 135 us (before: a thread a column and 8 rows, a block-wide sum of its parts, the
 // activation in every block of 16 columns).
 constexpr int LL_WARPS = 4, LL_LOAD_WARPS = 2, LL_COLS = 2 * LL_WARPS, LL_STAGES = 3;
 

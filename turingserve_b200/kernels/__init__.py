@@ -68,7 +68,7 @@ class LazyProduct:
 class CudaOps:
     """ctypes front of ``libturingserve_b200.so``."""
 
-    ABI = 18
+    ABI = 19
     UNSUPPORTED = -4            # a kernel's refusal of a shape or layout another kernel takes
 
     def __init__(self, lib_path: str) -> None:
@@ -131,8 +131,8 @@ class CudaOps:
             "ts_act_mul": [P, P, I, I, I, I, I, P],
             "ts_rope_pairs_write": [P, I, I, I, P, P, F, I, P, P, P, I, I, I, I, I, I, I, P],
             "ts_moe_gather": [P, P, P, P, I, I, I, I, P],
-            "ts_delta_prepare": [P, P, I, P, P, P, P, ctypes.c_longlong, P, P, P, I, I, I, I, I, I, F, I, P],
-            "ts_delta_scan": [P, P, P, I, P, ctypes.c_longlong, P, P, I, I, I, I, I, I, I, I, P],
+            "ts_delta_prepare": [P, I, P, I, P, P, P, P, ctypes.c_longlong, P, P, P, I, I, I, I, I, I, F, I, P],
+            "ts_delta_scan": [P, P, I, P, I, P, ctypes.c_longlong, P, P, I, I, I, I, I, I, I, I, P],
             "ts_head_gated_rmsnorm": [P, P, P, I, P, I, F, I, I, I, I, P],
             "ts_attention_biased": [P, I, I, P, I, I, P, P, P, P, P, I, I, I, I, I, I, I, I, F, F, P, I, I, P, P, I, I, P, I, P, P, I, P],
             "ts_attention_biased_mma": [P, I, I, P, I, I, P, P, P, P, P, I, I, I, I, I, I, I, I, F, F, P, I, I, P, P, I, I, P, I, P, P, I, P],
@@ -710,12 +710,12 @@ class CudaOps:
     # -- the gated delta rule --------------------------------------------------------------------------------------
     def delta_prepare(self, ready, proj, conv_w, a_log, dt_bias, state, step, H: int, G: int, D: int, V: int, taps: int,
                       unit_eps: float) -> None:
-        """ready (float32 [T, 2GD + HV + 2H + G]) = [q | k | v | g | beta | k.q] of every token: the columns q, k, v of
+        """ready (float32 [T, 2GD + HV + 2H + G], rows contiguous) = [q | k | v | g | beta | k.q] of every token: the columns q, k, v of
         ``proj`` through their causal filters (``conv_w`` float32 [2GD + HV, taps]; inputs before the step's first
         token come from the request's state slot) and SiLU, q and k to unit length per head and q / sqrt(D),
         g = exp(-exp(a_log) softplus(a + dt_bias)), beta = sigmoid(b); b and a are the last 2H columns of ``proj``."""
         T = proj.shape[0]
-        self._check(self.lib.ts_delta_prepare(_ptr(ready), _ptr(proj), proj.stride(0), _ptr(conv_w), _ptr(a_log),
+        self._check(self.lib.ts_delta_prepare(_ptr(ready), ready.stride(0), _ptr(proj), proj.stride(0), _ptr(conv_w), _ptr(a_log),
                                               _ptr(dt_bias), _ptr(state), state.stride(0), _ptr(step.token_request),
                                               _ptr(step.q_start), _ptr(step.state_slots), T, H, G, D, V, taps,
                                               float(unit_eps), _code(proj.dtype), self._stream()), "delta_prepare")
@@ -724,8 +724,8 @@ class CudaOps:
         """out (float32 [T, HV]): the recurrence over the rows ``delta_prepare`` made; ``state`` (float32
         [slots, HDV + (taps - 1)(2GD + HV)]) is read and left updated at each request's slot, the filter's last
         inputs (from ``proj``) included."""
-        self._check(self.lib.ts_delta_scan(_ptr(out), _ptr(ready), _ptr(proj), proj.stride(0), _ptr(state), state.stride(0),
-                                           _ptr(step.q_start), _ptr(step.state_slots), step.num_requests, H, G, D, V, taps,
+        self._check(self.lib.ts_delta_scan(_ptr(out), _ptr(ready), ready.stride(0), _ptr(proj), proj.stride(0), _ptr(state),
+                                           state.stride(0), _ptr(step.q_start), _ptr(step.state_slots), step.num_requests, H, G, D, V, taps,
                                            int(getattr(step, "max_q_len", 0) or 0), _code(proj.dtype), self._stream()), "delta_scan")
 
     def head_gated_rmsnorm(self, out, x, gate, weight, eps: float, H: int, V: int) -> None:

@@ -60,8 +60,9 @@ class DeltaRule(Mixer):
         H, G, D, V = self.H, self.G, self.D, self.V
         proj = torch.empty((T, self.channels + self.hv + 2 * H), dtype=x.dtype, device=x.device)
         ops.linear(proj, x, self.w_in)
-        # 32-bit rows [q | k | v | g | beta | k.q] for the scan
-        ready = torch.empty((T, self.channels + 2 * H + G), dtype=torch.float32, device=x.device)
+        # 32-bit rows [q | k | v | g | beta | k.q] for the scan, each on a 16-byte boundary (it fetches 16 bytes at a time then)
+        n_ready = self.channels + 2 * H + G
+        ready = torch.empty((T, -(-n_ready // 4) * 4), dtype=torch.float32, device=x.device)[:, :n_ready]
         ops.delta_prepare(ready, proj, self.conv, self.a_log, self.dt_bias, state, step, H, G, D, V, self.taps,
                           self.unit_eps)
         o = torch.empty((T, self.hv), dtype=torch.float32, device=x.device)
