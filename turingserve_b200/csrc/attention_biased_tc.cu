@@ -44,7 +44,7 @@ constexpr int SOFTMAX_THREADS = 2 * TQ;
 constexpr int THREADS = SOFTMAX_THREADS + 96;
 constexpr int MMA_WARP = SOFTMAX_THREADS / 32, LOAD_WARP = MMA_WARP + 1;    // (two loading warps)
 
-template <int DK, int DV, int TK, bool V_IN_K, int QT>
+template <int DK, int DV, int TK, bool V_IN_K, int QT, bool MAPS = false>
 struct Plan {
   static constexpr int KT = TK / 2, UNITS = TK / UNIT;     // keys of a tile per softmax thread; units of loading
   static constexpr uint32_t BLK_KV = TK * 128;             // bytes of 64 columns of a key / value tile
@@ -63,6 +63,7 @@ struct Plan {
 
 struct Args {
   bf16* out;
+  float* out32;            // two score maps a head: rows [T, H, 2, DV] in place of `out`
   const bf16* q;
   const int* block_tables;
   const int* q_start;
@@ -74,6 +75,7 @@ struct Args {
   int run;                 // pages per tile when a tile is several pages (then the run maps are valid), else 0
   float scale, softcap;
   int window, block_of, keep, v_chunks;
+  int min_rows;            // requests of so many rows or fewer are another kernel's
   AttnFinish fin;
   int* status;
 };
@@ -83,12 +85,12 @@ template <int N> using Int = std::integral_constant<int, N>;
 // The lowest n bits (n < 0: none; n > 31: all).
 __device__ __forceinline__ uint32_t below(int n) { return n <= 0 ? 0u : (n >= 32 ? 0xffffffffu : (1u << n) - 1u); }
 
-template <int DK, int DV, int TK, bool V_IN_K, int QT>
-__global__ void __launch_bounds__(THREADS, Plan<DK, DV, TK, V_IN_K, QT>::PER_SM)
+template <int DK, int DV, int TK, bool V_IN_K, int QT, bool MAPS = false>
+__global__ void __launch_bounds__(THREADS, Plan<DK, DV, TK, V_IN_K, QT, MAPS>::PER_SM)
 attention_biased_tc_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constant__ CUtensorMap v_map,
                            const __grid_constant__ CUtensorMap k_run_map, const __grid_constant__ CUtensorMap v_run_map,
                            const Args a) {
-  using PL = Plan<DK, DV, TK, V_IN_K, QT>;
+  using PL = Plan<DK, DV, TK, V_IN_K, QT, MAPS>;
   constexpr int KB = PL::KB, VB = PL::VB, STAGES = PL::STAGES, KT = PL::KT, UNITS = PL::UNITS;
   constexpr uint32_t BLK_KV = PL::BLK_KV;
   constexpr uint32_t K_BYTES = PL::K_BYTES, V_BYTES = PL::V_BYTES, S_COL = PL::S_COL, O_COL = PL::O_COL, Q_COL = PL::Q_COL;
@@ -111,7 +113,8 @@ attention_biased_tc_kernel(const __grid_constant__ CUtensorMap k_map, const __gr
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   float* max_x = reinterpret_cast<float*>(tmem_slot + 4);  // [tile & 1][2 halves][128 rows]
 
-  const int b = blockIdx.z, kvh = blockIdx.y;
+  // (two score maps a head, MAPS: a key row is [map 0 | map 1], a query [map 0 | map 1] too; a block takes one of them)
+  const int b = blockIdx.z, kvh = MAPS ? blockIdx.y >> 1 : blockIdx.y, map_col = MAPS ? (blockIdx.y & 1) * DK : 0;
   const int chunk = blockIdx.x % a.v_chunks, tile = blockIdx.x / a.v_chunks;
   const int G = a.H / a.KVH;
   const int qs = a.q_start[b];
@@ -119,7 +122,7 @@ attention_biased_tc_kernel(const __grid_constant__ CUtensorMap k_map, const __gr
   const int seq_len = a.seq_lens[b];
   const int n_rows = q_len * G;
   const int n_row_tiles = (n_rows + TQ - 1) / TQ;
-  if (tile >= n_row_tiles) return;
+  if (tile >= n_row_tiles || n_rows <= a.min_rows) return;
   const int row0 = (n_row_tiles - 1 - tile) * TQ;          // longest tiles first
   const int tid = threadIdx.x, warp = tid >> 5;
   const int prefix = seq_len - q_len;
@@ -191,7 +194,7 @@ attention_biased_tc_kernel(const __grid_constant__ CUtensorMap k_map, const __gr
       const int count = first ? (V_IN_K ? KB - VB : KB) : VB;
       const int v0 = chunk * VB;
       auto block = [&](int i) { return V_IN_K ? (first ? (i < v0 ? i : i + VB) : v0 + i) : i; };
-      const int col0 = (V_IN_K || first) ? 0 : chunk * DV;   // (the first column the block wants of a row)
+      const int col0 = V_IN_K ? 0 : (first ? map_col : chunk * DV);   // (the first column the block wants of a row)
       const CUtensorMap* map = V_IN_K || first ? &k_map : &v_map;
       const CUtensorMap* rmap = V_IN_K || first ? &k_run_map : &v_run_map;
       unsigned char* ring = V_IN_K || first ? k_s : v_s;
@@ -286,7 +289,7 @@ attention_biased_tc_kernel(const __grid_constant__ CUtensorMap k_map, const __gr
           const uint64_t vd = v_desc + (kk * 16 * 128 >> 4);
           const uint32_t hi = p + kk / (KT / 16) * KT + kk % (KT / 16) * 8;
           umma_ts(tmem + O_COL, hi, vd, idesc, (t > 0 || kk > 0) ? 1u : 0u);
-          umma_ts(tmem + O_COL, hi + KT / 2, vd, idesc, 1u);
+          if (!MAPS) umma_ts(tmem + O_COL, hi + KT / 2, vd, idesc, 1u);
         }
         umma_commit(&empty_v[t % STAGES]);
         umma_commit(bar_pv);
@@ -336,7 +339,7 @@ attention_biased_tc_kernel(const __grid_constant__ CUtensorMap k_map, const __gr
     // Query rows: 64-column blocks 0 .. QT - 1 -> tensor memory (lane = row, a 32-bit column = two neighbouring query columns),
     // the others -> shared memory, K-major with the 128-byte swizzle (16-byte chunk c of row r at c ^ (r & 7)); of a row's two
     // threads each takes every second block
-    const bf16* src = a.q + (size_t)(qs + tok) * a.q_ts + (size_t)(kvh * G + g) * a.q_hs;
+    const bf16* src = a.q + (size_t)(qs + tok) * a.q_ts + (size_t)(kvh * G + g) * a.q_hs + map_col;
 #pragma unroll 1
     for (int blk = hh; blk < KB; blk += 2) {
       uint32_t w[32];
@@ -452,11 +455,13 @@ attention_biased_tc_kernel(const __grid_constant__ CUtensorMap k_map, const __gr
           rs[i & 1] += p0 + p1;
           const __nv_bfloat162 h2 = __floats2bfloat162_rn(p0, p1);
           sv[i] = *reinterpret_cast<const uint32_t*>(&h2);
+          if (MAPS) continue;
           const __nv_bfloat162 l2 = __floats2bfloat162_rn(p0 - __uint_as_float(sv[i] << 16), p1 - __uint_as_float(sv[i] & 0xffff0000u));
           lw[i] = *reinterpret_cast<const uint32_t*>(&l2);
         }
 #pragma unroll
-        for (int i = 0; i < KT / 2; ++i) sv[KT / 2 + i] = lw[i];
+        for (int i = 0; i < KT / 2; ++i)
+          if (!MAPS) sv[KT / 2 + i] = lw[i];
         return rs[0] + rs[1];
       };
       // The reference moves rarely once a row has one: the exponentials are taken against the present one while the other
@@ -496,7 +501,7 @@ attention_biased_tc_kernel(const __grid_constant__ CUtensorMap k_map, const __gr
         }
       }
 #pragma unroll
-      for (int h = 0; h < KT / 32; ++h)                    // over this thread's own scores
+      for (int h = 0; h < (MAPS ? KT / 64 : KT / 32); ++h) // over this thread's own scores
         tmem_st32(s_addr + hh * KT + h * 32, reinterpret_cast<uint32_t(&)[32]>(sv[h * 32]));
       tmem_wait_st();                                      // P (and a rescaled O) are in tensor memory
       tc_fence_before();
@@ -543,6 +548,17 @@ attention_biased_tc_kernel(const __grid_constant__ CUtensorMap k_map, const __gr
           for (int i = 0; i < 16; ++i) x[i] = y[i] = 0u;
         }
         if (!row_ok) continue;
+        if (MAPS) {
+          float* dst32 = a.out32 + (size_t)(qs + tok) * a.out_ts + (size_t)head * a.out_hs + (MAPS && map_col ? DV : 0);
+#pragma unroll
+          for (int i = 0; i < 16; i += 4) {
+            *reinterpret_cast<float4*>(dst32 + c + i) = make_float4(__uint_as_float(x[i]) * inv, __uint_as_float(x[i + 1]) * inv,
+                                                                    __uint_as_float(x[i + 2]) * inv, __uint_as_float(x[i + 3]) * inv);
+            *reinterpret_cast<float4*>(dst32 + DV / 2 + c + i) = make_float4(__uint_as_float(y[i]) * inv, __uint_as_float(y[i + 1]) * inv,
+                                                                             __uint_as_float(y[i + 2]) * inv, __uint_as_float(y[i + 3]) * inv);
+          }
+          continue;
+        }
         if (a.fin.out_freq != nullptr) {                   // (whole value rows only)
 #pragma unroll
           for (int i = 0; i < 16; ++i) {
@@ -576,19 +592,49 @@ attention_biased_tc_kernel(const __grid_constant__ CUtensorMap k_map, const __gr
   }
 }
 
-template <int DK, int DV, int TK, bool V_IN_K, int QT>
+template <int DK, int DV, int TK, bool V_IN_K, int QT, bool MAPS = false>
 int launch(dim3 grid, cudaStream_t stream, const CUtensorMap& k_map, const CUtensorMap& v_map, const CUtensorMap& k_run,
            const CUtensorMap& v_run, const Args& a) {
-  using PL = Plan<DK, DV, TK, V_IN_K, QT>;
+  using PL = Plan<DK, DV, TK, V_IN_K, QT, MAPS>;
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(attention_biased_tc_kernel<DK, DV, TK, V_IN_K, QT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(attention_biased_tc_kernel<DK, DV, TK, V_IN_K, QT, MAPS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)PL::SMEM);
     if (e != cudaSuccess) TS_REFUSE((int)e, "ts_attention_biased_tc: shared memory %zu: %s", PL::SMEM, cudaGetErrorString(e));
     configured = true;
   }
-  ts_launch(attention_biased_tc_kernel<DK, DV, TK, V_IN_K, QT>, grid, dim3(THREADS), PL::SMEM, stream, k_map, v_map, k_run, v_run, a);
+  ts_launch(attention_biased_tc_kernel<DK, DV, TK, V_IN_K, QT, MAPS>, grid, dim3(THREADS), PL::SMEM, stream, k_map, v_map, k_run, v_run, a);
   TS_LAUNCH_CHECK();
+}
+
+// Two score maps a head (attention_diff.cu): every map of every kv head is a block's work like any other head's, with keys 64
+// columns of the 128-wide key row; the weights are one bfloat16, as in attention_diff_mma.cu, so one product; the two outputs
+// stay in 32-bit until the kernel below has joined them.  2,048 tokens, 12 heads over 2: 154 -> 51 us with the join, whole mixer 193 -> 90 us.
+// out[t, h] = out_scale * rms_norm(a_0 - lambda a_1) of the two maps' outputs, a warp a head; tokens of requests of min_rows
+// rows or fewer are left alone.
+template <int V>
+__global__ void __launch_bounds__(128)
+join_maps_kernel(bf16* __restrict__ out, const float* __restrict__ maps, const int* __restrict__ token_request,
+                 const int* __restrict__ q_start, int H, int G, int min_rows, float lambda, float eps, float out_scale) {
+  pdl_launch_dependents();
+  pdl_wait();
+  constexpr int PER = V / 32;
+  const int t = blockIdx.x, h = blockIdx.y * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const int b = token_request[t];
+  if (h >= H || (q_start[b + 1] - q_start[b]) * G <= min_rows) return;
+  const float* src = maps + ((size_t)t * H + h) * 2 * V + lane * PER;
+  float o[PER], ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < PER; i += 2) {
+    const float2 x = *reinterpret_cast<const float2*>(src + i), y = *reinterpret_cast<const float2*>(src + V + i);
+    o[i] = x.x - lambda * y.x;
+    o[i + 1] = x.y - lambda * y.y;
+    ss = fmaf(o[i], o[i], fmaf(o[i + 1], o[i + 1], ss));
+  }
+  const float f = out_scale / sqrtf(warp_sum(ss) / (float)V + eps);
+  bf16* dst = out + ((size_t)t * H + h) * V + lane * PER;
+#pragma unroll
+  for (int i = 0; i < PER; i += 2) *reinterpret_cast<__nv_bfloat162*>(dst + i) = __floats2bfloat162_rn(o[i] * f, o[i + 1] * f);
 }
 
 // which instance takes (key width, value width, values inside the key rows): 0 none
@@ -642,6 +688,8 @@ TS_API int ts_attention_biased_tc(void* out, int out_ts, int out_hs, const void*
     TS_REFUSE(TS_ERR_UNSUPPORTED, "ts_attention_biased_tc: cuTensorMapEncodeTiled (runs of pages) failed");
   Args a;
   a.out = (bf16*)out;
+  a.out32 = nullptr;
+  a.min_rows = 0;
   a.q = (const bf16*)q;
   a.block_tables = block_tables;
   a.q_start = q_start;
@@ -674,4 +722,70 @@ TS_API int ts_attention_biased_tc(void* out, int out_ts, int out_hs, const void*
   if (inst == 2) return launch<128, 128, 128, false, 0>(grid, s, k_map, v_map, k_run, v_run, a);
   if (inst == 3) return launch<576, 256, 64, true, 4>(grid, s, k_map, v_map, k_run, v_run, a);
   return launch<320, 256, 64, true, 0>(grid, s, k_map, v_map, k_run, v_run, a);
+}
+
+TS_API int ts_attention_maps_tc_supported(int H, int KVH, int D, int V, int page, int dtype) {
+  return dtype == TS_BF16 && KVH > 0 && H % KVH == 0 && page >= BOX_ROWS && page % BOX_ROWS == 0 && D == 64 && (V == 64 || V == 128);
+}
+
+// Attention with two score maps a head (see attention_diff.cu) for the portions of more than min_rows query rows: maps [T, H, 2,
+// V] 32-bit is work memory.  q: rows of proj, heads of 2 D; key rows of 2 D, value rows of V; out [T, H V].
+TS_API int ts_attention_maps_tc(void* out, float* maps, const void* proj, int proj_stride, const void* k_cache, const void* v_cache,
+                                const int* block_tables, const int* q_start, const int* seq_lens, const int* token_request, int B,
+                                int T, int table_width, int max_q_len, int H, int KVH, int D, int V, int page, int num_pages,
+                                float scale, float lambda, float eps, float out_scale, int min_rows, void* stream) {
+  if (B <= 0 || max_q_len <= 0 || T <= 0) return 0;
+  if (!ts_attention_maps_tc_supported(H, KVH, D, V, page, TS_BF16))
+    TS_REFUSE(TS_ERR_UNSUPPORTED, "ts_attention_maps_tc: H=%d KVH=%d maps of %d values %d pages of %d", H, KVH, D, V, page);
+  if ((proj_stride % 8) || (((uintptr_t)proj | (uintptr_t)out | (uintptr_t)maps | (uintptr_t)k_cache | (uintptr_t)v_cache) & 15))
+    TS_REFUSE(TS_ERR_UNSUPPORTED, "ts_attention_maps_tc: rows must start on 16-byte boundaries");
+  if (B > 65535 || KVH > 32767) TS_REFUSE(TS_ERR_LIMIT, "ts_attention_maps_tc: %d requests / %d kv heads", B, KVH);
+  const long long rows = (long long)num_pages * KVH * page;
+  if (num_pages <= 0 || rows > 0x7fffffffLL) TS_REFUSE(TS_ERR_UNSUPPORTED, "ts_attention_maps_tc: cache of %lld rows", rows);
+  int* status = ts_attn_status_word();
+  if (status == nullptr) TS_REFUSE(TS_ERR_LIMIT, "ts_attention_maps_tc: no status word");
+  const int box = page % 64 == 0 ? 64 : (page % 32 == 0 ? 32 : 16);
+  const int run = (page < UNIT && box == page) ? UNIT / page : 0;
+  CUtensorMap k_map, v_map, k_run, v_run;
+  if (!tensor_map(&k_map, k_cache, (int)rows, 2 * D, box) || !tensor_map(&v_map, v_cache, (int)rows, V, box))
+    TS_REFUSE(TS_ERR_UNSUPPORTED, "ts_attention_maps_tc: cuTensorMapEncodeTiled failed");
+  k_run = k_map;
+  v_run = v_map;
+  if (run > 1 && (!run_map(&k_run, k_cache, num_pages, KVH, page, run, 2 * D) || !run_map(&v_run, v_cache, num_pages, KVH, page, run, V)))
+    TS_REFUSE(TS_ERR_UNSUPPORTED, "ts_attention_maps_tc: cuTensorMapEncodeTiled (runs of pages) failed");
+  Args a = {};
+  a.out32 = maps;
+  a.q = (const bf16*)proj;
+  a.block_tables = block_tables;
+  a.q_start = q_start;
+  a.seq_lens = seq_lens;
+  a.out_ts = H * 2 * V;
+  a.out_hs = 2 * V;
+  a.q_ts = proj_stride;
+  a.q_hs = 2 * D;
+  a.table_width = table_width;
+  a.H = H;
+  a.KVH = KVH;
+  a.page = page;
+  a.box = box;
+  a.run = run > 1 ? run : 0;
+  a.scale = scale;
+  a.v_chunks = 1;
+  a.min_rows = min_rows;
+  a.status = status;
+  const int G = H / KVH;
+  const dim3 grid(ceil_div(max_q_len * G, TQ), 2 * KVH, B), join(T, ceil_div(H, 4));
+  cudaStream_t s = (cudaStream_t)stream;
+  int rc;
+  if (V == 128) {
+    rc = launch<64, 128, 128, false, 0, true>(grid, s, k_map, v_map, k_run, v_run, a);
+    if (rc == 0)
+      ts_launch(join_maps_kernel<128>, join, dim3(128), 0, s, (bf16*)out, maps, token_request, q_start, H, G, min_rows, lambda, eps, out_scale);
+  } else {
+    rc = launch<64, 64, 128, false, 0, true>(grid, s, k_map, v_map, k_run, v_run, a);
+    if (rc == 0)
+      ts_launch(join_maps_kernel<64>, join, dim3(128), 0, s, (bf16*)out, maps, token_request, q_start, H, G, min_rows, lambda, eps, out_scale);
+  }
+  if (rc != 0) return rc;
+  TS_LAUNCH_CHECK();
 }

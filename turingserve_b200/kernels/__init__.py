@@ -137,6 +137,8 @@ class CudaOps:
             "ts_attention_biased": [P, I, I, P, I, I, P, P, P, P, P, I, I, I, I, I, I, I, I, F, F, P, I, I, P, P, I, I, P, I, P, P, I, P],
             "ts_attention_biased_mma": [P, I, I, P, I, I, P, P, P, P, P, I, I, I, I, I, I, I, I, F, F, P, I, I, P, P, I, I, P, I, P, P, I, P],
             "ts_attention_biased_tc": [P, I, I, P, I, I, P, P, P, P, P, I, I, I, I, I, I, I, I, I, F, F, P, I, I, P, I, P, P, I, P],
+            "ts_attention_maps_tc": [P, P, P, I, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, F, F, F, F, I, P],
+            "ts_attention_maps_tc_supported": [I, I, I, I, I, I],
             "ts_rope_headnorm_write": [P, I, I, I, P, P, I, I, F, P, P, P, I, I, I, I, I, I, I, P, I, P],
             "ts_rope_headnorm_write_supports_parts": [I, I, I, I],
             "ts_rms_rows": [P, P, I, I, I, P, F, I, I, P],
@@ -672,6 +674,9 @@ class CudaOps:
                                               _ptr(slots), proj.shape[0], KVH, DK, DV, page_size, _code(proj.dtype),
                                               self._stream()), "kv_write_pair")
 
+    # portions (more than 16 query rows a kv head) that reach over at least this many keys go to the tcgen05 kernel
+    diff_tc_keys = int(os.environ.get("TURINGSERVE_B200_DIFF_TC_KEYS", "128"))
+
     def attention_diff(self, out, proj, k_cache, v_cache, block_tables, step, H: int, KVH: int, D: int, V: int,
                        page_size: int, scale: float, lam: float, eps: float, out_scale: float) -> None:
         """out [T, H V] = out_scale * rmsnorm_head(a1 - lam a2): two causal softmax maps a head (queries in
@@ -689,6 +694,22 @@ class CudaOps:
             G = H // KVH
             kinds = 3 if q_lens is None else ((1 if any(n * G <= 16 for n in q_lens) else 0)
                                               | (2 if any(n * G > 16 for n in q_lens) else 0))
+            token_request = getattr(step, "token_request", None)
+            if (kinds & 2 and q_lens is not None and token_request is not None and self.use_tc_attention
+                    and step.max_seq_len >= self.diff_tc_keys
+                    and self.lib.ts_attention_maps_tc_supported(H, KVH, D, V, page_size, _code(proj.dtype))):
+                maps = torch.empty((out.shape[0], H, 2, V), dtype=torch.float32, device=out.device)
+                rc = self.lib.ts_attention_maps_tc(
+                    _ptr(out), _ptr(maps), _ptr(proj), proj.stride(0), _ptr(k_cache), _ptr(v_cache), _ptr(block_tables),
+                    _ptr(step.q_start), _ptr(step.seq_lens), _ptr(token_request), B, out.shape[0], block_tables.shape[1],
+                    step.max_q_len, H, KVH, D, V, page_size, k_cache.shape[0], float(scale), float(lam), float(eps),
+                    float(out_scale), 16, self._stream())
+                if rc != self.UNSUPPORTED:
+                    self.launches += 1
+                    self._check(rc, "attention_maps_tc")
+                    kinds &= 1                          # (requests of at most 16 rows are left)
+                    if kinds == 0:
+                        return
             scratch = counters = None
             if splits > 1:
                 scratch = self._buffer("diff_scratch", self.lib.ts_attention_diff_mma_scratch_floats(B, KVH, V, splits),
