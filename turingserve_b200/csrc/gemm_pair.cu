@@ -20,6 +20,14 @@
 // epilogue warp of either block).  Every wait is bounded: a barrier that does not flip in time leaves a
 // code in the status word, the block stops, and still meets its peer at the last cluster barrier and frees
 // its tensor memory.  No TMA multicast.
+//
+// GROUPED: the rows of x come sorted by expert and every expert has weights of its own (w [E, N, K]): the tiles along the rows
+// are those of each expert's group, counted on the device from the groups' offsets, so nothing is read back by the host and
+// the launch may sit in a captured step.  A tile's last rows may be the next group's: computed and not stored.  The epilogue
+// applies a one-input activation, the clamped gated unit (gate and up columns taking turns) or leaves 32-bit rows.  2,048
+// tokens, 8 experts of 1,536 x 2,688, top 2, the whole feed-forward with its shared expert: 364 us with a library product an
+// expert (238 us of kernels, and the host that launched them) -> 213 us.
+#include "activations.cuh"
 #include "common.cuh"
 #include "tc_utils.cuh"
 
@@ -40,11 +48,14 @@ template <int BN> struct PairTile {
   static constexpr uint32_t B_BYTES = HALF_N * BK * 2, STAGE_BYTES = PA_BYTES + B_BYTES;
   static constexpr int STAGES = BN == 256 ? 6 : (BN == 192 ? 7 : 8);
   static constexpr size_t SMEM = 1024 + (size_t)STAGES * STAGE_BYTES + (2 * STAGES + 4) * 8 + 16;
+  static constexpr size_t GROUPED_SMEM = SMEM + 2 * 257 * 4;
   // bf16 x bf16 -> f32, M = 256 over the pair, N = BN, both operands K-major
   static constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
 };
 
-enum PairEpilogue : int { EPI_PLAIN = 0, EPI_GATED = 1, EPI_QKV = 2 };
+enum PairEpilogue : int { EPI_PLAIN = 0, EPI_GATED = 1, EPI_QKV = 2, EPI_GROUP = 3, EPI_GROUP_GLU = 4, EPI_GROUP_F32 = 5 };
+constexpr bool grouped_epilogue(int epi) { return epi >= EPI_GROUP; }
+constexpr int MAX_EXPERTS = 256;
 
 struct PairArgs {
   bf16* out;              // PLAIN: [M, N]; GATED: [M, N / 2]
@@ -62,6 +73,16 @@ struct PairArgs {
   bf16* k_cache;
   bf16* v_cache;
   int page, H, KVH, D;
+  // GROUPED: M rows in all; expert e's are [offsets[e], offsets[e + 1])
+  const int* offsets;
+  int experts, act;
+  float* out32;           // GROUP_F32: [M, N]
+  TsGlu glu;              // GROUP_GLU: out [M, N / 2]
+};
+
+// The groups' offsets and the first row tile of each group (GROUPED), behind the barriers.
+struct PairGroups {
+  int row[MAX_EXPERTS + 1], tile[MAX_EXPERTS + 1];
 };
 
 __device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* map, int x, int y, uint32_t leader_bar) {
@@ -111,7 +132,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
   unsigned rank;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
   const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
-  const int tiles = args.tiles_m * args.tiles_n;
+  constexpr bool GROUPED = grouped_epilogue(EPI);
+  PairGroups* groups = reinterpret_cast<PairGroups*>(tmem_slot + 4);
   const int n_kb = (args.K + BK - 1) / BK;
 
   if (threadIdx.x == 0) {
@@ -130,18 +152,45 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(ACC_COLS) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
+  if constexpr (GROUPED) {
+    pdl_wait();                                    // the offsets are the kernel's before
+    for (int e = threadIdx.x; e <= args.experts; e += PAIR_THREADS) groups->row[e] = args.offsets[e];
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      int n = 0;
+      for (int e = 0; e < args.experts; ++e) {
+        groups->tile[e] = n;
+        n += (groups->row[e + 1] - groups->row[e] + 2 * PM - 1) / (2 * PM);
+      }
+      groups->tile[args.experts] = n;
+    }
+  }
   tc_fence_before();
   __syncthreads();
   cluster_sync_all();                              // the peer's barriers exist before anything is sent to them
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  const int tiles_m = GROUPED ? groups->tile[args.experts] : args.tiles_m;
+  const int tiles = tiles_m * args.tiles_n;
+  // a tile's first row, the end of its rows, its weights' first row
+  struct Place { int row, end, row_w; };
+  auto place_of = [&](int tile) {
+    const int tm = tile % tiles_m, tn = tile / tiles_m;
+    if constexpr (!GROUPED) {
+      return Place{tm * 2 * PM, args.M, tn * PN};
+    } else {
+      int e = 0;
+      while (tm >= groups->tile[e + 1]) ++e;       // (groups without rows have no tile)
+      return Place{groups->row[e] + (tm - groups->tile[e]) * 2 * PM, groups->row[e + 1], e * args.N + tn * PN};
+    }
+  };
 
   if (warp == 0) {
     if (lane == 0) {
       // The weights do not depend on the kernel before this one: those of the first stages are on their
       // way before this block waits for its predecessor; the activations follow after the wait.
-      const int early = pair < tiles ? min(n_kb, PAIR_STAGES) : 0;
-      {
+      const int early = !GROUPED && pair < tiles ? min(n_kb, PAIR_STAGES) : 0;
+      if constexpr (!GROUPED) {
         const int row_w = (pair / args.tiles_m) * PN + (int)rank * HALF_N;
         for (int kb = 0; kb < early; ++kb) {
           if (rank == 0) mbar_expect_tx(&full[kb], 2 * PSTAGE_BYTES);
@@ -152,8 +201,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
       int it = 0;
       bool ok = true;
       for (int tile = pair; tile < tiles && ok; tile += pairs) {
-        const int tm = tile % args.tiles_m, tn = tile / args.tiles_m;
-        const int row_x = tm * 2 * PM + (int)rank * PM, row_w = tn * PN + (int)rank * HALF_N;
+        const Place at = place_of(tile);
+        const int row_x = at.row + (int)rank * PM, row_w = at.row_w + (int)rank * HALF_N;
         for (int kb = 0; kb < n_kb; ++kb, ++it) {
           const int s = it % PAIR_STAGES;
           const uint32_t ph = (it / PAIR_STAGES) & 1;
@@ -206,9 +255,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     int t = 0;
     bool ok = true;
     for (int tile = pair; tile < tiles && ok; tile += pairs, ++t) {
-      const int tm = tile % args.tiles_m, tn = tile / args.tiles_m;
+      const Place at = place_of(tile);
+      const int tn = tile / tiles_m;
       const int b = t & 1;
-      const int row = tm * 2 * PM + (int)rank * PM + q * 32 + lane;
+      const int row = at.row + (int)rank * PM + q * 32 + lane;
       // QKV: what the rotation needs of this thread's token is fetched while the products run: position, slot,
       // and the 32 cosines and sines of this warp's pairs (the same in every head), rounded to bfloat16 as
       // they are used and packed two to a register.
@@ -332,6 +382,41 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             }
           }
         }
+      } else if constexpr (GROUPED) {
+#pragma unroll 1
+        for (int c = part * 32; c < PN; c += 64) {
+          uint32_t a[32];
+          tmem_ld32(taddr + c, a);
+          tmem_wait_ld();
+          if (row >= at.end) continue;
+#pragma unroll
+          for (int v = 0; v < 4; ++v) {
+            const int col = tn * PN + c + v * 8;
+            if (col >= args.N) break;
+            float f[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) f[i] = __uint_as_float(a[v * 8 + i]);
+            if constexpr (EPI == EPI_GROUP_F32) {
+              float4* dst = reinterpret_cast<float4*>(args.out32 + (size_t)row * args.N + col);
+              dst[0] = make_float4(f[0], f[1], f[2], f[3]);
+              dst[1] = make_float4(f[4], f[5], f[6], f[7]);
+            } else if constexpr (EPI == EPI_GROUP_GLU) {
+              uint2 pack;
+              bf16* e = reinterpret_cast<bf16*>(&pack);
+              // (gate and up rounded first, as a product of its own would have left them)
+#pragma unroll
+              for (int i = 0; i < 4; ++i)
+                e[i] = from_f<bf16>(ts_glu_for<bf16>(round_to<bf16>(f[2 * i]), round_to<bf16>(f[2 * i + 1]), args.glu));
+              *reinterpret_cast<uint2*>(args.out + (size_t)row * (args.N / 2) + col / 2) = pack;
+            } else {
+              uint4 pack;
+              bf16* e = reinterpret_cast<bf16*>(&pack);
+#pragma unroll
+              for (int i = 0; i < 8; ++i) e[i] = from_f<bf16>(ts_activate_for<bf16>(round_to<bf16>(f[i]), args.act));
+              *reinterpret_cast<uint4*>(args.out + (size_t)row * args.N + col) = pack;
+            }
+          }
+        }
       } else {
         bf16* dst = args.out + (size_t)row * args.N + tn * PN;
 #pragma unroll 1
@@ -382,7 +467,7 @@ template <int EPI, int BN>
 cudaError_t allow_pair_smem() {
   static bool done = false;
   if (done) return cudaSuccess;
-  cudaError_t e = cudaFuncSetAttribute(gemm_pair_kernel<EPI, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PairTile<BN>::SMEM);
+  cudaError_t e = cudaFuncSetAttribute(gemm_pair_kernel<EPI, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(grouped_epilogue(EPI) ? PairTile<BN>::GROUPED_SMEM : PairTile<BN>::SMEM));
   if (e == cudaSuccess) done = true;
   return e;
 }
@@ -397,7 +482,7 @@ int pairs_that_fit() {
       cudaLaunchConfig_t cfg = {};
       cfg.gridDim = dim3(2);
       cfg.blockDim = dim3(PAIR_THREADS);
-      cfg.dynamicSmemBytes = PairTile<BN>::SMEM;
+      cfg.dynamicSmemBytes = grouped_epilogue(EPI) ? PairTile<BN>::GROUPED_SMEM : PairTile<BN>::SMEM;
       cudaLaunchAttribute attr[1];
       attr[0].id = cudaLaunchAttributeClusterDimension;
       attr[0].val.clusterDim.x = 2;
@@ -416,15 +501,17 @@ int pairs_that_fit() {
 template <int EPI, int BN>
 int launch_pair(const void* x, const void* w, PairArgs args, cudaStream_t s) {
   CUtensorMap mx, mw;
-  if (!tensor_map(&mx, x, args.M, args.K, PM) || !tensor_map(&mw, w, args.N, args.K, BN / 2))
+  constexpr size_t smem = grouped_epilogue(EPI) ? PairTile<BN>::GROUPED_SMEM : PairTile<BN>::SMEM;
+  const int w_rows = grouped_epilogue(EPI) ? args.experts * args.N : args.N;
+  if (!tensor_map(&mx, x, args.M, args.K, PM) || !tensor_map(&mw, w, w_rows, args.K, BN / 2))
     TS_REFUSE(TS_ERR_UNSUPPORTED, "ts_linear_pair: tensor map for M = %d, N = %d, K = %d", args.M, args.N, args.K);
   const int fit = pairs_that_fit<EPI, BN>();
   if (fit < 1)
-    TS_REFUSE(TS_ERR_UNSUPPORTED, "ts_linear_pair: no pair of blocks with %zu bytes of shared memory fits this device", PairTile<BN>::SMEM);
+    TS_REFUSE(TS_ERR_UNSUPPORTED, "ts_linear_pair: no pair of blocks with %zu bytes of shared memory fits this device", smem);
   args.tiles_n = (args.N + BN - 1) / BN;
   const int tiles = args.tiles_m * args.tiles_n;
   const int pairs = tiles < fit ? tiles : fit;
-  ts_launch_cluster(gemm_pair_kernel<EPI, BN>, dim3(2, 1, 1), dim3(2 * pairs), dim3(PAIR_THREADS), PairTile<BN>::SMEM, s, mx, mw, args);
+  ts_launch_cluster(gemm_pair_kernel<EPI, BN>, dim3(2, 1, 1), dim3(2 * pairs), dim3(PAIR_THREADS), smem, s, mx, mw, args);
   TS_LAUNCH_CHECK();
 }
 
@@ -524,6 +611,39 @@ TS_API int ts_linear_pair_qkv(void* qkv, const void* x, const void* w, const voi
   a.KVH = KVH;
   a.D = D;
   return launch_pair<EPI_QKV, 256>(x, w, a, (cudaStream_t)stream);
+}
+
+TS_API int ts_grouped_pair_supported(int E, int N, int K) {
+  return E > 0 && E <= MAX_EXPERTS && N > 0 && N % 8 == 0 && K > 0 && K % 8 == 0 && (long long)E * N <= 0x7fffffffLL;
+}
+
+// out rows = x rows . w[e]^T for the rows [offsets[e], offsets[e + 1]) of each of E experts: x [M, K] sorted by expert, w [E, N,
+// K], offsets [E + 1] on the device.  epilogue 3: bfloat16 [M, N] through the activation `act`; 4: bfloat16 [M, N / 2], the
+// clamped gated unit of columns (2 i, 2 i + 1); 5: 32-bit [M, N].  Rows behind offsets[E] are left alone.
+TS_API int ts_grouped_pair(void* out, const void* x, const void* w, const int* offsets, int M, int E, int N, int K, int epilogue,
+                           int act, float limit, float slope, float offset, void* stream) {
+  if (M <= 0) return 0;
+  if (!ts_grouped_pair_supported(E, N, K)) TS_REFUSE(TS_ERR_UNSUPPORTED, "ts_grouped_pair: %d experts of %d x %d", E, N, K);
+  if (((uintptr_t)out | (uintptr_t)x | (uintptr_t)w) & 15) TS_REFUSE(TS_ERR_UNSUPPORTED, "ts_grouped_pair: pointers must be 16-byte aligned");
+  if (act < 0 || act > TS_ACT_LAST) TS_REFUSE(TS_ERR_SHAPE, "ts_grouped_pair: activation %d", act);
+  PairArgs a = {};
+  a.out = (bf16*)out;
+  a.out32 = (float*)out;
+  a.M = M;
+  a.N = N;
+  a.K = K;
+  // (what the launch is sized and its tile width chosen by: every group's last tile is half full on average; the kernel counts)
+  a.tiles_m = (M + 2 * PM - 1) / (2 * PM) + E / 2;
+  a.status = ts_gemm_status_word();
+  a.offsets = offsets;
+  a.experts = E;
+  a.act = act;
+  a.glu = TsGlu{limit, slope, offset};
+  cudaStream_t s = (cudaStream_t)stream;
+  if (epilogue == EPI_GROUP) return launch_pair_any<EPI_GROUP>(x, w, a, s);
+  if (epilogue == EPI_GROUP_GLU) return launch_pair_any<EPI_GROUP_GLU>(x, w, a, s);
+  if (epilogue == EPI_GROUP_F32) return launch_pair_any<EPI_GROUP_F32>(x, w, a, s);
+  TS_REFUSE(TS_ERR_UNSUPPORTED, "ts_grouped_pair: epilogue %d", epilogue);
 }
 
 // 256, 192 or 128: every product takes tiles of this width; 0: the width with the shortest schedule.

@@ -68,7 +68,7 @@ class LazyProduct:
 class CudaOps:
     """ctypes front of ``libturingserve_b200.so``."""
 
-    ABI = 19
+    ABI = 20
     UNSUPPORTED = -4            # a kernel's refusal of a shape or layout another kernel takes
 
     def __init__(self, lib_path: str) -> None:
@@ -163,6 +163,8 @@ class CudaOps:
             "ts_rglru_scan": [P, P, P, I, I, I, P, ctypes.c_longlong, P, P, P, I, I, I, I, I, P],
             "ts_rglru_step": [P, P, I, I, I, P, P, P, P, P, P, P, P, ctypes.c_longlong, P, P, I, I, I, I, I, P],
             "ts_rglru_step_supported": [I, I, I, I],
+            "ts_grouped_pair": [P, P, P, P, I, I, I, I, I, I, F, F, F, P],
+            "ts_grouped_pair_supported": [I, I, I],
             "ts_batched_linear": [P, I, I, P, I, I, P, I, I, I, I, I, P],
         }
         for name, args in sigs.items():
@@ -1112,6 +1114,31 @@ class CudaOps:
         self._check(self.lib.ts_grouped_glu(_ptr(out), _ptr(x), _ptr(w), _ptr(order), _ptr(row_scale), _ptr(offsets),
                                             _ptr(tiles), P, E, top, N, K, *(float(v) for v in glu), _code(x.dtype),
                                             _code(out.dtype), self._stream()), "grouped_glu")
+
+    # From this many (token, choice) pairs an expert (and 128 in all) the experts' products run on pairs of SMs over gathered
+    # rows.  8 experts of 1,536 x 2,688, the whole feed-forward captured: 64 pairs 119 us against 94 of the grouped kernels, 128
+    # pairs 115 against 129, 1,024 pairs 111 against 197, 4,096 pairs 197 against 510; of 3,584 x 7,104: 32 pairs 227 against
+    # 192, 64 pairs 246 against 289, 128 pairs 250 against 428, 4,096 pairs 594 against 2,522 us.
+    grouped_pair_rows = int(os.environ.get("TURINGSERVE_B200_GROUPED_PAIR_ROWS", "16"))
+
+    def grouped_pair_takes(self, x, w_up, w_down, pairs: int) -> bool:
+        """Whether ``grouped_pair`` should take the experts' two products of so many pairs (x [T, K], w_up [E, N, K], w_down
+        [E, K, I])."""
+        return (x.dtype == torch.bfloat16 and self.gemm_mode != "library"
+                and pairs >= max(8 * self.grouped_pair_rows, self.grouped_pair_rows * w_up.shape[0])
+                and all(t.is_contiguous() and t.data_ptr() % 16 == 0 and self.lib.ts_grouped_pair_supported(*t.shape)
+                        for t in (w_up, w_down)))
+
+    def grouped_pair(self, out, x, w, offsets, act: str = "none", glu=None) -> None:
+        """out rows = x rows @ w[e]^T for the rows [offsets[e], offsets[e + 1]) of each expert (x bfloat16 [P, K] sorted by
+        expert, w [E, N, K]); ``out`` float32 [P, N], or bfloat16: [P, N] through ``act``, or [P, N / 2] through the clamped gated
+        unit ``glu`` (limit, slope, offset) of neighbouring columns.  Rows behind the last expert's are left alone."""
+        E, N, K = w.shape
+        epilogue = 5 if out.dtype == torch.float32 else (4 if glu is not None else 3)
+        limit, slope, offset = glu if glu is not None else (0.0, 0.0, 0.0)
+        self._check(self.lib.ts_grouped_pair(_ptr(out), _ptr(x), _ptr(w), _ptr(offsets), x.shape[0], E, N, K, epilogue,
+                                             self.ACTIVATIONS[act], float(limit), float(slope), float(offset), self._stream()),
+                    "grouped_pair")
 
     def glu_pairs(self, out, gu, glu) -> None:
         """out [T, I] = the clamped gated unit of the column pairs (2 i, 2 i + 1) of ``gu`` [T, 2 I] (see ``grouped_glu``);

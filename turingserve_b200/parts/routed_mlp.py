@@ -16,10 +16,11 @@ two products run over the sorted groups; the chosen score multiplies the expert'
 summed in 32-bit in the order of their rank.  No count comes back to the host, so the chain may sit in a
 captured step.  The experts' weights are stacked [E, ff, hidden] and [E, hidden, ff] when they arrive.
 
-Many rows (``LIBRARY_ROWS`` pairs or more, outside a capture): the group sizes are read back once, the input
-rows are gathered in sorted order, and every expert's rows go through ``ops().linear`` as a product of their own,
-i.e. to the many-row kernels and the vendor library that the dense products of such steps use.  (With a table the host
-counts the groups itself from the step's ids, and nothing is read back.)
+More rows, bfloat16: the input rows are gathered in sorted order and both products run over the groups on pairs of SMs
+(``ops().grouped_pair``), nothing read back, captured or not.  What that kernel does not take (32-bit, over 256 experts, widths
+that are no multiple of 8) and has many rows (``LIBRARY_ROWS`` pairs or more, outside a capture): the group sizes are read back
+once and every expert's gathered rows go through ``ops().linear`` as a product of their own.  (With a table the host counts the
+groups itself from the step's ids, and nothing is read back.)
 
 Without a router (``table_rows``): an integer table ('table' [ids, top_k]) gives every token id its experts; the choices
 weigh 1 / top_k each, and the sort reads the table itself, so neither router scores nor weights exist.
@@ -196,6 +197,16 @@ class RoutedMLP(FeedForward):
         T, top = x.shape[0], self.top
         y = torch.empty((T * top, self.hidden), dtype=torch.float32, device=x.device)
         up_width = (2 if self.gated else 1) * self.inter
+        if x.is_cuda and ops.grouped_pair_takes(x, self.w_up, self.w_down, T * top):
+            # the experts' input rows in sorted order, weighted and rounded once; both products read them group by group
+            xs = torch.empty((T * top, self.hidden), dtype=x.dtype, device=x.device)
+            ops.moe_gather(xs, x, order, scale, top)
+            a = torch.empty((T * top, self.inter if self.glu else up_width), dtype=x.dtype, device=x.device)
+            ops.grouped_pair(a, xs, self.w_up, offsets, "none" if self.gated else self.activation, self.glu_args if self.glu else None)
+            if self.gated and not self.glu:
+                a = self._activate(a, T * top)
+            ops.grouped_pair(y, a, self.w_down, offsets)
+            return y
         if T * top >= self.LIBRARY_ROWS and x.is_cuda and not torch.cuda.is_current_stream_capturing():
             # the experts' input rows in sorted order, weighted and rounded once (the products then read plain rows)
             xs = torch.empty((T * top, self.hidden), dtype=x.dtype, device=x.device)
