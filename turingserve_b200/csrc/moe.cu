@@ -547,8 +547,8 @@ __global__ void moe_combine_kernel(T* __restrict__ out, const float* __restrict_
 
 // The same, four columns a thread with the token's places and weights read once (N a multiple of 4, at most 8 choices, rows on
 // 16-byte boundaries): 2,048 tokens x 1,536, top 2, an added row: 24 -> 18 us.
-template <typename T>
-__global__ void __launch_bounds__(256)
+template <typename T, int TOP>
+__global__ void __launch_bounds__(512)
 moe_combine_vec_kernel(T* __restrict__ out, const float* __restrict__ y, const int* __restrict__ place,
                        const float* __restrict__ pair_w, int top, int N, const T* __restrict__ x, const int* __restrict__ pass_from,
                        const T* __restrict__ add, const float* __restrict__ share) {
@@ -556,10 +556,10 @@ moe_combine_vec_kernel(T* __restrict__ out, const float* __restrict__ y, const i
   pdl_wait();
   const int t = blockIdx.x;
   const int first_pass = pass_from != nullptr ? *pass_from : 0x7fffffff;
-  int at[8];
-  float w[8];
+  int at[TOP];
+  float w[TOP];
 #pragma unroll
-  for (int r = 0; r < 8; ++r) {
+  for (int r = 0; r < TOP; ++r) {
     at[r] = r < top ? place[(size_t)t * top + r] : 0;
     w[r] = r < top && pair_w != nullptr ? pair_w[(size_t)t * top + r] : 1.f;
   }
@@ -576,9 +576,9 @@ moe_combine_vec_kernel(T* __restrict__ out, const float* __restrict__ y, const i
     }
   };
   for (int n = 4 * threadIdx.x; n < N; n += 4 * blockDim.x) {
-    float v[8][4], acc[4] = {0.f, 0.f, 0.f, 0.f};
+    float v[TOP][4], acc[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-    for (int r = 0; r < 8; ++r) {
+    for (int r = 0; r < TOP; ++r) {
       if (r < top && at[r] >= first_pass) {
         four(x + (size_t)t * N + n, v[r]);
       } else if (r < top) {
@@ -587,7 +587,7 @@ moe_combine_vec_kernel(T* __restrict__ out, const float* __restrict__ y, const i
       }
     }
 #pragma unroll
-    for (int r = 0; r < 8; ++r)
+    for (int r = 0; r < TOP; ++r)
 #pragma unroll
       for (int i = 0; i < 4; ++i)
         if (r < top) acc[i] = fmaf(w[r], v[r][i], acc[i]);
@@ -821,11 +821,18 @@ TS_API int ts_moe_combine(void* out, const float* y, const int* place, const flo
   cudaStream_t s = (cudaStream_t)stream;
   const uintptr_t rows = (uintptr_t)out | (uintptr_t)x | (uintptr_t)add, mask = dtype == TS_F32 ? 15 : 7;
   if ((dtype == TS_F32 || dtype == TS_BF16) && N % 4 == 0 && top <= 8 && !(rows & mask) && !((uintptr_t)y & 15)) {
-    const dim3 block(N >= 1024 ? 256 : ceil_div(ceil_div(N, 4), 32) * 32);
-    if (dtype == TS_F32)
-      ts_launch(moe_combine_vec_kernel<float>, dim3(T), block, 0, s, (float*)out, y, place, pair_w, top, N, (const float*)x, pass_from, (const float*)add, share);
-    else
-      ts_launch(moe_combine_vec_kernel<bf16>, dim3(T), block, 0, s, (bf16*)out, y, place, pair_w, top, N, (const bf16*)x, pass_from, (const bf16*)add, share);
+    const dim3 block(N >= 2048 ? 512 : ceil_div(N, 128) * 32);
+#define TS_MC(TT, TOP)                                                                                                    \
+  ts_launch(moe_combine_vec_kernel<TT, TOP>, dim3(T), block, 0, s, (TT*)out, y, place, pair_w, top, N, (const TT*)x, pass_from, \
+            (const TT*)add, share)
+    if (dtype == TS_F32) {
+      if (top <= 2) TS_MC(float, 2);
+      else TS_MC(float, 8);
+    } else {
+      if (top <= 2) TS_MC(bf16, 2);
+      else TS_MC(bf16, 8);
+    }
+#undef TS_MC
     TS_LAUNCH_CHECK();
   }
   if (dtype == TS_F32)

@@ -113,6 +113,66 @@ ssm_prepare_kernel(float* __restrict__ ready, const T* __restrict__ proj, int pr
   }
 }
 
+// The same for many tokens and filters of four taps, two neighbouring channels a thread (Cn, the strides and the offset even,
+// pairs on their boundaries): the same arithmetic, so the same bits.  2,048 tokens of 3,584 channels: 38 -> 17 us.
+template <typename T>
+__global__ void __launch_bounds__(256)
+ssm_prepare_pairs_kernel(float* __restrict__ ready, const T* __restrict__ proj, int proj_stride, int xbc_off, int dt_off,
+                         const float* __restrict__ conv_w, const float* __restrict__ conv_b, const float* __restrict__ a_log,
+                         const float* __restrict__ dt_bias, const float* __restrict__ state, size_t state_stride, size_t tail_off,
+                         const int* __restrict__ token_request, const int* __restrict__ q_start, const int* __restrict__ slots,
+                         int T_, int H, int Cn) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int t_base = blockIdx.x * SS_PREP_TOKENS, at = blockIdx.y * blockDim.x + threadIdx.x, count = min(SS_PREP_TOKENS, T_ - t_base);
+  const int W = Cn + 2 * H, c = 2 * at;
+  if (c >= Cn) {
+    const int h = at - Cn / 2;
+    if (h >= H) return;
+    const float bias = dt_bias[h], rate = expf(a_log[h]);
+    for (int k = 0; k < count; ++k) {
+      const int t = t_base + k;
+      const float dt = ss_softplus(to_f(proj[(size_t)t * proj_stride + dt_off + h]) + bias);
+      ready[(size_t)t * W + Cn + h] = dt;
+      ready[(size_t)t * W + Cn + H + h] = expf(-rate * dt);
+    }
+    return;
+  }
+  auto two = [](const T* p) {
+    if constexpr (sizeof(T) == 4) return *reinterpret_cast<const float2*>(p);
+    else return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p));
+  };
+  float2 x[SS_PREP_TOKENS];
+#pragma unroll
+  for (int k = 0; k < SS_PREP_TOKENS; ++k)
+    x[k] = k < count ? two(proj + (size_t)(t_base + k) * proj_stride + xbc_off + c) : make_float2(0.f, 0.f);
+  const float4 wa = *reinterpret_cast<const float4*>(conv_w + 4 * (size_t)c), wb = *reinterpret_cast<const float4*>(conv_w + 4 * (size_t)c + 4);
+  const float ba = conv_b != nullptr ? conv_b[c] : 0.f, bb = conv_b != nullptr ? conv_b[c + 1] : 0.f;
+  float2 w0 = make_float2(0.f, 0.f), w1 = w0, w2 = w0;     // the three inputs before the present token's, oldest first
+#pragma unroll
+  for (int k = 0; k < SS_PREP_TOKENS; ++k) {
+    if (k < count) {
+      const int t = t_base + k, b = token_request[t], t0 = q_start[b], i = t - t0;
+      if (k == 0 || i == 0) {
+        const float* tail = state + (size_t)slots[b] * state_stride + tail_off;                     // [3][Cn]
+        auto input = [&](int rel) {
+          if (rel >= 0) return two(proj + (size_t)(t0 + rel) * proj_stride + xbc_off + c);
+          return make_float2(tail[(size_t)(rel + 3) * Cn + c], tail[(size_t)(rel + 3) * Cn + c + 1]);
+        };
+        w0 = input(i - 3);
+        w1 = input(i - 2);
+        w2 = input(i - 1);
+      }
+      const float a = fmaf(wa.w, x[k].x, fmaf(wa.z, w2.x, fmaf(wa.y, w1.x, fmaf(wa.x, w0.x, ba))));
+      const float e = fmaf(wb.w, x[k].y, fmaf(wb.z, w2.y, fmaf(wb.y, w1.y, fmaf(wb.x, w0.y, bb))));
+      *reinterpret_cast<float2*>(ready + (size_t)t * W + c) = make_float2(a / (1.f + expf(-a)), e / (1.f + expf(-e)));
+      w0 = w1;
+      w1 = w2;
+      w2 = x[k];
+    }
+  }
+}
+
 // The filter's new last inputs: the step's last taps - 1 raw rows, or, of a step shorter than that, the old ones moved up (a
 // thread reads all it needs of a channel before it writes that channel).
 template <int THREADS, typename T>
@@ -428,6 +488,18 @@ TS_API int ts_ssm_prepare(float* ready, const void* proj, int proj_stride, int x
   const bool few = T <= 64;
   dim3 grid(few ? T : ceil_div(T, SS_PREP_TOKENS), ceil_div(Cn + H, 256));
   if (grid.y > 65535) TS_REFUSE(TS_ERR_LIMIT, "ts_ssm_prepare: %d channels", Cn);
+  const int pair_bytes = dtype == TS_F32 ? 8 : 4;
+  if (!few && taps == 4 && (dtype == TS_F32 || dtype == TS_BF16) && Cn % 2 == 0 && proj_stride % 2 == 0 && xbc_off % 2 == 0 &&
+      (uintptr_t)proj % pair_bytes == 0 && !((uintptr_t)ready & 7) && !((uintptr_t)conv_w & 15)) {
+    const dim3 pairs(ceil_div(T, SS_PREP_TOKENS), ceil_div(Cn / 2 + H, 256));
+    if (dtype == TS_F32)
+      ts_launch(ssm_prepare_pairs_kernel<float>, pairs, dim3(256), 0, s, ready, (const float*)proj, proj_stride, xbc_off, dt_off, conv_w, conv_b,
+                a_log, dt_bias, state, (size_t)state_stride, (size_t)tail_off, token_request, q_start, slots, T, H, Cn);
+    else
+      ts_launch(ssm_prepare_pairs_kernel<bf16>, pairs, dim3(256), 0, s, ready, (const bf16*)proj, proj_stride, xbc_off, dt_off, conv_w, conv_b,
+                a_log, dt_bias, state, (size_t)state_stride, (size_t)tail_off, token_request, q_start, slots, T, H, Cn);
+    TS_LAUNCH_CHECK();
+  }
 #define TS_SP1(TT, N)                                                                                                 \
   ts_launch(ssm_prepare_kernel<TT, N>, grid, dim3(256), 0, s, ready, (const TT*)proj, proj_stride, xbc_off, dt_off, conv_w, \
             conv_b, a_log, dt_bias, state, (size_t)state_stride, (size_t)tail_off, token_request, q_start, slots, T, H, Cn, taps)

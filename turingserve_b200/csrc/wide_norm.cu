@@ -222,6 +222,44 @@ __global__ void gated_group_rmsnorm_kernel(T* __restrict__ out, int out_stride, 
   }
 }
 
+// The same in bfloat16 with eight columns a thread, held in registers between the sum and the result (a part's width a multiple
+// of 8 and at most 4,096, rows and strides on 16-byte boundaries): 2,048 rows of 3,072 in two parts 25 -> 10 us.
+__global__ void __launch_bounds__(512)
+gated_group_rmsnorm_vec_kernel(bf16* __restrict__ out, int out_stride, const float* __restrict__ x, const bf16* __restrict__ gate,
+                               int gate_stride, const float* __restrict__ w, float eps, int n, int groups, int gate_kind,
+                               int gate_first, float scale) {
+  pdl_launch_dependents();
+  pdl_wait();
+  __shared__ float scratch[32];
+  const int m = n / groups, c0 = blockIdx.y * m, i = 8 * threadIdx.x;
+  const bool here = i < m;
+  float v[8], g[8], ss = 0.f;
+  if (here) {
+    const float* xr = x + (size_t)blockIdx.x * n + c0 + i;
+    const float4 a = *reinterpret_cast<const float4*>(xr), b = *reinterpret_cast<const float4*>(xr + 4);
+    const uint4 z = *reinterpret_cast<const uint4*>(gate + (size_t)blockIdx.x * gate_stride + c0 + i);
+    const bf16* ze = reinterpret_cast<const bf16*>(&z);
+    v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      g[k] = ts_gate_for<bf16>(to_f(ze[k]), gate_kind);
+      if (gate_first) v[k] *= g[k];
+      ss = fmaf(v[k], v[k], ss);
+    }
+  }
+  ss = block_sum(ss, scratch);
+  const float rstd = 1.f / sqrtf(ss / (float)m + eps);
+  if (!here) return;
+  uint4 o;
+  bf16* oe = reinterpret_cast<bf16*>(&o);
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const float r = v[k] * rstd * w[c0 + i + k];
+    oe[k] = from_f<bf16>((gate_first ? r : r * g[k]) * scale);
+  }
+  *reinterpret_cast<uint4*>(out + (size_t)blockIdx.x * out_stride + c0 + i) = o;
+}
+
 // out[t, i] = T(a[t, i] * gate(z[t, i]) * scale): the gate on a mixer's heads before its output projection
 template <typename T>
 __global__ void gate_mul_kernel(T* __restrict__ out, int out_stride, const T* __restrict__ a, int a_stride,
@@ -369,7 +407,13 @@ TS_API int ts_gated_group_rmsnorm(void* out, int out_stride, const float* x, con
   if (groups < 1 || n % groups) TS_REFUSE(TS_ERR_SHAPE, "ts_gated_group_rmsnorm: %d columns in %d parts", n, groups);
   if (groups > 65535) TS_REFUSE(TS_ERR_LIMIT, "ts_gated_group_rmsnorm: %d parts", groups);
   cudaStream_t s = (cudaStream_t)stream;
-  const int th = threads_for(n / groups);
+  const int th = threads_for(n / groups), m = n / groups;
+  if (dtype == TS_BF16 && m % 8 == 0 && m <= 4096 && out_stride % 8 == 0 && gate_stride % 8 == 0 &&
+      !(((uintptr_t)out | (uintptr_t)x | (uintptr_t)gate) & 15)) {
+    ts_launch(gated_group_rmsnorm_vec_kernel, dim3(T, groups), dim3(ceil_div(m, 256) * 32), 0, s, (bf16*)out, out_stride, x,
+              (const bf16*)gate, gate_stride, w, eps, n, groups, gate_kind, gate_first, scale);
+    TS_LAUNCH_CHECK();
+  }
   if (dtype == TS_F32)
     ts_launch(gated_group_rmsnorm_kernel<float>, dim3(T, groups), dim3(th), 0, s, (float*)out, out_stride, x, (const float*)gate,
               gate_stride, w, eps, n, groups, gate_kind, gate_first, scale);
