@@ -57,7 +57,7 @@ def test_linear_attention_long_portions(ops, dtype, H, D, V):
     proj = torch.randn(sum(lens), width + 16, generator=g, device=DEV).to(dtype)
     decay = 1 - torch.rand(H, generator=g, device=DEV) * 0.2
     first = torch.randn(9, H, D, V, generator=g, device=DEV)
-    assert ops.lib.ts_lightning_long_supported(D, V, width + 16, 64, int(dtype == torch.bfloat16))
+    assert ops.lib.ts_lightning_long_supported(D, V, width + 16, 128, int(dtype == torch.bfloat16))
     results = []
     for cuts in CUTS:
         state, out = first.clone(), torch.full((sum(lens), H * V), float("nan"), device=DEV)

@@ -318,9 +318,10 @@ lightning_long_kernel(float* __restrict__ out, const float* __restrict__ ready, 
 // decay: [H] 32-bit on the device.  out: [T, H V] 32-bit.
 // longest: the most tokens a request brings (0: not known); from LT_LATE_TOKENS on the kernel is launched late (see
 // ts_launch_late).
-// ts_lightning_long takes such portions where ts_lightning_long_supported says so, with ready [T, H (2 D + V)] 32-bit
-// as work memory; outputs and states are the same bits.
-constexpr int LT_LATE_TOKENS = 64;
+// ts_lightning_long takes portions from LL_TOKENS on where ts_lightning_long_supported says so, with ready [T, H (2 D + V)]
+// 32-bit as work memory; outputs and states are the same bits.  (At 64 tokens it saves the GPU a few microseconds and costs the
+// host one launch more.)
+constexpr int LT_LATE_TOKENS = 64, LL_TOKENS = 128;
 
 TS_API int ts_lightning_ex(float* out, const void* proj, int proj_stride, float* state, const float* decay,
                            const int* q_start, const int* slots, int B, int H, int D, int V, int longest, int dtype,
@@ -371,7 +372,7 @@ TS_API int ts_lightning_ex(float* out, const void* proj, int proj_stride, float*
 
 TS_API int ts_lightning_long_supported(int D, int V, int proj_stride, int longest, int dtype) {
   const int per16 = dtype == TS_F32 ? 4 : 8;
-  return (dtype == TS_F32 || dtype == TS_BF16) && longest >= LT_LATE_TOKENS && D > 0 && D <= 256 && D % per16 == 0 && V > 0 &&
+  return (dtype == TS_F32 || dtype == TS_BF16) && longest >= LL_TOKENS && D > 0 && D <= 256 && D % per16 == 0 && V > 0 &&
          V % per16 == 0 && proj_stride % per16 == 0;
 }
 

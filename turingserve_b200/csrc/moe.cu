@@ -39,46 +39,11 @@ constexpr int GL_BM = 64, GL_BN = 64, GL_BK = 16, GL_PAD = 4;
 // lane by lane, then warp by warp, in a fixed order.  Warp 0 then picks the experts.
 constexpr int RT_THREADS = 256;
 
-template <typename T>
-__global__ void __launch_bounds__(RT_THREADS)
-router_topk_kernel(int* __restrict__ idx_out, float* __restrict__ w_out, const T* __restrict__ x,
-                   const float* __restrict__ wr, int T_, int E, int K, int top, int softmax, int renorm,
-                   const float* __restrict__ correction, int groups, int keep, float scale, float* __restrict__ share) {
-  pdl_launch_dependents();
-  pdl_wait();
-  extern __shared__ float smem[];
-  const int rows = E + (share != nullptr ? 1 : 0);     // (the shared expert's row lies behind the experts')
-  float* z = smem;                       // [E + 1]
-  float* part = z + E + 1;               // [RT_THREADS / 32][8]
-  float* pick = part + RT_THREADS / 32 * 8;   // [E] what the choice goes by, when it is not z itself
-  float* gsum = pick + E;                // [groups]
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int t = blockIdx.x;
-  const T* xr = x + (size_t)t * K;
-  for (int e0 = 0; e0 < rows; e0 += 8) {
-    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-#pragma unroll 2
-    for (int k = threadIdx.x; k < K; k += RT_THREADS) {
-      const float xv = to_f(xr[k]);
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-        if (e0 + i < rows) acc[i] = fmaf(xv, __ldg(wr + (size_t)(e0 + i) * K + k), acc[i]);
-    }
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const float v = warp_sum(acc[i]);
-      if (lane == 0) part[warp * 8 + i] = v;
-    }
-    __syncthreads();
-    if (threadIdx.x < 8 && e0 + threadIdx.x < rows) {
-      float v = 0.f;
-      for (int w = 0; w < RT_THREADS / 32; ++w) v += part[w * 8 + threadIdx.x];
-      z[e0 + threadIdx.x] = v;
-    }
-    __syncthreads();
-  }
-  if (warp != 0) return;
-  __syncwarp();
+// One warp picks the experts of token t from its logits z (which it may overwrite); pick [E] and gsum [groups] are its own.
+__device__ __forceinline__ void choose_experts(int t, float* z, float* pick, float* gsum, int lane, int* __restrict__ idx_out,
+                                               float* __restrict__ w_out, int E, int top, int softmax, int renorm,
+                                               const float* __restrict__ correction, int groups, int keep, float scale,
+                                               float* __restrict__ share) {
   float zmax = -INFINITY, denom = 1.f;
   if (softmax) {
     for (int e = lane; e < E; e += 32) zmax = fmaxf(zmax, z[e]);
@@ -157,6 +122,117 @@ router_topk_kernel(int* __restrict__ idx_out, float* __restrict__ w_out, const T
   if ((renorm || scale != 1.f) && lane == 0)
     for (int r = 0; r < top; ++r)
       w_out[(size_t)t * top + r] = (renorm ? w_out[(size_t)t * top + r] / (total + 1e-20f) : w_out[(size_t)t * top + r]) * scale;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(RT_THREADS)
+router_topk_kernel(int* __restrict__ idx_out, float* __restrict__ w_out, const T* __restrict__ x,
+                   const float* __restrict__ wr, int T_, int E, int K, int top, int softmax, int renorm,
+                   const float* __restrict__ correction, int groups, int keep, float scale, float* __restrict__ share) {
+  pdl_launch_dependents();
+  pdl_wait();
+  extern __shared__ float smem[];
+  const int rows = E + (share != nullptr ? 1 : 0);     // (the shared expert's row lies behind the experts')
+  float* z = smem;                       // [E + 1]
+  float* part = z + E + 1;               // [RT_THREADS / 32][8]
+  float* pick = part + RT_THREADS / 32 * 8;   // [E] what the choice goes by, when it is not z itself
+  float* gsum = pick + E;                // [groups]
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int t = blockIdx.x;
+  const T* xr = x + (size_t)t * K;
+  for (int e0 = 0; e0 < rows; e0 += 8) {
+    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll 2
+    for (int k = threadIdx.x; k < K; k += RT_THREADS) {
+      const float xv = to_f(xr[k]);
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (e0 + i < rows) acc[i] = fmaf(xv, __ldg(wr + (size_t)(e0 + i) * K + k), acc[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float v = warp_sum(acc[i]);
+      if (lane == 0) part[warp * 8 + i] = v;
+    }
+    __syncthreads();
+    if (threadIdx.x < 8 && e0 + threadIdx.x < rows) {
+      float v = 0.f;
+      for (int w = 0; w < RT_THREADS / 32; ++w) v += part[w * 8 + threadIdx.x];
+      z[e0 + threadIdx.x] = v;
+    }
+    __syncthreads();
+  }
+  if (warp != 0) return;
+  __syncwarp();
+  choose_experts(t, z, pick, gsum, lane, idx_out, w_out, E, top, softmax, renorm, correction, groups, keep, scale, share);
+}
+
+// Many tokens: RT_TOKENS a block, because one token a block reads the whole router from L2 for every token (8 experts over 2,688
+// columns, 2,048 tokens: 176 MB).  Thread i keeps the same columns and the sums are added along the same tree, so the logits
+// are the same bits: the 32 sums that a thread holds of four tokens cross the lanes together, each step halving what a lane keeps, and lane
+// l ends with sum l.  Warp w picks for token w.  Four tokens a block while one wave of three blocks an SM holds them all
+// (1,776), eight behind that: 2,048 tokens 20 us with one a block, 14.6 with four, 12.4 with eight; 1,024 tokens 8.3 with four, 10.3
+// with eight; below 512 one a block is as fast (8.2).
+constexpr int RT_MANY_TOKENS = 512, RT_MOST_TOKENS = 1777;
+
+template <typename T, int RT_TOKENS>
+__global__ void __launch_bounds__(RT_THREADS, RT_TOKENS == 8 ? 2 : 0)
+router_topk_tokens_kernel(int* __restrict__ idx_out, float* __restrict__ w_out, const T* __restrict__ x,
+                          const float* __restrict__ wr, int T_, int E, int K, int top, int softmax, int renorm,
+                          const float* __restrict__ correction, int groups, int keep, float scale, float* __restrict__ share) {
+  pdl_launch_dependents();
+  pdl_wait();
+  extern __shared__ float smem[];
+  const int rows = E + (share != nullptr ? 1 : 0), own = 2 * E + 1 + groups;     // (z, pick and gsum of a token)
+  float* part = smem + RT_TOKENS * own;  // [RT_TOKENS / 4][RT_THREADS / 32][32]
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int t0 = blockIdx.x * RT_TOKENS;
+  const T* xr[RT_TOKENS];
+#pragma unroll
+  for (int j = 0; j < RT_TOKENS; ++j) xr[j] = x + (size_t)min(t0 + j, T_ - 1) * K;
+  for (int e0 = 0; e0 < rows; e0 += 8) {
+    float acc[RT_TOKENS * 8];
+#pragma unroll
+    for (int i = 0; i < RT_TOKENS * 8; ++i) acc[i] = 0.f;
+#pragma unroll 2
+    for (int k = threadIdx.x; k < K; k += RT_THREADS) {
+      float xv[RT_TOKENS];
+#pragma unroll
+      for (int j = 0; j < RT_TOKENS; ++j) xv[j] = to_f(xr[j][k]);
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (e0 + i < rows) {
+          const float wv = __ldg(wr + (size_t)(e0 + i) * K + k);
+#pragma unroll
+          for (int j = 0; j < RT_TOKENS; ++j) acc[j * 8 + i] = fmaf(xv[j], wv, acc[j * 8 + i]);
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < RT_TOKENS / 4; ++q) {                      // 32 sums of four tokens
+      float* sum = acc + q * 32;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const bool upper = (lane & o) != 0;
+#pragma unroll
+        for (int i = 0; i < o; ++i) {
+          const float kept = upper ? sum[i + o] : sum[i], sent = upper ? sum[i] : sum[i + o];
+          sum[i] = kept + __shfl_xor_sync(0xffffffffu, sent, o);
+        }
+      }
+      part[(q * (RT_THREADS / 32) + warp) * 32 + lane] = sum[0];
+    }
+    __syncthreads();
+    if (warp < RT_TOKENS / 4 && e0 + (lane & 7) < rows) {
+      float v = 0.f;
+      for (int w = 0; w < RT_THREADS / 32; ++w) v += part[(warp * (RT_THREADS / 32) + w) * 32 + lane];
+      smem[(warp * 4 + (lane >> 3)) * own + e0 + (lane & 7)] = v;
+    }
+    __syncthreads();
+  }
+  if (warp >= RT_TOKENS || t0 + warp >= T_) return;
+  float* z = smem + warp * own;
+  choose_experts(t0 + warp, z, z + E + 1, z + 2 * E + 1, lane, idx_out, w_out, E, top, softmax, renorm, correction, groups, keep,
+                 scale, share);
 }
 
 // ---------------------------------------------------------------------------------------------------
@@ -546,7 +622,7 @@ __global__ void moe_combine_kernel(T* __restrict__ out, const float* __restrict_
 }
 
 // The same, four columns a thread with the token's places and weights read once (N a multiple of 4, at most 8 choices, rows on
-// 16-byte boundaries): 2,048 tokens x 1,536, top 2, an added row: 24 -> 18 us.
+// 16-byte boundaries): 2,048 tokens x 1,536, top 2, an added row: 24 -> 8 us.
 template <typename T, int TOP>
 __global__ void __launch_bounds__(512)
 moe_combine_vec_kernel(T* __restrict__ out, const float* __restrict__ y, const int* __restrict__ place,
@@ -700,6 +776,18 @@ TS_API int ts_router_topk(int* idx_out, float* w_out, const void* x, const float
   cudaStream_t s = (cudaStream_t)stream;
   if (groups < 1 || keep < 1 || keep > groups || E % groups || (groups > 1 && top > E / groups * keep))
     TS_REFUSE(TS_ERR_SHAPE, "ts_router_topk: %d of %d groups of %d experts, top %d", keep, groups, E, top);
+  const int tokens = T >= RT_MOST_TOKENS ? 8 : 4;
+  const size_t many_smem = sizeof(float) * (tokens * (2 * E + 1 + groups) + tokens / 4 * RT_THREADS);
+  if (T >= RT_MANY_TOKENS && many_smem <= 48 * 1024 && (dtype == TS_F32 || dtype == TS_BF16)) {
+    const dim3 grid(ceil_div(T, tokens));
+    if (dtype == TS_F32)
+      ts_launch(tokens == 8 ? router_topk_tokens_kernel<float, 8> : router_topk_tokens_kernel<float, 4>, grid, dim3(RT_THREADS), many_smem,
+                s, idx_out, w_out, (const float*)x, wr, T, E, K, top, softmax, renorm, correction, groups, keep, scale, share);
+    else
+      ts_launch(tokens == 8 ? router_topk_tokens_kernel<bf16, 8> : router_topk_tokens_kernel<bf16, 4>, grid, dim3(RT_THREADS), many_smem, s,
+                idx_out, w_out, (const bf16*)x, wr, T, E, K, top, softmax, renorm, correction, groups, keep, scale, share);
+    TS_LAUNCH_CHECK();
+  }
   const size_t smem = sizeof(float) * (2 * E + 1 + RT_THREADS / 32 * 8 + groups);
   if (dtype == TS_F32)
     ts_launch(router_topk_kernel<float>, dim3(T), dim3(RT_THREADS), smem, s, idx_out, w_out, (const float*)x, wr, T,

@@ -653,7 +653,7 @@ class CudaOps:
         q, k, v = silu of the columns [0, HD), [HD, 2HD), [2HD, 2HD + HV) of ``proj``; ``state``
         (float32 [slots, H, D, V]) is read and left updated at each request's slot."""
         longest = int(getattr(step, "max_q_len", 0) or 0)
-        if self.lib.ts_lightning_long_supported(D, V, proj.stride(0), longest, _code(proj.dtype)):
+        if longest >= 128 and self.lib.ts_lightning_long_supported(D, V, proj.stride(0), longest, _code(proj.dtype)):
             ready = torch.empty((proj.shape[0], H * (2 * D + V)), dtype=torch.float32, device=proj.device)
             rc = self.lib.ts_lightning_long(_ptr(out), _ptr(proj), proj.stride(0), _ptr(ready), _ptr(state), _ptr(decay),
                                             _ptr(step.q_start), _ptr(step.state_slots), step.num_requests, proj.shape[0], H, D, V,
@@ -676,8 +676,12 @@ class CudaOps:
                                               _ptr(slots), proj.shape[0], KVH, DK, DV, page_size, _code(proj.dtype),
                                               self._stream()), "kv_write_pair")
 
-    # portions (more than 16 query rows a kv head) that reach over at least this many keys go to the tcgen05 kernel
-    diff_tc_keys = int(os.environ.get("TURINGSERVE_B200_DIFF_TC_KEYS", "128"))
+    # Portions (more than 16 query rows a kv head) that reach over at least this many keys go to the tcgen05 kernel and the one
+    # that joins its two maps.  The GPU is faster with them from 128 keys on (the whole mixer at width 1,536: 128 tokens 45.1
+    # against 45.5 us, 256 tokens 24.7 against 38.5, 512 tokens 30.8 against 59.3; 16 tokens behind 2,000: 47 against 169), but
+    # their launches and tensor maps cost the host 6 us more, and below 512 keys the host is what such a call waits for
+    # (70 tokens behind 184: 79.6 against 73.2 us a call).
+    diff_tc_keys = int(os.environ.get("TURINGSERVE_B200_DIFF_TC_KEYS", "512"))
 
     def attention_diff(self, out, proj, k_cache, v_cache, block_tables, step, H: int, KVH: int, D: int, V: int,
                        page_size: int, scale: float, lam: float, eps: float, out_scale: float) -> None:
@@ -937,8 +941,7 @@ class CudaOps:
 
             def portions(first: int, count: int) -> int:
                 """Requests whose keys are not cut: by tcgen05 from ``biased_tc_keys`` keys on."""
-                if (self.use_tc_attention and reach >= self.biased_tc_keys
-                        and self.lib.ts_attention_biased_tc_supported(H, KVH, Dk, Dv, v_in_k, page_size, _code(q.dtype))):
+                if self.use_tc_attention and reach >= self.biased_tc_keys and page_size % 16 == 0:
                     rc = self.lib.ts_attention_biased_tc(
                         _ptr(out), out.stride(0), out.stride(1), _ptr(q), q.stride(0), q.stride(1), _ptr(k_cache), _ptr(v_cache),
                         block_tables.data_ptr() + 4 * first * width, step.q_start.data_ptr() + 4 * first,
@@ -1124,10 +1127,11 @@ class CudaOps:
     def grouped_pair_takes(self, x, w_up, w_down, pairs: int) -> bool:
         """Whether ``grouped_pair`` should take the experts' two products of so many pairs (x [T, K], w_up [E, N, K], w_down
         [E, K, I])."""
-        return (x.dtype == torch.bfloat16 and self.gemm_mode != "library"
-                and pairs >= max(8 * self.grouped_pair_rows, self.grouped_pair_rows * w_up.shape[0])
-                and all(t.is_contiguous() and t.data_ptr() % 16 == 0 and self.lib.ts_grouped_pair_supported(*t.shape)
-                        for t in (w_up, w_down)))
+        if pairs < 8 * self.grouped_pair_rows or x.dtype != torch.bfloat16 or self.gemm_mode == "library":
+            return False
+        return (pairs >= self.grouped_pair_rows * w_up.shape[0]
+                and all(w.dtype == x.dtype and w.is_contiguous() and w.data_ptr() % 16 == 0
+                        and self.lib.ts_grouped_pair_supported(*w.shape) for w in (w_up, w_down)))
 
     def grouped_pair(self, out, x, w, offsets, act: str = "none", glu=None) -> None:
         """out rows = x rows @ w[e]^T for the rows [offsets[e], offsets[e + 1]) of each expert (x bfloat16 [P, K] sorted by

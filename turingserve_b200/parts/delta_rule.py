@@ -62,7 +62,7 @@ class DeltaRule(Mixer):
         ops.linear(proj, x, self.w_in)
         # 32-bit rows [q | k | v | g | beta | k.q] for the scan, each on a 16-byte boundary (it fetches 16 bytes at a time then)
         n_ready = self.channels + 2 * H + G
-        ready = torch.empty((T, -(-n_ready // 4) * 4), dtype=torch.float32, device=x.device)[:, :n_ready]
+        ready = torch.empty_strided((T, n_ready), (-(-n_ready // 4) * 4, 1), dtype=torch.float32, device=x.device)
         ops.delta_prepare(ready, proj, self.conv, self.a_log, self.dt_bias, state, step, H, G, D, V, self.taps,
                           self.unit_eps)
         o = torch.empty((T, self.hv), dtype=torch.float32, device=x.device)
