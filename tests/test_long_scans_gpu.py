@@ -51,12 +51,13 @@ def close(got, want):
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("H,D,V", [(2, 128, 128), (3, 64, 40), (1, 8, 8), (2, 40, 24), (1, 256, 16), (2, 136, 8)])
-def test_linear_attention_long_portions(ops, dtype, H, D, V):
+def test_linear_attention_long_portions(ops, monkeypatch, dtype, H, D, V):
     lens, width = [150, 64, 7, 200], H * (2 * D + V)
     g = torch.Generator(device=DEV).manual_seed(D + V)
     proj = torch.randn(sum(lens), width + 16, generator=g, device=DEV).to(dtype)
     decay = 1 - torch.rand(H, generator=g, device=DEV) * 0.2
     first = torch.randn(9, H, D, V, generator=g, device=DEV)
+    monkeypatch.setattr(ops, "lightning_long_tokens", 128)
     assert ops.lib.ts_lightning_long_supported(D, V, width + 16, 128, int(dtype == torch.bfloat16))
     results = []
     for cuts in CUTS:

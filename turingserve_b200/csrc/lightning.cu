@@ -319,8 +319,8 @@ lightning_long_kernel(float* __restrict__ out, const float* __restrict__ ready, 
 // longest: the most tokens a request brings (0: not known); from LT_LATE_TOKENS on the kernel is launched late (see
 // ts_launch_late).
 // ts_lightning_long takes portions from LL_TOKENS on where ts_lightning_long_supported says so, with ready [T, H (2 D + V)]
-// 32-bit as work memory; outputs and states are the same bits.  (At 64 tokens it saves the GPU a few microseconds and costs the
-// host one launch more.)
+// 32-bit as work memory; outputs and states are the same bits.  (From how
+// many tokens on its second launch pays is the caller's to say.)
 constexpr int LT_LATE_TOKENS = 64, LL_TOKENS = 128;
 
 TS_API int ts_lightning_ex(float* out, const void* proj, int proj_stride, float* state, const float* decay,

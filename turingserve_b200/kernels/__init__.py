@@ -648,12 +648,18 @@ class CudaOps:
                                            self._stream()), "activation")
 
     # -- linear attention with a decaying matrix state ----------------------------------------------------
+    # Steps whose longest portion has at least this many tokens go to the two kernels for long portions (the scan takes the GPU a
+    # third of the time a token, 54 against 165 ns with 6 heads of 128 x 128).  Their work memory and second launch cost the host
+    # a few microseconds, and a mixer of fewer tokens waits for the host (three requests of 188 tokens, width 1,536: 130 us
+    # a call with them, 123 without; its kernels take less).
+    lightning_long_tokens = int(os.environ.get("TURINGSERVE_B200_LIGHTNING_LONG_TOKENS", "384"))
+
     def lightning(self, out, proj, state, decay, step, H: int, D: int, V: int) -> None:
         """out (float32 [T, H V]): per head o_t = S_t^T q_t with S_t = decay_h S_(t-1) + k_t v_t^T, where
         q, k, v = silu of the columns [0, HD), [HD, 2HD), [2HD, 2HD + HV) of ``proj``; ``state``
         (float32 [slots, H, D, V]) is read and left updated at each request's slot."""
         longest = int(getattr(step, "max_q_len", 0) or 0)
-        if longest >= 128 and self.lib.ts_lightning_long_supported(D, V, proj.stride(0), longest, _code(proj.dtype)):
+        if longest >= self.lightning_long_tokens and self.lib.ts_lightning_long_supported(D, V, proj.stride(0), longest, _code(proj.dtype)):
             ready = torch.empty((proj.shape[0], H * (2 * D + V)), dtype=torch.float32, device=proj.device)
             rc = self.lib.ts_lightning_long(_ptr(out), _ptr(proj), proj.stride(0), _ptr(ready), _ptr(state), _ptr(decay),
                                             _ptr(step.q_start), _ptr(step.state_slots), step.num_requests, proj.shape[0], H, D, V,
