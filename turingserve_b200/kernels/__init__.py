@@ -651,7 +651,7 @@ class CudaOps:
     # Steps whose longest portion has at least this many tokens go to the two kernels for long portions (the scan takes the GPU a
     # third of the time a token, 54 against 165 ns with 6 heads of 128 x 128).  Their work memory and second launch cost the host
     # a few microseconds, and a mixer of fewer tokens waits for the host (three requests of 188 tokens, width 1,536: 130 us
-    # a call with them, 123 without; its kernels take less).
+    # a call with them, 123 before them; its kernels take less).
     lightning_long_tokens = int(os.environ.get("TURINGSERVE_B200_LIGHTNING_LONG_TOKENS", "384"))
 
     def lightning(self, out, proj, state, decay, step, H: int, D: int, V: int) -> None:
