@@ -127,3 +127,57 @@ def test_prompt_portions_by_tcgen05(ops, H, KVH, Dk, Dv, page, reqs, opt, shuffl
         got = out[at:at + n, :, :Dv].double()
         # (scores in the tens of thousands: a 32-bit sum of them is off by up to 1e-2, and so is a weight)
         assert torch.allclose(got, want, rtol=2 ** -8, atol=2e-3 * size * (20 if opt.get("big") else 1)), (n, c, float((got - want).abs().max()))
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf"), float("-inf")])
+@pytest.mark.parametrize("H,KVH,Dk,Dv,page,n,ctx,opt", [
+    (6, 2, 128, 128, 64, 300, 0, {}), (2, 2, 128, 128, 16, 200, 70, dict(window=50)), (4, 1, 128, 128, 16, 150, 333, dict(window=33, keep=5)),
+    (4, 2, 128, 128, 32, 129, 100, dict(block_of=48)), (8, 2, 64, 64, 16, 130, 9, dict(window=40)), (12, 1, 576, 512, 64, 77, 130, {}),
+    (5, 1, 576, 512, 16, 90, 40, dict(window=30)), (4, 2, 320, 256, 16, 65, 20, dict(window=20, keep=3))])
+def test_values_that_are_no_numbers_stay_with_the_rows_that_see_them(ops, H, KVH, Dk, Dv, page, n, ctx, opt, bad):
+    """One column of some keys' values holds an infinity or NaN: that column is no number in every row that sees such a
+    key, and every other element is the same bits as without (a weight of zero times it would be NaN)."""
+    g = torch.Generator(device=DEV).manual_seed(n + Dk)
+    rnd = lambda *s: torch.randn(*s, generator=g, device=DEV)
+    m, window, block_of, keep = n + ctx, opt.get("window"), opt.get("block_of"), opt.get("keep", 0)
+    pages = -(-m // page)
+    pool_k = rnd(pages, KVH, page, Dk).bfloat16()
+    pool_v = None if Dv != Dk else rnd(pages, KVH, page, Dv).bfloat16()
+    step = SimpleNamespace(q_start=i32([0, n]), seq_lens=i32([m]), num_requests=1, num_decode=0, max_q_len=n, max_seq_len=m)
+    q, table = rnd(n, H, Dk).bfloat16(), i32([list(range(pages))])
+    if pool_v is None:
+        q[:, :, :Dv] = 0                                   # (the latent column that is spoiled is also a key's: no score may see it)
+
+    def attend():
+        out = torch.full((n, H, Dv), -7.0, device=DEV).bfloat16()
+        keys, ops.biased_tc_keys = ops.biased_tc_keys, 1
+        try:
+            ops.attention_biased(out, q, pool_k, pool_v, table, step, KVH, page, Dk ** -0.5, 0.0, None, window, chunk=block_of, keep=keep)
+        finally:
+            ops.biased_tc_keys = keys
+        assert ops.tc_status() == 0
+        return out
+
+    clean = attend()
+    i, j = torch.arange(n, device=DEV)[:, None] + ctx, torch.arange(m, device=DEV)[None, :]
+    seen = j <= i
+    if window:
+        seen &= (j > i - window) | (j < keep)
+    if block_of:
+        seen &= j >= i // block_of * block_of
+    spoiled = [(m - 1, 3), (ctx + n // 2, Dv - 1), (ctx + 1, Dv // 2), (max(0, ctx - 20), 17), (2, 40)]
+    for at, col in spoiled:
+        rows = pool_v if pool_v is not None else pool_k
+        rows[at // page, KVH - 1, at % page, col] = bad
+    dirty = attend()
+    spoilt, per = torch.zeros_like(clean, dtype=torch.bool), H // KVH
+    for at, col in spoiled:
+        spoilt[:, (KVH - 1) * per:, col] |= seen[:, at, None]
+    if pool_v is None:
+        # (zero times the spoiled column is NaN in the score of every row that sees the key)
+        hit = torch.stack([seen[:, at] for at, _ in spoiled]).any(0)
+        assert bool(dirty[hit][:, (KVH - 1) * per:].isnan().all()) and torch.equal(dirty[~hit], clean[~hit])
+        assert torch.equal(dirty[:, :(KVH - 1) * per], clean[:, :(KVH - 1) * per])
+    else:
+        # (an infinity times a weight's two terms, of which the second may be negative, is NaN too)
+        assert torch.equal(~dirty.isfinite(), spoilt) and torch.equal(dirty[~spoilt], clean[~spoilt])

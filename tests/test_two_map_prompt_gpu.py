@@ -64,3 +64,33 @@ def test_two_maps_in_portions(H, KVH, V, page, reqs, shuffled):
             o = maps[0] - lam * maps[1]
             want = o / torch.sqrt(o.pow(2).mean(-1, keepdim=True) + 1e-6) * 0.5
             assert torch.allclose(out[at:at + n, h * V:(h + 1) * V].double(), want, rtol=2 ** -7, atol=2 ** -7), (n, c, h)
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("H,KVH,V,page,n,ctx", [(6, 2, 128, 16, 300, 9), (2, 2, 64, 64, 129, 70)])
+def test_values_that_are_no_numbers_reach_no_earlier_row(H, KVH, V, page, n, ctx, bad):
+    """A value that is an infinity or NaN: heads of rows that see its key are NaN, all others the same bits as without it."""
+    from turingserve_b200 import kernels
+    ops = kernels.ops()
+    g = torch.Generator(device=DEV).manual_seed(n + V)
+    rnd = lambda *s: torch.randn(*s, generator=g, device=DEV).bfloat16()
+    pages = -(-(n + ctx) // page)
+    pool_k, pool_v, proj = rnd(pages, KVH, page, 128), rnd(pages, KVH, page, V), rnd(n, H * 128)
+    step = SimpleNamespace(q_start=i32([0, n]), seq_lens=i32([n + ctx]), num_requests=1, num_decode=0, max_q_len=n, max_seq_len=n + ctx,
+                           q_lens=[n], token_request=i32([0] * n))
+
+    def attend():
+        out = torch.full((n, H * V), -7.0, device=DEV).bfloat16()
+        keys, ops.diff_tc_keys = ops.diff_tc_keys, 1
+        try:
+            ops.attention_diff(out, proj, pool_k, pool_v, i32([list(range(pages))]), step, H, KVH, 64, V, page, 0.125, 0.4, 1e-6, 0.5)
+        finally:
+            ops.diff_tc_keys = keys
+        assert ops.tc_status() == 0
+        return out.view(n, KVH, -1)
+
+    clean, at = attend(), ctx + n // 2
+    pool_v[at // page, 0, at % page, 5] = bad
+    dirty = attend()
+    assert torch.equal(dirty[:n // 2], clean[:n // 2]) and torch.equal(dirty[:, 1:], clean[:, 1:])
+    assert bool(dirty[n // 2:, 0].isnan().all())

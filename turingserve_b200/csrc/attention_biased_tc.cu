@@ -16,7 +16,11 @@
 //     its scores are there, the value blocks only when its O product is done: two rings, and the scores begin with the
 //     former;
 //   * keys a block must not see are masked, and their value rows are cleared in shared memory before the second product
-//     reads them: a weight of zero times whatever a page holds behind a request's last token must stay zero.
+//     reads them: a weight of zero times whatever a page holds behind a request's last token must stay zero;
+//   * the same holds for a key that some rows of the block see and others do not: in the tiles where that happens (those of
+//     the block's own tokens and of the window's lower edge) infinities and NaN among the values are taken out before the
+//     product and added at the end to the rows that see them, read from memory once more.  The look at such a tile's values
+//     costs about a hundred instructions a thread, in one or two tiles of a block.
 // Order of the products: S(0) S(1) O(0) S(2) O(1) S(3) ...: a tile's softmax runs beside the O of the tile before and the
 // S of the tile behind.
 //
@@ -65,6 +69,8 @@ struct Args {
   bf16* out;
   float* out32;            // two score maps a head: rows [T, H, 2, DV] in place of `out`
   const bf16* q;
+  const bf16* values;      // the rows the values lie in ([page, kv head, token], value_row wide), and for a block's slow path only
+  int value_row;
   const int* block_tables;
   const int* q_start;
   const int* seq_lens;
@@ -81,6 +87,14 @@ struct Args {
 };
 
 template <int N> using Int = std::integral_constant<int, N>;
+
+// Whether one of two bfloat16 values is an infinity or NaN (its exponent all ones: adding the exponent's last bit carries
+// into the sign's place), and the pair with such values replaced by zero.
+__device__ __forceinline__ uint32_t odd(uint32_t pair) { return ((pair & 0x7f807f80u) + 0x00800080u) & 0x80008000u; }
+__device__ __forceinline__ uint32_t without_odd(uint32_t pair) {
+  const uint32_t o = odd(pair);
+  return pair & ~(((o >> 15) & 0x00010001u) * 0xffffu);
+}
 
 // The lowest n bits (n < 0: none; n > 31: all).
 __device__ __forceinline__ uint32_t below(int n) { return n <= 0 ? 0u : (n >= 32 ? 0xffffffffu : (1u << n) - 1u); }
@@ -111,6 +125,7 @@ attention_biased_tc_kernel(const __grid_constant__ CUtensorMap k_map, const __gr
   uint64_t* bar_q = bar_o + 1;                             // the query rows are in place
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(full_k + (PL::BARRIERS + 1) / 2 * 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  volatile int* odd_flag = abort_flag + 1;                 // a tile held infinities or NaN that not all rows may see
   float* max_x = reinterpret_cast<float*>(tmem_slot + 4);  // [tile & 1][2 halves][128 rows]
 
   // (two score maps a head, MAPS: a key row is [map 0 | map 1], a query [map 0 | map 1] too; a block takes one of them)
@@ -146,6 +161,7 @@ attention_biased_tc_kernel(const __grid_constant__ CUtensorMap k_map, const __gr
     mbar_init(bar_o, 1);
     mbar_init(bar_q, SOFTMAX_THREADS);
     *abort_flag = 0;
+    *odd_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == MMA_WARP) {
@@ -163,6 +179,11 @@ attention_biased_tc_kernel(const __grid_constant__ CUtensorMap k_map, const __gr
   const int j_lo = j_first & ~(box - 1);
   const int keep_end = a.keep > 0 ? min(a.keep, j_lo) : 0;
   const int kept = (keep_end + TK - 1) / TK;
+  // Keys [lo_all, hi_all] are seen by every row (its last row sees the fewest from below, its first from above); of those outside
+  // them [j_first, j_hi] are seen by some.
+  const int hi_all = prefix + row0 / G;
+  int lo_all = a.window > 0 ? max(0, j_hi - a.window + 1) : 0;
+  if (a.block_of > 0) lo_all = max(lo_all, j_hi / a.block_of * a.block_of);
   const int n_tiles = (seq_len > 0 && j_hi >= j_lo) ? kept + (j_hi - j_lo) / TK + 1 : 0;
   // Tiles are taken from the last to the first: with a bias that falls with the distance, and mostly without one, a row's
   // largest score comes early, and the reference that its exponentials refer to then stays where it is.
@@ -390,18 +411,26 @@ attention_biased_tc_kernel(const __grid_constant__ CUtensorMap k_map, const __gr
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       tc_fence_after();
-      // clear the value rows of keys the block must not see (the first and the last tile of a stretch of keys only)
-      if (jt + TK - 1 > j_end || (u == kept && jt < j_first)) {
+      // Value rows of keys the block must not see are cleared (the first and the last tile of a stretch of keys only); what is
+      // not finite among those that only some of its rows see is taken out.  (The kept first tokens are seen by all.)
+      const bool partial = u >= kept && ((hi_all < j_hi && jt + TK - 1 > hi_all) || (lo_all > j_first && jt < lo_all));
+      if (partial || jt + TK - 1 > j_end || (u == kept && jt < j_first)) {
         unsigned char* vt = V_IN_K ? k_s + (t % STAGES) * K_BYTES + chunk * VB * BLK_KV : v_s + (t % STAGES) * V_BYTES;
-        if (!V_IN_K) {
-          ok = mbar_wait_spin(&full_v[t % STAGES], (uint32_t)((t / STAGES) & 1), a.status, 14, abort_flag);
-          ok = __all_sync(0xffffffffu, ok);
-          if (!ok) break;
-        }
+        ok = mbar_wait_spin(&full_v[t % STAGES], (uint32_t)((t / STAGES) & 1), a.status, 14, abort_flag);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
         for (int i = tid; i < TK * VB * 8; i += SOFTMAX_THREADS) {
           const int key = i / (VB * 8), c = i % (VB * 8), j = jt + key;
-          if (j > j_end || (j < j_first && u >= kept && j >= a.keep))
-            *reinterpret_cast<uint4*>(vt + (c >> 3) * BLK_KV + key * 128 + (c & 7) * 16) = make_uint4(0u, 0u, 0u, 0u);
+          uint4* at = reinterpret_cast<uint4*>(vt + (c >> 3) * BLK_KV + key * 128 + (c & 7) * 16);
+          if (j > j_end || (j < j_first && u >= kept && j >= a.keep)) {
+            *at = make_uint4(0u, 0u, 0u, 0u);
+          } else if (partial) {
+            const uint4 v = *at;
+            if (odd(v.x) | odd(v.y) | odd(v.z) | odd(v.w)) {
+              *at = make_uint4(without_odd(v.x), without_odd(v.y), without_odd(v.z), without_odd(v.w));
+              *odd_flag = 1;
+            }
+          }
         }
         fence_async_smem();                                // (before this thread's arrival for P(t), which the product waits for)
       }
@@ -548,6 +577,26 @@ attention_biased_tc_kernel(const __grid_constant__ CUtensorMap k_map, const __gr
           for (int i = 0; i < 16; ++i) x[i] = y[i] = 0u;
         }
         if (!row_ok) continue;
+        if (*odd_flag) {
+          // what the tiles of partly seen keys held that is no number, for the keys that this row sees (other tiles' keys it
+          // may add once more: an infinity or NaN stays what it is)
+          const int lo_end = lo_all > j_first ? lo_all + TK - 2 : j_lo - 1, hi_first = hi_all - TK + 2;
+          for (int j = j_lo; j <= pos; ++j) {
+            if (j > lo_end && j < hi_first) {
+              j = hi_first;
+              if (j > pos) break;
+            }
+            if (j < lo && j >= a.keep) continue;
+            const int page = a.block_tables[(size_t)b * a.table_width + j / a.page];
+            const bf16* v = a.values + ((size_t)(page * a.KVH + kvh) * a.page + j % a.page) * a.value_row + chunk * DV + c;
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+              const float vx = to_f(v[i]), vy = to_f(v[DV / 2 + i]);
+              if (!isfinite(vx)) x[i] = __float_as_uint(__uint_as_float(x[i]) + vx);
+              if (!isfinite(vy)) y[i] = __float_as_uint(__uint_as_float(y[i]) + vy);
+            }
+          }
+        }
         if (MAPS) {
           float* dst32 = a.out32 + (size_t)(qs + tok) * a.out_ts + (size_t)head * a.out_hs + (MAPS && map_col ? DV : 0);
 #pragma unroll
@@ -691,6 +740,8 @@ TS_API int ts_attention_biased_tc(void* out, int out_ts, int out_hs, const void*
   a.out32 = nullptr;
   a.min_rows = 0;
   a.q = (const bf16*)q;
+  a.values = (const bf16*)(v_in_k ? k_cache : v_cache);
+  a.value_row = v_in_k ? Dk : Dv;
   a.block_tables = block_tables;
   a.q_start = q_start;
   a.seq_lens = seq_lens;
@@ -756,6 +807,8 @@ TS_API int ts_attention_maps_tc(void* out, float* maps, const void* proj, int pr
   Args a = {};
   a.out32 = maps;
   a.q = (const bf16*)proj;
+  a.values = (const bf16*)v_cache;
+  a.value_row = V;
   a.block_tables = block_tables;
   a.q_start = q_start;
   a.seq_lens = seq_lens;
