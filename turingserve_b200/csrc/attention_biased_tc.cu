@@ -310,7 +310,7 @@ attention_biased_tc_kernel(const __grid_constant__ CUtensorMap k_map, const __gr
           const uint64_t vd = v_desc + (kk * 16 * 128 >> 4);
           const uint32_t hi = p + kk / (KT / 16) * KT + kk % (KT / 16) * 8;
           umma_ts(tmem + O_COL, hi, vd, idesc, (t > 0 || kk > 0) ? 1u : 0u);
-          if (!MAPS) umma_ts(tmem + O_COL, hi + KT / 2, vd, idesc, 1u);
+          umma_ts(tmem + O_COL, hi + KT / 2, vd, idesc, 1u);
         }
         umma_commit(&empty_v[t % STAGES]);
         umma_commit(bar_pv);
@@ -484,13 +484,12 @@ attention_biased_tc_kernel(const __grid_constant__ CUtensorMap k_map, const __gr
           rs[i & 1] += p0 + p1;
           const __nv_bfloat162 h2 = __floats2bfloat162_rn(p0, p1);
           sv[i] = *reinterpret_cast<const uint32_t*>(&h2);
-          if (MAPS) continue;
           const __nv_bfloat162 l2 = __floats2bfloat162_rn(p0 - __uint_as_float(sv[i] << 16), p1 - __uint_as_float(sv[i] & 0xffff0000u));
           lw[i] = *reinterpret_cast<const uint32_t*>(&l2);
         }
 #pragma unroll
         for (int i = 0; i < KT / 2; ++i)
-          if (!MAPS) sv[KT / 2 + i] = lw[i];
+          sv[KT / 2 + i] = lw[i];
         return rs[0] + rs[1];
       };
       // The reference moves rarely once a row has one: the exponentials are taken against the present one while the other
@@ -530,7 +529,7 @@ attention_biased_tc_kernel(const __grid_constant__ CUtensorMap k_map, const __gr
         }
       }
 #pragma unroll
-      for (int h = 0; h < (MAPS ? KT / 64 : KT / 32); ++h) // over this thread's own scores
+      for (int h = 0; h < KT / 32; ++h)                    // over this thread's own scores
         tmem_st32(s_addr + hh * KT + h * 32, reinterpret_cast<uint32_t(&)[32]>(sv[h * 32]));
       tmem_wait_st();                                      // P (and a rescaled O) are in tensor memory
       tc_fence_before();
@@ -657,8 +656,9 @@ int launch(dim3 grid, cudaStream_t stream, const CUtensorMap& k_map, const CUten
 }
 
 // Two score maps a head (attention_diff.cu): every map of every kv head is a block's work like any other head's, with keys 64
-// columns of the 128-wide key row; the weights are one bfloat16, as in attention_diff_mma.cu, so one product; the two outputs
-// stay in 32-bit until the kernel below has joined them.  2,048 tokens, 12 heads over 2: 154 -> 51 us with the join, whole mixer 193 -> 90 us.
+// columns of the 128-wide key row.  The weights are two bfloat16 terms here too, although attention_diff_mma.cu has one: there the
+// largest weight of a row is an exact 1, here it refers to a maximum that may lag behind, and with one term the outputs were
+// up to 1.6 times further from 64 bits.  The two outputs stay in 32-bit until the kernel below has joined them.  2,048 tokens, 12 heads over 2: 154 -> 51 us with the join, whole mixer 193 -> 90 us.
 // out[t, h] = out_scale * rms_norm(a_0 - lambda a_1) of the two maps' outputs, a warp a head; tokens of requests of min_rows
 // rows or fewer are left alone.
 template <int V>
