@@ -412,7 +412,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
               uint4 pack;
               bf16* e = reinterpret_cast<bf16*>(&pack);
 #pragma unroll
-              for (int i = 0; i < 8; ++i) e[i] = from_f<bf16>(ts_activate_for<bf16>(round_to<bf16>(f[i]), args.act));
+              for (int i = 0; i < 8; ++i) {        // (rounded first; the same functions as the activation kernel's)
+                const float z = round_to<bf16>(f[i]);
+                e[i] = from_f<bf16>(args.act == TS_ACT_GELU ? ts_gelu(z) : ts_activate(z, args.act));
+              }
               *reinterpret_cast<uint4*>(args.out + (size_t)row * args.N + col) = pack;
             }
           }
