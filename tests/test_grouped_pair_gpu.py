@@ -89,3 +89,41 @@ def test_activations_of_products_are_those_of_the_activation_kernel(ops):
         assert bool(((out[:, 0].double() - true).abs() <= (2.0 ** -8 + 2.0 ** -15) * true.abs() + 1e-37).all())
     assert ops.tc_status() == 0
 
+
+
+def test_refused_launches_go_to_the_older_kernels(ops, monkeypatch):
+    """Where the device refuses the products on pairs (at the first or at the second) the feed-forward takes the way it had."""
+    from turingserve_b200.models import gugezen
+    from turingserve_b200.parts.base import BuildContext, build
+    mixer = {"type": "mamba2", "mixer": {"heads": 4, "vdim": 16, "state": 16, "groups": 1, "conv": 4, "norm_groups": 1}}
+    mlp = {"kind": "moe", "expert": {"ff": 72}, "router": {"experts": 4, "top": 2}, "shared": {"ff": 32}}
+    cfg = gugezen.make_config(width=64, vocab=64, layers=[{**mixer, "mlp": mlp}], eps=1e-6, streams=2)
+    part = build("feed_forward", cfg.layers[0].feed_forward,
+                 BuildContext(hidden_size=64, dtype=torch.bfloat16, device=torch.device(DEV, 0), max_positions=64))
+    g = torch.Generator(device=DEV).manual_seed(3)
+    rnd = lambda *s: torch.randn(*s, generator=g, device=DEV) * 0.1
+    w = {"router": rnd(4, 64), "shared.up": rnd(32, 64).bfloat16(), "shared.down": rnd(64, 32).bfloat16()}
+    for e in range(4):
+        w[f"e{e}.up"], w[f"e{e}.down"] = rnd(72, 64).bfloat16(), rnd(64, 72).bfloat16()
+    part.load(w)
+    real = ops.lib
+    for T in (90, 700):                                    # the grouped kernels, a product an expert
+        x = rnd(T, 64).mul(10).bfloat16()
+        assert ops.grouped_pair_takes(x, part.w_up, part.w_down, 2 * T)
+        want = ops.materialize(part.forward(x)).clone()
+        for refused_from in (0, 1):
+            class Lib:
+                calls = 0
+
+                def __getattr__(self, name):
+                    return getattr(real, name)
+
+                def ts_grouped_pair(self, *args):
+                    Lib.calls += 1
+                    return ops.UNSUPPORTED if Lib.calls > refused_from else real.ts_grouped_pair(*args)
+
+            with monkeypatch.context() as m:
+                m.setattr(ops, "lib", Lib())
+                got = ops.materialize(part.forward(x))
+            assert Lib.calls == refused_from + 1
+            assert torch.allclose(got.double(), want.double(), rtol=2 ** -6, atol=2 ** -6 * float(want.abs().max()))

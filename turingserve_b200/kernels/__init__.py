@@ -1127,7 +1127,9 @@ class CudaOps:
     # From this many (token, choice) pairs an expert (and 128 in all) the experts' products run on pairs of SMs over gathered
     # rows.  8 experts of 1,536 x 2,688, the whole feed-forward captured: 64 pairs 119 us against 94 of the grouped kernels, 128
     # pairs 115 against 129, 1,024 pairs 111 against 197, 4,096 pairs 197 against 510; of 3,584 x 7,104: 32 pairs 227 against
-    # 192, 64 pairs 246 against 289, 128 pairs 250 against 428, 4,096 pairs 594 against 2,522 us.
+    # 192, 64 pairs 246 against 289, 128 pairs 250 against 428, 4,096 pairs 594 against 2,522 us.  Outside a capture, from 1,024
+    # pairs on, it stands in for a product an expert: 3,584 x 7,104, 1,024 pairs 241 against 456, 4,096 pairs 523 against 626; 64
+    # experts of 1,536 x 512, 1,536 pairs 158 against 1,917; 256 of 1,536 x 256, 4,096 pairs 450 against 7,343 us.
     grouped_pair_rows = int(os.environ.get("TURINGSERVE_B200_GROUPED_PAIR_ROWS", "16"))
 
     def grouped_pair_takes(self, x, w_up, w_down, pairs: int) -> bool:
@@ -1139,16 +1141,20 @@ class CudaOps:
                 and all(w.dtype == x.dtype and w.is_contiguous() and w.data_ptr() % 16 == 0
                         and self.lib.ts_grouped_pair_supported(*w.shape) for w in (w_up, w_down)))
 
-    def grouped_pair(self, out, x, w, offsets, act: str = "none", glu=None) -> None:
+    def grouped_pair(self, out, x, w, offsets, act: str = "none", glu=None) -> bool:
         """out rows = x rows @ w[e]^T for the rows [offsets[e], offsets[e + 1]) of each expert (x bfloat16 [P, K] sorted by
         expert, w [E, N, K]); ``out`` float32 [P, N], or bfloat16: [P, N] through ``act``, or [P, N / 2] through the clamped gated
-        unit ``glu`` (limit, slope, offset) of neighbouring columns.  Rows behind the last expert's are left alone."""
+        unit ``glu`` (limit, slope, offset) of neighbouring columns.  Rows behind the last expert's are left alone.  False: the
+        device refuses the launch (no pair of blocks fits it, no tensor map), nothing was done."""
         E, N, K = w.shape
         epilogue = 5 if out.dtype == torch.float32 else (4 if glu is not None else 3)
         limit, slope, offset = glu if glu is not None else (0.0, 0.0, 0.0)
-        self._check(self.lib.ts_grouped_pair(_ptr(out), _ptr(x), _ptr(w), _ptr(offsets), x.shape[0], E, N, K, epilogue,
-                                             self.ACTIVATIONS[act], float(limit), float(slope), float(offset), self._stream()),
-                    "grouped_pair")
+        rc = self.lib.ts_grouped_pair(_ptr(out), _ptr(x), _ptr(w), _ptr(offsets), x.shape[0], E, N, K, epilogue,
+                                      self.ACTIVATIONS[act], float(limit), float(slope), float(offset), self._stream())
+        if rc == self.UNSUPPORTED:
+            return False
+        self._check(rc, "grouped_pair")
+        return True
 
     def glu_pairs(self, out, gu, glu) -> None:
         """out [T, I] = the clamped gated unit of the column pairs (2 i, 2 i + 1) of ``gu`` [T, 2 I] (see ``grouped_glu``);

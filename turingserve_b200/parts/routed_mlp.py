@@ -18,7 +18,7 @@ captured step.  The experts' weights are stacked [E, ff, hidden] and [E, hidden,
 
 More rows, bfloat16: the input rows are gathered in sorted order and both products run over the groups on pairs of SMs
 (``ops().grouped_pair``), nothing read back, captured or not.  What that kernel does not take (32-bit, over 256 experts, widths
-that are no multiple of 8) and has many rows (``LIBRARY_ROWS`` pairs or more, outside a capture): the group sizes are read back
+that are no multiple of 8, a device that refuses the launch) and has many rows (``LIBRARY_ROWS`` pairs or more, outside a capture): the group sizes are read back
 once and every expert's gathered rows go through ``ops().linear`` as a product of their own.  (With a table the host counts the
 groups itself from the step's ids, and nothing is read back.)
 
@@ -202,11 +202,11 @@ class RoutedMLP(FeedForward):
             xs = torch.empty((T * top, self.hidden), dtype=x.dtype, device=x.device)
             ops.moe_gather(xs, x, order, scale, top)
             a = torch.empty((T * top, self.inter if self.glu else up_width), dtype=x.dtype, device=x.device)
-            ops.grouped_pair(a, xs, self.w_up, offsets, "none" if self.gated else self.activation, self.glu_args if self.glu else None)
-            if self.gated and not self.glu:
-                a = self._activate(a, T * top)
-            ops.grouped_pair(y, a, self.w_down, offsets)
-            return y
+            if ops.grouped_pair(a, xs, self.w_up, offsets, "none" if self.gated else self.activation, self.glu_args if self.glu else None):
+                if self.gated and not self.glu:
+                    a = self._activate(a, T * top)
+                if ops.grouped_pair(y, a, self.w_down, offsets):
+                    return y
         if T * top >= self.LIBRARY_ROWS and x.is_cuda and not torch.cuda.is_current_stream_capturing():
             # the experts' input rows in sorted order, weighted and rounded once (the products then read plain rows)
             xs = torch.empty((T * top, self.hidden), dtype=x.dtype, device=x.device)
