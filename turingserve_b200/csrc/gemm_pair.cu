@@ -53,7 +53,7 @@ template <int BN> struct PairTile {
   static constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
 };
 
-enum PairEpilogue : int { EPI_PLAIN = 0, EPI_GATED = 1, EPI_QKV = 2, EPI_GROUP = 3, EPI_GROUP_GLU = 4, EPI_GROUP_F32 = 5 };
+enum PairEpilogue : int { EPI_PLAIN = 0, EPI_GATED = 1, EPI_QKV = 2, EPI_GROUP = 3, EPI_GROUP_GLU = 4, EPI_GROUP_F32 = 5, EPI_GROUP_GELU = 6 };
 constexpr bool grouped_epilogue(int epi) { return epi >= EPI_GROUP; }
 constexpr int MAX_EXPERTS = 256;
 
@@ -412,9 +412,17 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
               uint4 pack;
               bf16* e = reinterpret_cast<bf16*>(&pack);
 #pragma unroll
-              for (int i = 0; i < 8; ++i) {        // (rounded first; the same functions as the activation kernel's)
-                const float z = round_to<bf16>(f[i]);
-                e[i] = from_f<bf16>(args.act == TS_ACT_GELU ? ts_gelu(z) : ts_activate(z, args.act));
+              for (int i = 0; i < 8; ++i) f[i] = round_to<bf16>(f[i]);  // (rounded first; the same functions as the activation kernel's)
+              if constexpr (EPI == EPI_GROUP_GELU) {
+#pragma unroll
+                for (int i = 0; i < 8; i += 2) {
+                  const float2 g = ts_gelu2(make_float2(f[i], f[i + 1]));
+                  e[i] = from_f<bf16>(g.x);
+                  e[i + 1] = from_f<bf16>(g.y);
+                }
+              } else {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) e[i] = from_f<bf16>(ts_activate(f[i], args.act));
               }
               *reinterpret_cast<uint4*>(args.out + (size_t)row * args.N + col) = pack;
             }
@@ -643,6 +651,8 @@ TS_API int ts_grouped_pair(void* out, const void* x, const void* w, const int* o
   a.act = act;
   a.glu = TsGlu{limit, slope, offset};
   cudaStream_t s = (cudaStream_t)stream;
+  // (GELU by an instance of its own: the choice between the activations costs the epilogue more than most of them do)
+  if (epilogue == EPI_GROUP && act == TS_ACT_GELU) return launch_pair_any<EPI_GROUP_GELU>(x, w, a, s);
   if (epilogue == EPI_GROUP) return launch_pair_any<EPI_GROUP>(x, w, a, s);
   if (epilogue == EPI_GROUP_GLU) return launch_pair_any<EPI_GROUP_GLU>(x, w, a, s);
   if (epilogue == EPI_GROUP_F32) return launch_pair_any<EPI_GROUP_F32>(x, w, a, s);
