@@ -81,6 +81,16 @@ __device__ __forceinline__ float block_sum(float v, float* scratch) {
 
 static inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
+// SMs of the current device (1 if that cannot be read).
+inline int ts_sm_count() {
+  static const int sms = [] {
+    int n = 1, dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) n = 1;
+    return n;
+  }();
+  return sms;
+}
+
 // What an attention kernel does to a head's output on its way to memory: the pairs (m, m + Dv/2) turned by -position *
 // out_freq[m] (null: not), then the head times sigmoid(gate[token * gate_ts + head]) (null: not).
 struct AttnFinish {

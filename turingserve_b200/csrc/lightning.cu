@@ -26,7 +26,9 @@ constexpr int LT_ROWS = 8;       // state rows per thread (registers)
 
 template <typename T> __device__ __forceinline__ float act_silu(float z) { return round_to<T>(silu_for<T>(z)); }
 
-template <typename T>
+// PLAN: an instance of its own for portions (its per-thread plan of copies and activations costs 60 registers more, which
+// halves the threads an SM holds: see ts_lightning_ex for where it pays)
+template <typename T, bool PLAN>
 __global__ void __launch_bounds__(512)
 lightning_kernel(float* __restrict__ out, const T* __restrict__ proj, int proj_stride, float* __restrict__ state,
                  const float* __restrict__ decay, const int* __restrict__ q_start, const int* __restrict__ slots,
@@ -61,8 +63,62 @@ lightning_kernel(float* __restrict__ out, const T* __restrict__ proj, int proj_s
   const int raw_row = 2 * D + LT_COLS;
   const int cols_here = min(LT_COLS, V - (int)blockIdx.x * LT_COLS);
   constexpr int PER16 = 16 / (int)sizeof(T);
+  // Which pieces of a group a thread copies, and which it activates, is the same for every group: with PLAN both are
+  // worked out once instead of by two divisions a piece and group.  At most LT_MAX_COPIES 16-byte copies a thread (16 rows
+  // of 2 D / PER16 + LT_COLS / PER16 pieces over 2 D threads) and LT_MAX_ACT pieces to activate.
+  constexpr int LT_MAX_COPIES = 8, LT_MAX_ACT = 4;
+  int cp_row[LT_MAX_COPIES], cp_src[LT_MAX_COPIES], cp_dst[LT_MAX_COPIES];
+  int ac_row[LT_MAX_ACT], ac_src[LT_MAX_ACT], ac_dst[LT_MAX_ACT];
+  const bool planned = PLAN && fast_rows;
+  if (planned) {
+    const int chunks_qk = D / PER16, chunks_v = LT_COLS / PER16, per_row = 2 * chunks_qk + chunks_v;
+#pragma unroll
+    for (int k = 0; k < LT_MAX_COPIES; ++k) {
+      const int i = threadIdx.x + k * blockDim.x;
+      cp_row[k] = LT_GROUP;                                // (beyond every group: never copied)
+      cp_src[k] = cp_dst[k] = 0;
+      if (i < LT_GROUP * per_row) {
+        const int r = i / per_row, c = i % per_row;
+        if (c < chunks_qk) {
+          cp_row[k] = r;
+          cp_src[k] = r * proj_stride + q_off + c * PER16;
+          cp_dst[k] = r * raw_row + c * PER16;
+        } else if (c < 2 * chunks_qk) {
+          cp_row[k] = r;
+          cp_src[k] = r * proj_stride + k_off + (c - chunks_qk) * PER16;
+          cp_dst[k] = r * raw_row + D + (c - chunks_qk) * PER16;
+        } else if ((c - 2 * chunks_qk) * PER16 < cols_here) {
+          cp_row[k] = r;
+          cp_src[k] = r * proj_stride + v_off + blockIdx.x * LT_COLS + (c - 2 * chunks_qk) * PER16;
+          cp_dst[k] = r * raw_row + 2 * D + (c - 2 * chunks_qk) * PER16;
+        }
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < LT_MAX_ACT; ++k) {
+      const int i = threadIdx.x + k * blockDim.x;
+      ac_row[k] = LT_GROUP;
+      ac_src[k] = ac_dst[k] = 0;
+      if (i < LT_GROUP * 2 * chunks_qk) {
+        const int r = i / (2 * chunks_qk), c = i % (2 * chunks_qk);
+        const int which = c >= chunks_qk, cc = (which ? c - chunks_qk : c) * PER16;
+        ac_row[k] = r;
+        ac_src[k] = r * raw_row + which * D + cc;
+        ac_dst[k] = which * LT_GROUP * Dp + r * Dp + cc;   // (k_s lies LT_GROUP * Dp behind q_s)
+      }
+    }
+  }
   auto fetch = [&](int g0, int buf) {
     if (!fast_rows) return;
+    if (planned) {
+      const int gn = min(LT_GROUP, n - g0);
+      const T* first = proj + (size_t)(t0 + g0) * proj_stride;
+      T* dst0 = raw + (size_t)buf * LT_GROUP * raw_row;
+#pragma unroll
+      for (int k = 0; k < LT_MAX_COPIES; ++k)
+        if (cp_row[k] < gn) cp_async_16(dst0 + cp_dst[k], first + cp_src[k], true);
+      return;
+    }
     const int gn = min(LT_GROUP, n - g0);
     const int chunks_qk = D / PER16, chunks_v = LT_COLS / PER16, per_row = 2 * chunks_qk + chunks_v;
     for (int i = threadIdx.x; i < gn * per_row; i += blockDim.x) {
@@ -88,7 +144,19 @@ lightning_kernel(float* __restrict__ out, const T* __restrict__ proj, int proj_s
     cp_async_commit();
     cp_async_wait<1>();
     __syncthreads();                                       // this group's raw rows are here; the group before is stored
-    if (fast_rows) {
+    if (planned) {
+      const T* raw0 = raw + (size_t)buf * LT_GROUP * raw_row;
+#pragma unroll
+      for (int k = 0; k < LT_MAX_ACT; ++k) {
+        if (ac_row[k] < gn) {
+          const uint4 rawv = *reinterpret_cast<const uint4*>(raw0 + ac_src[k]);
+          const T* e = reinterpret_cast<const T*>(&rawv);
+          float* dst = q_s + ac_dst[k];
+#pragma unroll
+          for (int u = 0; u < PER16; ++u) dst[u] = act_silu<T>(to_f(e[u]));
+        }
+      }
+    } else if (fast_rows) {
       // 16 bytes (PER16 values) of q or k at a time: the index arithmetic once a piece, not once a value
       const int chunks = D / PER16;
       for (int i = threadIdx.x; i < gn * 2 * chunks; i += blockDim.x) {
@@ -144,7 +212,7 @@ lightning_kernel(float* __restrict__ out, const T* __restrict__ proj, int proj_s
       const int r = i / LT_COLS, c = i % LT_COLS;
       const int jj = blockIdx.x * LT_COLS + c;
       if (jj >= V) continue;
-      out[(size_t)(t0 + g0 + r) * H * V + h * V + jj] = scan::tree_of_parts(o_s + r * parts * LT_COLS + c, parts, LT_COLS);
+      out[(size_t)(t0 + g0 + r) * H * V + h * V + jj] = scan::tree_of_parts<PLAN>(o_s + r * parts * LT_COLS + c, parts, LT_COLS);
     }
   }
   cp_async_wait<0>();
@@ -316,24 +384,24 @@ lightning_long_kernel(float* __restrict__ out, const float* __restrict__ ready, 
 
 // proj: [T, proj_stride] rows holding q at column 0, k at H D, v at 2 H D.  state: [slots, H, D, V] 32-bit.
 // decay: [H] 32-bit on the device.  out: [T, H V] 32-bit.
-// longest: the most tokens a request brings (0: not known); from LT_LATE_TOKENS on the kernel is launched late (see
-// ts_launch_late).
+// T: tokens of all requests.  longest: the most tokens a request brings (0: not known); from LT_LATE_TOKENS on the kernel is
+// launched late (see ts_launch_late).
 // ts_lightning_long takes portions from LL_TOKENS on where ts_lightning_long_supported says so, with ready [T, H (2 D + V)]
 // 32-bit as work memory; outputs and states are the same bits.  (From how
 // many tokens on its second launch pays is the caller's to say.)
 constexpr int LT_LATE_TOKENS = 64, LL_TOKENS = 128;
 
 TS_API int ts_lightning_ex(float* out, const void* proj, int proj_stride, float* state, const float* decay,
-                           const int* q_start, const int* slots, int B, int H, int D, int V, int longest, int dtype,
+                           const int* q_start, const int* slots, int B, int T, int H, int D, int V, int longest, int dtype,
                            void* stream);
 
 TS_API int ts_lightning(float* out, const void* proj, int proj_stride, float* state, const float* decay,
                         const int* q_start, const int* slots, int B, int H, int D, int V, int dtype, void* stream) {
-  return ts_lightning_ex(out, proj, proj_stride, state, decay, q_start, slots, B, H, D, V, 0, dtype, stream);
+  return ts_lightning_ex(out, proj, proj_stride, state, decay, q_start, slots, B, 0, H, D, V, 0, dtype, stream);
 }
 
 TS_API int ts_lightning_ex(float* out, const void* proj, int proj_stride, float* state, const float* decay,
-                           const int* q_start, const int* slots, int B, int H, int D, int V, int longest, int dtype,
+                           const int* q_start, const int* slots, int B, int T, int H, int D, int V, int longest, int dtype,
                            void* stream) {
   if (B <= 0) return 0;
   if (H <= 0 || D <= 0 || V <= 0) TS_REFUSE(TS_ERR_SHAPE, "ts_lightning: %d heads of %d x %d", H, D, V);
@@ -348,19 +416,30 @@ TS_API int ts_lightning_ex(float* out, const void* proj, int proj_stride, float*
   const size_t smem = sizeof(float) * LT_GROUP * ((size_t)2 * parts * LT_ROWS + LT_COLS + (size_t)parts * LT_COLS) +
                       (size_t)2 * LT_GROUP * (2 * D + LT_COLS) * elem;
   dim3 grid(ceil_div(V, LT_COLS), H, B);
+  // Portions of 64 tokens or more go to the planned instance while the chip holds all its blocks at once (512 threads an SM).  6
+  // heads of 128 x 128, planned against lean: 127 tokens 24.1 / 26.9 us, 383 tokens of 6 requests 89 / 101, of 8 requests 147 /
+  // 136, 256 tokens beside 8 single ones 55 / 52; of 64 x 64, 383 tokens 58 / 75.  Keys over 128 wide count requests by their length,
+  // because one of their blocks fills an SM either way (383 tokens beside 8 single ones 98 / 106).
+  const long long room = 512LL * ts_sm_count(), threads = (long long)grid.x * H * parts * LT_COLS;
+  const bool planned = longest >= LT_LATE_TOKENS && (threads * B <= room || (parts > 16 && threads * T <= room * longest));
 #define TS_LT(TT)                                                                                                   \
   do {                                                                                                              \
     static size_t configured = 0;                                                                                   \
     if (smem > 48 * 1024 && smem > configured) {                                                                    \
-      cudaError_t e = cudaFuncSetAttribute(lightning_kernel<TT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+      cudaError_t e = cudaFuncSetAttribute(lightning_kernel<TT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+      if (e == cudaSuccess)                                                                                         \
+        e = cudaFuncSetAttribute(lightning_kernel<TT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
       if (e != cudaSuccess) TS_REFUSE((int)e, "ts_lightning: shared memory %zu: %s", smem, cudaGetErrorString(e)); \
       configured = smem;                                                                                            \
     }                                                                                                               \
-    if (longest >= LT_LATE_TOKENS)                                                                                  \
-      ts_launch_late(lightning_kernel<TT>, dim3(grid), dim3(parts * LT_COLS), smem, s, out, (const TT*)proj, proj_stride, \
+    if (planned)                                                                                                    \
+      ts_launch_late(lightning_kernel<TT, true>, dim3(grid), dim3(parts * LT_COLS), smem, s, out, (const TT*)proj, proj_stride, \
+                     state, decay, q_start, slots, H, D, V, parts, fast_rows);                                      \
+    else if (longest >= LT_LATE_TOKENS)                                                                             \
+      ts_launch_late(lightning_kernel<TT, false>, dim3(grid), dim3(parts * LT_COLS), smem, s, out, (const TT*)proj, proj_stride, \
                      state, decay, q_start, slots, H, D, V, parts, fast_rows);                                      \
     else                                                                                                            \
-      ts_launch(lightning_kernel<TT>, dim3(grid), dim3(parts * LT_COLS), smem, s, out, (const TT*)proj, proj_stride, \
+      ts_launch(lightning_kernel<TT, false>, dim3(grid), dim3(parts * LT_COLS), smem, s, out, (const TT*)proj, proj_stride, \
                 state, decay, q_start, slots, H, D, V, parts, fast_rows);                                           \
   } while (0)
   if (dtype == TS_F32) TS_LT(float);

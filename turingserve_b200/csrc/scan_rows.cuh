@@ -92,20 +92,24 @@ __device__ __forceinline__ float sum_scatter(float (&x)[16], int lane) {
 }
 
 // The sums of `parts` (at most 32) groups of eight rows, `stride` apart, as the tree above.
-__device__ __forceinline__ float tree_of_16(const float* p, int parts, int stride) {
-  float x[16];
+// FEW: with a way for few parts (planned instances: keys of 64 3 % faster, of 16 12 %; in the lean ones keys of 128 would lose 4 %).
+template <int MOST>
+__device__ __forceinline__ float tree_of(const float* p, int parts, int stride) {
+  float x[MOST];
 #pragma unroll
-  for (int i = 0; i < 16; ++i) x[i] = i < parts ? p[i * stride] : 0.f;
+  for (int i = 0; i < MOST; ++i) x[i] = i < parts ? p[i * stride] : 0.f;
 #pragma unroll
-  for (int n = 8; n > 0; n >>= 1)
+  for (int n = MOST / 2; n > 0; n >>= 1)
 #pragma unroll
     for (int i = 0; i < n; ++i) x[i] = x[2 * i] + x[2 * i + 1];
   return x[0];
 }
+template <bool FEW>
 __device__ __forceinline__ float tree_of_parts(const float* p, int parts, int stride) {
-  float x = tree_of_16(p, parts, stride);
-  if (parts > 16) x += tree_of_16(p + 16 * stride, parts - 16, stride);
-  return x;
+  if (FEW && parts <= 4) return tree_of<4>(p, parts, stride);              // (absent parts add nothing)
+  if (FEW && parts <= 8) return tree_of<8>(p, parts, stride);
+  const float x = tree_of<16>(p, parts, stride);
+  return parts > 16 ? x + tree_of<16>(p + 16 * stride, parts - 16, stride) : x;
 }
 
 }  // namespace scan

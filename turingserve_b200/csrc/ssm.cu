@@ -299,7 +299,7 @@ ssm_scan_kernel(float* __restrict__ out, const float* __restrict__ ready, const 
       const int r = i / SS_COLS, c = i % SS_COLS;
       const int jj = blockIdx.x * SS_COLS + c;
       if (jj >= P) continue;
-      out[(size_t)(t0 + g0 + r) * inner + h * P + jj] = scan::tree_of_parts(o_s + r * parts * SS_COLS + c, parts, SS_COLS);
+      out[(size_t)(t0 + g0 + r) * inner + h * P + jj] = scan::tree_of_parts<false>(o_s + r * parts * SS_COLS + c, parts, SS_COLS);
     }
   }
   cp_async_wait<0>();

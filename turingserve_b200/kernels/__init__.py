@@ -68,7 +68,7 @@ class LazyProduct:
 class CudaOps:
     """ctypes front of ``libturingserve_b200.so``."""
 
-    ABI = 20
+    ABI = 21
     UNSUPPORTED = -4            # a kernel's refusal of a shape or layout another kernel takes
 
     def __init__(self, lib_path: str) -> None:
@@ -123,7 +123,7 @@ class CudaOps:
             "ts_hyper_norm": [P, P, P, P, I, P, P, P, P, P, F, I, I, I, I, F, I, P],
             "ts_ssm_prepare": [P, P, I, I, I, P, P, P, P, P, ctypes.c_longlong, ctypes.c_longlong, P, P, P, I, I, I, I, I, P],
             "ts_ssm_scan": [P, P, P, I, I, P, ctypes.c_longlong, P, P, P, I, I, I, I, I, I, I, I, P],
-            "ts_lightning_ex": [P, P, I, P, P, P, P, I, I, I, I, I, I, P],
+            "ts_lightning_ex": [P, P, I, P, P, P, P, I, I, I, I, I, I, I, P],
             "ts_lightning_long": [P, P, I, P, P, P, P, P, I, I, I, I, I, I, I, P],
             "ts_lightning_long_supported": [I, I, I, I, I],
             "ts_gated_group_rmsnorm": [P, I, P, P, I, P, F, I, I, I, I, I, F, I, P],
@@ -651,7 +651,8 @@ class CudaOps:
     # Steps whose longest portion has at least this many tokens go to the two kernels for long portions (the scan takes the GPU a
     # third of the time a token, 54 against 165 ns with 6 heads of 128 x 128).  Their work memory and second launch cost the host
     # a few microseconds, and a mixer of fewer tokens waits for the host (three requests of 188 tokens, width 1,536: 130 us
-    # a call with them, 123 before them; its kernels take less).
+    # a call with them, 123 with the planned instance of the other kernel, which takes such portions; captured, the scan of 384
+    # tokens is 26.8 us here and 67.7 there).
     lightning_long_tokens = int(os.environ.get("TURINGSERVE_B200_LIGHTNING_LONG_TOKENS", "384"))
 
     def lightning(self, out, proj, state, decay, step, H: int, D: int, V: int) -> None:
@@ -659,7 +660,10 @@ class CudaOps:
         q, k, v = silu of the columns [0, HD), [HD, 2HD), [2HD, 2HD + HV) of ``proj``; ``state``
         (float32 [slots, H, D, V]) is read and left updated at each request's slot."""
         longest = int(getattr(step, "max_q_len", 0) or 0)
-        if longest >= self.lightning_long_tokens and self.lib.ts_lightning_long_supported(D, V, proj.stride(0), longest, _code(proj.dtype)):
+        # (a lane group of the long kernel holds a column whatever the keys' width, so that narrow keys leave lanes idle, which costs once
+        # the chip is full: 16 heads of 64 x 64, 384 tokens of 4 requests 77 us there and 68 here, of 8 requests 135 and 91)
+        roomy = D > 64 or -(-V // 8) * H * step.num_requests <= 3 * self.num_sms
+        if longest >= self.lightning_long_tokens and roomy and self.lib.ts_lightning_long_supported(D, V, proj.stride(0), longest, _code(proj.dtype)):
             ready = torch.empty((proj.shape[0], H * (2 * D + V)), dtype=torch.float32, device=proj.device)
             rc = self.lib.ts_lightning_long(_ptr(out), _ptr(proj), proj.stride(0), _ptr(ready), _ptr(state), _ptr(decay),
                                             _ptr(step.q_start), _ptr(step.state_slots), step.num_requests, proj.shape[0], H, D, V,
@@ -669,7 +673,7 @@ class CudaOps:
                 self._check(rc, "lightning_long")
                 return
         self._check(self.lib.ts_lightning_ex(_ptr(out), _ptr(proj), proj.stride(0), _ptr(state), _ptr(decay),
-                                             _ptr(step.q_start), _ptr(step.state_slots), step.num_requests, H, D, V,
+                                             _ptr(step.q_start), _ptr(step.state_slots), step.num_requests, proj.shape[0], H, D, V,
                                              longest, _code(proj.dtype), self._stream()),
                     "lightning")
 
