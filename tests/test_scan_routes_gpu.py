@@ -59,3 +59,17 @@ def test_linear_attention_portions(ops, H, D, V, lens):
     known, unknown = device_us(*(lambda s=s: ops.lightning(out, proj, state, decay, s, H, D, V) for s in (step_of(lens), step_of(lens, False))))
     assert known < 0.96 * unknown, (known, unknown)
 
+
+
+@pytest.mark.parametrize("H,P,N,lens", [(112, 64, 128, [64]), (112, 64, 128, [96]), (48, 64, 128, [64]), (48, 64, 64, [100]),
+                                        (32, 64, 16, [1] * 8 + [100])])
+def test_state_space_portions(ops, H, P, N, lens):
+    G, taps, T = 2, 4, sum(lens)
+    inner = H * P
+    channels = inner + 2 * G * N
+    ready, out = torch.rand(T, channels + 2 * H, device=DEV), torch.empty(T, inner, device=DEV)
+    proj = torch.randn(T, 2 * inner + 2 * G * N + H, device=DEV).bfloat16()
+    state, skip = torch.zeros(len(lens), H * N * P + 3 * channels, device=DEV), torch.ones(H, device=DEV)
+    known, unknown = device_us(*(lambda s=s: ops.ssm_scan(out, ready, proj, inner, state, skip, s, H, G, N, P, taps)
+                                 for s in (step_of(lens), step_of(lens, False))))
+    assert known < 1.03 * unknown, (known, unknown)

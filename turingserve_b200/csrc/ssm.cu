@@ -193,7 +193,9 @@ __device__ __forceinline__ void store_last_inputs(float* tail, const T* proj, in
   }
 }
 
-template <typename T>
+// PLAN: an instance of its own for portions (its per-thread copy plan costs 60 registers more, which would halve the
+// blocks an SM holds in single-token steps: 51 -> 59 us at 112 heads)
+template <typename T, bool PLAN>
 __global__ void __launch_bounds__(512)
 ssm_scan_kernel(float* __restrict__ out, const float* __restrict__ ready, const T* __restrict__ proj, int proj_stride,
                 int xbc_off, float* __restrict__ state, size_t state_stride, const float* __restrict__ skip,
@@ -226,13 +228,47 @@ ssm_scan_kernel(float* __restrict__ out, const float* __restrict__ ready, const 
   for (int i = threadIdx.x; i < 2 * stage; i += blockDim.x) smem[i] = 0.f;     // (what no copy writes stays zero)
   __syncthreads();
 
+  // Which pieces of a group a thread copies is the same for every group: with PLAN it is worked out
+  // once (the divisions of the index by the pieces a row would otherwise cost more instructions a group than the copies
+  // themselves; for a single token the plan itself is what costs: 28.7 -> 36.9 us).  16-byte pieces: at most
+  // SS_MAX_COPIES a thread (16 rows of N / 2 + 4 pieces over 16 ceil(N / 8) threads).
+  constexpr int SS_MAX_COPIES = 8;
+  int cp_row[SS_MAX_COPIES], cp_src[SS_MAX_COPIES], cp_dst[SS_MAX_COPIES];
+  if (PLAN && vec4) {
+    const int nb = N / 4, nx = cols_here / 4, per_row = 2 * nb + nx;
+#pragma unroll
+    for (int k = 0; k < SS_MAX_COPIES; ++k) {
+      const int i = threadIdx.x + k * blockDim.x;
+      cp_row[k] = SS_GROUP;                                // (beyond every group: never copied)
+      cp_src[k] = cp_dst[k] = 0;
+      if (i < SS_GROUP * per_row) {
+        const int r = i / per_row, c = i % per_row;
+        cp_row[k] = r;
+        if (c < nb) {
+          cp_src[k] = r * W + inner + g * N + 4 * c;
+          cp_dst[k] = r * Np + 4 * c;
+        } else if (c < 2 * nb) {
+          cp_src[k] = r * W + inner + GN + g * N + 4 * (c - nb);
+          cp_dst[k] = SS_GROUP * Np + r * Np + 4 * (c - nb);
+        } else {
+          cp_src[k] = r * W + h * P + blockIdx.x * SS_COLS + 4 * (c - 2 * nb);
+          cp_dst[k] = 2 * SS_GROUP * Np + r * SS_COLS + 4 * (c - 2 * nb);
+        }
+      }
+    }
+  }
   auto fetch = [&](int g0, int buf) {
     const int gn = min(SS_GROUP, n - g0);
     float* Bs = smem + (size_t)buf * stage;
     float* Cs = Bs + SS_GROUP * Np;
     float* xs = Cs + SS_GROUP * Np;
     float* da = xs + SS_GROUP * SS_COLS;
-    if (vec4) {
+    if (PLAN && vec4) {
+      const float* first = ready + (size_t)(t0 + g0) * W;
+#pragma unroll
+      for (int k = 0; k < SS_MAX_COPIES; ++k)
+        if (cp_row[k] < gn) cp_async_16(Bs + cp_dst[k], first + cp_src[k], true);
+    } else if (vec4) {
       const int nb = N / 4, nx = cols_here / 4, per_row = 2 * nb + nx;
       for (int i = threadIdx.x; i < gn * per_row; i += blockDim.x) {
         const int r = i / per_row, c = i % per_row;
@@ -299,7 +335,7 @@ ssm_scan_kernel(float* __restrict__ out, const float* __restrict__ ready, const 
       const int r = i / SS_COLS, c = i % SS_COLS;
       const int jj = blockIdx.x * SS_COLS + c;
       if (jj >= P) continue;
-      out[(size_t)(t0 + g0 + r) * inner + h * P + jj] = scan::tree_of_parts<false>(o_s + r * parts * SS_COLS + c, parts, SS_COLS);
+      out[(size_t)(t0 + g0 + r) * inner + h * P + jj] = scan::tree_of_parts<PLAN>(o_s + r * parts * SS_COLS + c, parts, SS_COLS);
     }
   }
   cp_async_wait<0>();
@@ -518,13 +554,29 @@ TS_API int ts_ssm_prepare(float* ready, const void* proj, int proj_stride, int x
 
 // out [T, H P] 32-bit; ready as ts_ssm_prepare left it; skip [H] 32-bit (D, may be null); state [slots, state_stride]:
 // [H N P | (taps - 1) x Cn], read and left updated at each request's slot.
-// longest: the most tokens a request brings (0: not known); from SS_LATE_TOKENS on the kernel is launched late (see
-// ts_launch_late).
+// T: tokens of all requests.  longest: the most tokens a request brings (0: not known); from SS_LATE_TOKENS on the kernel is
+// launched late (see ts_launch_late).
 constexpr int SS_LATE_TOKENS = 64;
 
+// Whether portions go to ssm_scan_long_kernel and not to the planned instance of the other (the same bits).  The long one has
+// more of a start and less of a token; a half warp of it holds a column whatever the state's rows, so that narrow states
+// leave lanes idle, which costs once the chip is full.  us, planned / long, heads of 64 x 128: 48 heads, 64 tokens 23.1 / 28.7,
+// 144 tokens 35.6 / 38.7, 160 tokens 39.3 / 38.9, 192 tokens 45.4 / 42.5, two of 128 tokens 43.2 / 41.0, four of 80 50.9 / 48.6; 112 heads, 64
+// tokens 33 / 51, 160 tokens 64.8 / 62.5.  48 heads of 64 x 64: 96 tokens 31.8 / 30.3, three requests of 160 tokens 49 / 58; 32
+// heads of 64 x 16: four of 128 tokens 67 / 44, eight of them 71 / 76.
+inline bool takes_long(int B, int T, int H, int N, int P, int longest) {
+  if (longest < SS_LATE_TOKENS) return false;
+  if (N > 64) return longest >= 160 || T >= (longest >= 128 ? 256 : 320);
+  // (requests count by their length where that is what the time goes by: single tokens beside a portion come and go)
+  const long long blocks = (long long)ceil_div(P, SS_COLS) * H, sms = ts_sm_count();
+  const bool one_wave = blocks * T <= 2 * sms * longest;
+  if (N > 32) return longest >= 300 ? one_wave : longest >= 96 && blocks * B <= 2 * sms;
+  return one_wave || (longest <= 384 && blocks * T <= 5 * sms * longest);
+}
+
 TS_API int ts_ssm_scan(float* out, const float* ready, const void* proj, int proj_stride, int xbc_off, float* state,
-                       long long state_stride, const float* skip, const int* q_start, const int* slots, int B, int H,
-                       int G, int N, int P, int taps, int longest, int dtype, void* stream) {
+                       long long state_stride, const float* skip, const int* q_start, const int* slots, int B, int T,
+                       int H, int G, int N, int P, int taps, int longest, int dtype, void* stream) {
   if (B <= 0) return 0;
   if (H <= 0 || G <= 0 || H % G || N <= 0 || P <= 0) TS_REFUSE(TS_ERR_SHAPE, "ts_ssm_scan: %d heads in %d groups, state %d x %d", H, G, N, P);
   if (taps < 1 || taps > SS_MAX_TAPS) TS_REFUSE(TS_ERR_LIMIT, "ts_ssm_scan: a filter of %d taps (1 to %d)", taps, SS_MAX_TAPS);
@@ -536,7 +588,7 @@ TS_API int ts_ssm_scan(float* out, const float* ready, const void* proj, int pro
   // 16-byte copies: every piece of a row (B, C, this block's x columns) on a 16-byte boundary
   const int vec4 = N % 4 == 0 && P % 4 == 0 && W % 4 == 0 && !((uintptr_t)ready & 15);
   const size_t smem = sizeof(float) * ((size_t)2 * SS_GROUP * (2 * parts * SS_ROWS + SS_COLS + 4) + (size_t)SS_GROUP * parts * SS_COLS);
-  if (longest >= SS_LATE_TOKENS && vec4) {
+  if (vec4 && takes_long(B, T, H, N, P, longest)) {
 #define TS_SL(TT, RR)                                                                                                   \
   do {                                                                                                                  \
     constexpr size_t bytes = sizeof(float) * SL_STAGES * SS_GROUP * (2 * 16 * RR + SL_COLS + 4);                        \
@@ -567,15 +619,17 @@ TS_API int ts_ssm_scan(float* out, const float* ready, const void* proj, int pro
   do {                                                                                                                  \
     static size_t configured = 0;                                                                                       \
     if (smem > 48 * 1024 && smem > configured) {                                                                        \
-      cudaError_t e = cudaFuncSetAttribute(ssm_scan_kernel<TT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+      cudaError_t e = cudaFuncSetAttribute(ssm_scan_kernel<TT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+      if (e == cudaSuccess)                                                                                             \
+        e = cudaFuncSetAttribute(ssm_scan_kernel<TT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);    \
       if (e != cudaSuccess) TS_REFUSE((int)e, "ts_ssm_scan: shared memory %zu: %s", smem, cudaGetErrorString(e));       \
       configured = smem;                                                                                                \
     }                                                                                                                   \
     if (longest >= SS_LATE_TOKENS)                                                                                      \
-      ts_launch_late(ssm_scan_kernel<TT>, grid, dim3(parts * SS_COLS), smem, s, out, ready, (const TT*)proj, proj_stride, xbc_off, \
+      ts_launch_late(ssm_scan_kernel<TT, true>, grid, dim3(parts * SS_COLS), smem, s, out, ready, (const TT*)proj, proj_stride, xbc_off, \
                      state, (size_t)state_stride, skip, q_start, slots, H, G, N, P, taps, parts, vec4);                 \
     else                                                                                                                \
-      ts_launch(ssm_scan_kernel<TT>, grid, dim3(parts * SS_COLS), smem, s, out, ready, (const TT*)proj, proj_stride, xbc_off, \
+      ts_launch(ssm_scan_kernel<TT, false>, grid, dim3(parts * SS_COLS), smem, s, out, ready, (const TT*)proj, proj_stride, xbc_off, \
                 state, (size_t)state_stride, skip, q_start, slots, H, G, N, P, taps, parts, vec4);                      \
   } while (0)
   if (dtype == TS_F32) TS_SC(float);

@@ -68,7 +68,7 @@ class LazyProduct:
 class CudaOps:
     """ctypes front of ``libturingserve_b200.so``."""
 
-    ABI = 21
+    ABI = 22
     UNSUPPORTED = -4            # a kernel's refusal of a shape or layout another kernel takes
 
     def __init__(self, lib_path: str) -> None:
@@ -122,7 +122,7 @@ class CudaOps:
             "ts_moe_combine": [P, P, P, P, I, I, I, I, P, P, P, P, P],
             "ts_hyper_norm": [P, P, P, P, I, P, P, P, P, P, F, I, I, I, I, F, I, P],
             "ts_ssm_prepare": [P, P, I, I, I, P, P, P, P, P, ctypes.c_longlong, ctypes.c_longlong, P, P, P, I, I, I, I, I, P],
-            "ts_ssm_scan": [P, P, P, I, I, P, ctypes.c_longlong, P, P, P, I, I, I, I, I, I, I, I, P],
+            "ts_ssm_scan": [P, P, P, I, I, P, ctypes.c_longlong, P, P, P, I, I, I, I, I, I, I, I, I, P],
             "ts_lightning_ex": [P, P, I, P, P, P, P, I, I, I, I, I, I, I, P],
             "ts_lightning_long": [P, P, I, P, P, P, P, P, I, I, I, I, I, I, I, P],
             "ts_lightning_long_supported": [I, I, I, I, I],
@@ -1034,8 +1034,8 @@ class CudaOps:
         filter's last inputs (from ``proj``) included."""
         self._check(self.lib.ts_ssm_scan(_ptr(out), _ptr(ready), _ptr(proj), proj.stride(0), xbc_off, _ptr(state),
                                          state.stride(0), _ptr(skip), _ptr(step.q_start), _ptr(step.state_slots),
-                                         step.num_requests, H, G, N, P, taps, int(getattr(step, "max_q_len", 0) or 0),
-                                         _code(proj.dtype), self._stream()), "ssm_scan")
+                                         step.num_requests, proj.shape[0], H, G, N, P, taps,
+                                         int(getattr(step, "max_q_len", 0) or 0), _code(proj.dtype), self._stream()), "ssm_scan")
 
     GATES = {"sigmoid": 0, "silu": 1}
 
