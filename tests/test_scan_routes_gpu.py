@@ -73,3 +73,18 @@ def test_state_space_portions(ops, H, P, N, lens):
     known, unknown = device_us(*(lambda s=s: ops.ssm_scan(out, ready, proj, inner, state, skip, s, H, G, N, P, taps)
                                  for s in (step_of(lens), step_of(lens, False))))
     assert known < 1.03 * unknown, (known, unknown)
+
+
+@pytest.mark.parametrize("H,G,lens", [(12, 6, [64]), (12, 6, [128]), (12, 6, [1] * 32 + [64]), (28, 14, [1] * 8 + [56]), (28, 14, [512])])
+def test_delta_rule_preparation(ops, H, G, lens):
+    """Beside filters off their 16-byte boundary, which go to the kernel for any sizes."""
+    D, V, taps, T = 128, 128, 4, sum(lens)
+    C = 2 * G * D + H * V
+    width = C + 2 * H + G
+    ready = torch.empty_strided((T, width), (width + -width % 4, 1), dtype=torch.float32, device=DEV)
+    proj, state = torch.randn(T, C + H * V + 2 * H, device=DEV).bfloat16(), torch.zeros(len(lens), H * D * V + 3 * C, device=DEV)
+    step, a_log, dt = step_of(lens), torch.rand(H, device=DEV), torch.rand(H, device=DEV)
+    room = torch.rand(C * taps + 4, device=DEV)
+    chosen, general = device_us(*(lambda w=room[k:k + C * taps].view(C, taps): ops.delta_prepare(
+        ready, proj, w, a_log, dt, state, step, H, G, D, V, taps, 1e-6) for k in (0, 1)))
+    assert chosen < 1.04 * general, (chosen, general)

@@ -98,7 +98,11 @@ delta_prepare_kernel(float* __restrict__ ready, int W, const T* __restrict__ pro
 // tokens, their inputs loaded before the first is used, the filter's window in registers (refilled where a request begins); the
 // 24 sums of a q / k head cross the lanes together, in the order of the kernel above, so every value is the same bits.  1,537
 // tokens of 12 heads over 6 of 128: 42 -> 16 us.
-constexpr int DP_TOKENS = 8;
+// Taken from so many (token, head) pairs an SM on that the kernel above, a block each, needs two waves; it waits for a token's
+// inputs less often but each time a request begins, so steps of short requests count differently.  us, above / this one:
+// 12 + 6 heads, 192 tokens 6.4 / 6.9, 256 tokens 8.0 / 7.2; 28 + 14 heads, 64 tokens 5.4 / 6.7, 96 tokens 7.2 / 6.9, 128 tokens
+// 8.7 / 7.6, of which 16 are alone 8.7 / 9.6; 32 + 16 heads, 192 tokens, of which 32 are alone, 13.8 / 11.6.
+constexpr int DP_TOKENS = 8, DP_MANY = 27, DP_MANY_SHORT = 40;
 
 template <typename T>
 __global__ void __launch_bounds__(128)
@@ -582,7 +586,7 @@ TS_API void ts_set_delta_rows(int rows) { g_delta_rows = rows; }
 // 2 G D, then the gate (H V), b (H) and a (H).  conv_w: [2 G D + H V, taps] 32-bit.  state: [slots, state_stride].
 TS_API int ts_delta_prepare(float* ready, int ready_stride, const void* proj, int proj_stride, const float* conv_w, const float* a_log,
                             const float* dt_bias, const float* state, long long state_stride, const int* token_request,
-                            const int* q_start, const int* slots, int T, int H, int G, int D, int V, int taps,
+                            const int* q_start, const int* slots, int B, int T, int H, int G, int D, int V, int taps,
                             float unit_eps, int dtype, void* stream) {
   if (T <= 0) return 0;
   if (H <= 0 || G <= 0 || H % G || D <= 0 || V <= 0) TS_REFUSE(TS_ERR_SHAPE, "ts_delta_prepare: %d heads over %d of %d x %d", H, G, D, V);
@@ -592,7 +596,7 @@ TS_API int ts_delta_prepare(float* ready, int ready_stride, const void* proj, in
   if (smem > 200 * 1024) TS_REFUSE(TS_ERR_LIMIT, "ts_delta_prepare: keys of %d", D);
   if (G + H > 65535) TS_REFUSE(TS_ERR_LIMIT, "ts_delta_prepare: %d heads", G + H);
   cudaStream_t s = (cudaStream_t)stream;
-  if (T >= 64 && taps == 4 && D <= 128 && V <= 128 && !((uintptr_t)conv_w & 15) && (dtype == TS_F32 || dtype == TS_BF16)) {
+  if ((long long)T * (G + H) > (long long)(8 * B > T ? DP_MANY_SHORT : DP_MANY) * ts_sm_count() && T >= 64 && taps == 4 && D <= 128 && V <= 128 && !((uintptr_t)conv_w & 15) && (dtype == TS_F32 || dtype == TS_BF16)) {
     const dim3 grid(ceil_div(T, DP_TOKENS), G + H);
     if (dtype == TS_F32)
       ts_launch(delta_prepare_tokens_kernel<float>, grid, dim3(128), 0, s, ready, ready_stride, (const float*)proj, proj_stride, conv_w, a_log,

@@ -68,7 +68,7 @@ class LazyProduct:
 class CudaOps:
     """ctypes front of ``libturingserve_b200.so``."""
 
-    ABI = 22
+    ABI = 23
     UNSUPPORTED = -4            # a kernel's refusal of a shape or layout another kernel takes
 
     def __init__(self, lib_path: str) -> None:
@@ -131,7 +131,7 @@ class CudaOps:
             "ts_act_mul": [P, P, I, I, I, I, I, P],
             "ts_rope_pairs_write": [P, I, I, I, P, P, F, I, P, P, P, I, I, I, I, I, I, I, P],
             "ts_moe_gather": [P, P, P, P, I, I, I, I, P],
-            "ts_delta_prepare": [P, I, P, I, P, P, P, P, ctypes.c_longlong, P, P, P, I, I, I, I, I, I, F, I, P],
+            "ts_delta_prepare": [P, I, P, I, P, P, P, P, ctypes.c_longlong, P, P, P, I, I, I, I, I, I, I, F, I, P],
             "ts_delta_scan": [P, P, I, P, I, P, ctypes.c_longlong, P, P, I, I, I, I, I, I, I, I, P],
             "ts_head_gated_rmsnorm": [P, P, P, I, P, I, F, I, I, I, I, P],
             "ts_attention_biased": [P, I, I, P, I, I, P, P, P, P, P, I, I, I, I, I, I, I, I, F, F, P, I, I, P, P, I, I, P, I, P, P, I, P],
@@ -754,7 +754,7 @@ class CudaOps:
         T = proj.shape[0]
         self._check(self.lib.ts_delta_prepare(_ptr(ready), ready.stride(0), _ptr(proj), proj.stride(0), _ptr(conv_w), _ptr(a_log),
                                               _ptr(dt_bias), _ptr(state), state.stride(0), _ptr(step.token_request),
-                                              _ptr(step.q_start), _ptr(step.state_slots), T, H, G, D, V, taps,
+                                              _ptr(step.q_start), _ptr(step.state_slots), step.num_requests, T, H, G, D, V, taps,
                                               float(unit_eps), _code(proj.dtype), self._stream()), "delta_prepare")
 
     def delta_scan(self, out, ready, proj, state, step, H: int, G: int, D: int, V: int, taps: int) -> None:
