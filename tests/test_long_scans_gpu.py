@@ -170,3 +170,36 @@ def test_delta_rule_portions(ops, dtype, H, G, D, V, taps, pad):
         at += n
     for r in results[1:]:
         assert torch.equal(r[0], results[0][0]) and torch.equal(r[1], results[0][1])
+
+
+@pytest.mark.parametrize("D", [8, 64, 104, 136])
+@pytest.mark.parametrize("kind", ["linear", "state_space", "delta"])
+def test_infinite_values_in_narrow_states(ops, monkeypatch, kind, D):
+    """An infinite value in one column, keys and queries positive: that column's output is infinite from there on (in the delta
+    rule at that token), not NaN, although a state of fewer rows than the lanes hold leaves some of them without any."""
+    monkeypatch.setattr(ops, "lightning_long_tokens", 128)
+    T, V, at, col = 150, 16, 70, 5
+    g = torch.Generator(device=DEV).manual_seed(D)
+    some = lambda *s: torch.rand(*s, generator=g, device=DEV) * 0.2 + 0.1
+    step = SimpleNamespace(q_start=i32([0, T]), state_slots=i32([0]), num_requests=1, max_q_len=T, token_request=i32([0] * T))
+    out, inf = torch.empty(T, V, device=DEV), float("inf")
+    if kind == "linear":
+        proj, state = some(T, 2 * D + V), torch.zeros(1, 1, D, V, device=DEV)
+        proj[at, 2 * D + col] = inf
+        ops.lightning(out, proj, state, some(1), step, 1, D, V)
+    elif kind == "state_space":
+        H, P = 2, V // 2                                   # (rows of 16 + 2 D + 4: on their boundaries)
+        ready, proj, state = some(T, V + 2 * D + 2 * H), some(T, 2 * V + 2 * D + H), torch.zeros(1, H * D * P + 3 * (V + 2 * D), device=DEV)
+        ready[at, col] = inf
+        ops.ssm_scan(out, ready, proj, V, state, some(H), step, H, 1, D, P, 4)
+    else:
+        width = 2 * D + V + 3
+        if D > 128:
+            pytest.skip("wider keys go to another kernel")
+        ready, proj = some(T, width + (-width) % 4)[:, :width], some(T, 2 * D + 2 * V + 2)
+        state = torch.zeros(1, D * V + 3 * (2 * D + V), device=DEV)
+        ready[at, 2 * D + col] = inf
+        ops.delta_scan(out, ready, proj, state, step, 1, 1, D, V, 4)
+    others = [c for c in range(V) if c != col]
+    assert bool(out[:, others].isfinite().all()) and bool(out[:at, col].isfinite().all())
+    assert bool((out[at:at + 1 if kind == "delta" else T, col] == inf).all())

@@ -381,8 +381,11 @@ delta_scan_kernel(float* __restrict__ out, const float* __restrict__ ready, int 
 // a lane 8 rows, four shuffles for each of two sums, rows fetched by 4-byte copies because they were 3,102 values apart; they
 // start on 16-byte boundaries now).  Single tokens stay with the kernel above: one trip through the chain, and half as many
 // threads to a column.
+// PAD: keys narrower than the lanes' 128 rows.  Absent rows have keys and queries of zero, but times an infinite u that is NaN,
+// so they take no part in the update there (by halves of a lane).
 constexpr int DL_WARPS = 4, DL_LOAD_WARPS = 2, DL_COLS = 4 * DL_WARPS, DL_STAGES = 3, DL_ROWS = 16, DL_KEYS = 8 * DL_ROWS;
 
+template <bool PAD>
 __global__ void __launch_bounds__((DL_WARPS + DL_LOAD_WARPS) * 32, 2)
 delta_scan_rows_kernel(float* __restrict__ out, const float* __restrict__ ready, int W, const void* __restrict__ proj,
                        int proj_stride, int proj_is_bf16, float* __restrict__ state, size_t state_stride,
@@ -499,9 +502,10 @@ delta_scan_rows_kernel(float* __restrict__ out, const float* __restrict__ ready,
     const float2 d0 = unpack2(c0), d1 = unpack2(c1);
     const float c = t.g * ((d0.x + d0.y) + (d1.x + d1.y));
     const float u = fmaf(-bg, a, bv);
-    const f2 u2 = pack2(u, u);
+    const float ua = PAD && p * DL_ROWS >= D ? 0.f : u, ub = PAD && p * DL_ROWS + 8 >= D ? 0.f : u;
+    const f2 u2[2] = {pack2(ua, ua), pack2(ub, ub)};
 #pragma unroll
-    for (int i = 0; i < DL_ROWS / 2; ++i) s[i] = fma2(t.k[i], u2, gs[i]);
+    for (int i = 0; i < DL_ROWS / 2; ++i) s[i] = fma2(t.k[i], u2[i / 4], gs[i]);
     x[r] = p == 0 ? fmaf(t.kq, u, c) : c;
   };
   int st = 0;
@@ -643,18 +647,20 @@ TS_API int ts_delta_scan(float* out, const float* ready, int ready_stride, const
   cudaStream_t s = (cudaStream_t)stream;
   if (max_q_len != 1 && vec4 && V % 4 == 0 && D <= DL_KEYS && g_delta_rows == 0) {
     constexpr size_t bytes = sizeof(float) * DL_STAGES * DR_GROUP * (2 * DL_KEYS + DL_COLS + 4);
+    auto kernel = D < DL_KEYS ? delta_scan_rows_kernel<true> : delta_scan_rows_kernel<false>;
     static bool ready_to_go = false;
     if (!ready_to_go) {
-      cudaError_t e = cudaFuncSetAttribute(delta_scan_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+      cudaError_t e = cudaFuncSetAttribute(delta_scan_rows_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(delta_scan_rows_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
       if (e != cudaSuccess) TS_REFUSE((int)e, "ts_delta_scan: shared memory %zu: %s", bytes, cudaGetErrorString(e));
       ready_to_go = true;
     }
     const dim3 rows_grid(ceil_div(V, DL_COLS), H, B), rows_block((DL_WARPS + DL_LOAD_WARPS) * 32);
     if (max_q_len >= DL_LATE_TOKENS)
-      ts_launch_late(delta_scan_rows_kernel, rows_grid, rows_block, bytes, s, out, ready, W, proj, proj_stride, dtype == TS_BF16 ? 1 : 0, state,
+      ts_launch_late(kernel, rows_grid, rows_block, bytes, s, out, ready, W, proj, proj_stride, dtype == TS_BF16 ? 1 : 0, state,
                      (size_t)state_stride, q_start, slots, H, G, D, V, taps);
     else
-      ts_launch(delta_scan_rows_kernel, rows_grid, rows_block, bytes, s, out, ready, W, proj, proj_stride, dtype == TS_BF16 ? 1 : 0, state,
+      ts_launch(kernel, rows_grid, rows_block, bytes, s, out, ready, W, proj, proj_stride, dtype == TS_BF16 ? 1 : 0, state,
                 (size_t)state_stride, q_start, slots, H, G, D, V, taps);
     TS_LAUNCH_CHECK();
   }

@@ -332,10 +332,12 @@ lightning_long_kernel(float* __restrict__ out, const float* __restrict__ ready, 
     float v;
   };
   const uint32_t ring = (uint32_t)__cvta_generic_to_shared(smem);
+  const int v_at = p * ROWS < D ? 2 * DP + col : 4 * 15;   // (a lane of absent rows: the last lane's query row, which is zero)
+  const bool second = p * ROWS + 8 < D;
   auto load = [&](Token& t, uint32_t at) {
     load_rows<ROWS>(at, p, t.q);
     load_rows<ROWS>(at + 4 * DP, p, t.k);
-    t.v = load_f32(at + 4 * (2 * DP + col));
+    t.v = load_f32(at + 4 * v_at);
   };
   auto take = [&](const Token& t, int r, Token& next, uint32_t next_at, bool more) {
     const f2 v2 = pack2(t.v, t.v);
@@ -345,7 +347,7 @@ lightning_long_kernel(float* __restrict__ out, const float* __restrict__ ready, 
     if (more) load(next, next_at);
 #pragma unroll
     for (int i = 0; i < ROWS / 2; ++i) s[i] = fma2(lam2, s[i], kv[i]);
-    x[r] = dot_rows<ROWS>(s, t.q, 0.f);
+    x[r] = dot_rows<ROWS>(s, t.q, 0.f, second);
   };
   int st = 0;
   for (int g0 = 0; g0 < n; g0 += LT_GROUP, st = st + 1 == LL_STAGES ? 0 : st + 1) {

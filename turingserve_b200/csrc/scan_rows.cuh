@@ -61,9 +61,11 @@ __device__ __forceinline__ f2 mul2_first(f2 a, f2 b) {
   return d;
 }
 
-// The products of one state column's rows with q, summed within the lane (`first` starts the first row's chain).
+// The products of one state column's rows with q, summed within the lane (`first` starts the first row's chain).  `second`: the
+// second part of 16 rows exists.  (Absent rows have keys and queries of zero, but times an infinite value that is NaN: absent
+// parts are left out here, and a lane without any row takes its value from a place that holds zero.)
 template <int ROWS>
-__device__ __forceinline__ float dot_rows(const f2 (&s)[ROWS / 2], const f2 (&q)[ROWS / 2], float first) {
+__device__ __forceinline__ float dot_rows(const f2 (&s)[ROWS / 2], const f2 (&q)[ROWS / 2], float first, bool second) {
   float part[ROWS / 8];
 #pragma unroll
   for (int m = 0; m < ROWS / 8; ++m) {
@@ -73,7 +75,7 @@ __device__ __forceinline__ float dot_rows(const f2 (&s)[ROWS / 2], const f2 (&q)
     const float2 v = unpack2(e);
     part[m] = v.x + v.y;
   }
-  return ROWS == 8 ? part[0] : part[0] + part[ROWS / 8 - 1];
+  return ROWS == 8 ? part[0] : part[0] + (second ? part[ROWS / 8 - 1] : 0.f);
 }
 
 // x[i] of every lane summed over the 16 lanes of its half warp; lane p gets the sum of x[p].  15 shuffles for 16 sums; lanes

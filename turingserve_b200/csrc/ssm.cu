@@ -441,10 +441,12 @@ ssm_scan_long_kernel(float* __restrict__ out, const float* __restrict__ ready, c
     float2 x, da;
   };
   const uint32_t ring = (uint32_t)__cvta_generic_to_shared(smem);
+  const int x_at = p * ROWS < N ? 2 * NP + col : 4 * 15;   // (a lane of absent rows: the last lane's row of B, which is zero)
+  const bool second = p * ROWS + 8 < N;
   auto load = [&](Token& t, uint32_t at) {
     load_rows<ROWS>(at, p, t.B);
     load_rows<ROWS>(at + 4 * NP, p, t.C);
-    t.x = load_pair(at + 4 * (2 * NP + col));
+    t.x = load_pair(at + 4 * x_at);
     t.da = load_pair(at + 4 * (2 * NP + COLS));
   };
   auto take = [&](const Token& t, int r, Token& next, uint32_t next_at, bool more) {
@@ -463,7 +465,7 @@ ssm_scan_long_kernel(float* __restrict__ out, const float* __restrict__ ready, c
 #pragma unroll
       for (int i = 0; i < ROWS / 2; ++i) s[c][i] = fma2(a2, s[c][i], bx[c][i]);
       // (the skip term starts the first row's chain)
-      x[r * SL_OWN + c] = dot_rows<ROWS>(s[c], t.C, p == 0 ? dskip * (c == 0 ? t.x.x : t.x.y) : 0.f);
+      x[r * SL_OWN + c] = dot_rows<ROWS>(s[c], t.C, p == 0 ? dskip * (c == 0 ? t.x.x : t.x.y) : 0.f, second);
     }
   };
   int st = 0;
