@@ -373,7 +373,7 @@ delta_scan_kernel(float* __restrict__ out, const float* __restrict__ ready, int 
                       (h * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x, H * gridDim.x * blockDim.x);
 }
 
-// ---- portions of keys up to 128 wide: eight lanes of a warp own a column, a lane 16 rows of it, two 32-bit operations an
+// ---- portions of keys up to 128 wide: eight lanes of a warp own a column, a lane 8 or 16 rows of it, two 32-bit operations an
 // instruction.  A token's chain is the sum a over the eight lanes (three shuffles), u, and the update; the read-out's sum is
 // not on it: a lane keeps its share of eight tokens' outputs, and eight sums cross the lanes at once.  Tokens arrive in groups
 // of 16 by cp.async, two groups ahead, issued by two warps of their own; a token's operands are loaded while the one before is
@@ -381,17 +381,19 @@ delta_scan_kernel(float* __restrict__ out, const float* __restrict__ ready, int 
 // a lane 8 rows, four shuffles for each of two sums, rows fetched by 4-byte copies because they were 3,102 values apart; they
 // start on 16-byte boundaries now).  Single tokens stay with the kernel above: one trip through the chain, and half as many
 // threads to a column.
-// PAD: keys narrower than the lanes' 128 rows.  Absent rows have keys and queries of zero, but times an infinite u that is NaN,
+// ROWS: rows of a column a lane (8 for keys of up to 64, where 16 would leave half of the lanes idle: eight requests of 64 tokens,
+// 16 heads of 64 x 128, 69 us with 16).  PAD: keys narrower than the lanes' rows.  Absent rows have keys and queries of zero, but times an infinite u that is NaN,
 // so they take no part in the update there (by halves of a lane).
-constexpr int DL_WARPS = 4, DL_LOAD_WARPS = 2, DL_COLS = 4 * DL_WARPS, DL_STAGES = 3, DL_ROWS = 16, DL_KEYS = 8 * DL_ROWS;
+constexpr int DL_WARPS = 4, DL_LOAD_WARPS = 2, DL_COLS = 4 * DL_WARPS, DL_STAGES = 3, DL_KEYS = 128;
+constexpr size_t dl_bytes(int rows) { return sizeof(float) * DL_STAGES * DR_GROUP * (2 * 8 * rows + DL_COLS + 4); }
 
-template <bool PAD>
+template <int ROWS, bool PAD>
 __global__ void __launch_bounds__((DL_WARPS + DL_LOAD_WARPS) * 32, 2)
 delta_scan_rows_kernel(float* __restrict__ out, const float* __restrict__ ready, int W, const void* __restrict__ proj,
                        int proj_stride, int proj_is_bf16, float* __restrict__ state, size_t state_stride,
                        const int* __restrict__ q_start, const int* __restrict__ slots, int H, int G, int D, int V, int taps) {
   using namespace scan;
-  constexpr int TOK = 2 * DL_KEYS + DL_COLS + 4;           // q | k | v of the block's columns | g, beta, k.q, 1 unused
+  constexpr int KEYS = 8 * ROWS, PAIRS = ROWS / 2, TOK = 2 * KEYS + DL_COLS + 4;           // q | k | v of the block's columns | g, beta, k.q, 1 unused
   pdl_launch_dependents();
   pdl_wait();
   extern __shared__ __align__(16) float smem[];            // [DL_STAGES][DR_GROUP][TOK]
@@ -402,7 +404,7 @@ delta_scan_rows_kernel(float* __restrict__ out, const float* __restrict__ ready,
   const int qk = G * D, hv = H * V, C = 2 * qk + hv;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, p = lane & 7, col = 4 * warp + (lane >> 3);
   const int j0 = blockIdx.x * DL_COLS, j = j0 + col;
-  if (D < DL_KEYS || j0 + DL_COLS > V) {                   // what no copy writes stays zero
+  if (D < KEYS || j0 + DL_COLS > V) {                   // what no copy writes stays zero
     for (int i = threadIdx.x; i < DL_STAGES * DR_GROUP * TOK / 4; i += blockDim.x)
       reinterpret_cast<float4*>(smem)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     __syncthreads();
@@ -411,7 +413,7 @@ delta_scan_rows_kernel(float* __restrict__ out, const float* __restrict__ ready,
     // Loading warp w brings tokens w, w + DL_LOAD_WARPS, ... of a group, a lane piece `lane` (four rows) of q and k: lane p's
     // k-th piece lies at piece k * 8 + p, so that a column's lanes read neighbouring pieces.
     const int w = warp - DL_WARPS;
-    const int chunks = D / 4, v_chunks = min(DL_COLS, V - j0) / 4, at = 4 * ((lane & 3) * 8 + (lane >> 2));
+    const int chunks = D / 4, v_chunks = min(DL_COLS, V - j0) / 4, at = 4 * (lane % (ROWS / 4) * 8 + lane / (ROWS / 4));
     const float* src = ready + (size_t)(t0 + w) * W + kvh * D + 4 * lane;
     const float* v_src = ready + (size_t)(t0 + w) * W + 2 * qk + h * V + j0 + 4 * lane;
     const float* s_src = ready + (size_t)(t0 + w) * W + C + (lane == 16 ? h : lane == 17 ? H + h : 2 * H + kvh);
@@ -426,10 +428,10 @@ delta_scan_rows_kernel(float* __restrict__ out, const float* __restrict__ ready,
         float* d = dst + rr * DL_LOAD_WARPS * TOK;
         if (lane < chunks) {
           cp_async_16(d + at, src + off, true);
-          cp_async_16(d + DL_KEYS + at, src + off + qk, true);
+          cp_async_16(d + KEYS + at, src + off + qk, true);
         }
-        if (lane < v_chunks) cp_async_16(d + 2 * DL_KEYS + 4 * lane, v_src + off, true);
-        else if (lane >= 16 && lane < 19) cp_async_4(d + 2 * DL_KEYS + DL_COLS + lane - 16, s_src + off);
+        if (lane < v_chunks) cp_async_16(d + 2 * KEYS + 4 * lane, v_src + off, true);
+        else if (lane >= 16 && lane < 19) cp_async_4(d + 2 * KEYS + DL_COLS + lane - 16, s_src + off);
       }
     };
 #pragma unroll
@@ -451,36 +453,36 @@ delta_scan_rows_kernel(float* __restrict__ out, const float* __restrict__ ready,
   const bool live = j < V;
   float* base = state + (size_t)slots[b] * state_stride;
   float* S = base + (size_t)h * D * V + j;
-  f2 s[DL_ROWS / 2];
+  f2 s[PAIRS];
 #pragma unroll
-  for (int i = 0; i < DL_ROWS / 2; ++i) {
-    const int d = p * DL_ROWS + 2 * i;                     // (D is a multiple of 4: both rows or none)
+  for (int i = 0; i < PAIRS; ++i) {
+    const int d = p * ROWS + 2 * i;                     // (D is a multiple of 4: both rows or none)
     const bool there = live && d < D;
     s[i] = pack2(there ? S[(size_t)d * V] : 0.f, there ? S[(size_t)(d + 1) * V] : 0.f);
   }
   struct Token {
-    f2 k[DL_ROWS / 2], q[DL_ROWS / 2];
+    f2 k[PAIRS], q[PAIRS];
     float v, g, beta, kq;
   };
   const uint32_t ring = (uint32_t)__cvta_generic_to_shared(smem);
   auto load = [&](Token& t, uint32_t at) {
 #pragma unroll
-    for (int k = 0; k < DL_ROWS / 4; ++k) {
-      asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(t.k[2 * k]), "=l"(t.k[2 * k + 1]) : "r"(at + 4 * DL_KEYS + 16 * (k * 8 + p)));
+    for (int k = 0; k < ROWS / 4; ++k) {
+      asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(t.k[2 * k]), "=l"(t.k[2 * k + 1]) : "r"(at + 4 * KEYS + 16 * (k * 8 + p)));
       asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(t.q[2 * k]), "=l"(t.q[2 * k + 1]) : "r"(at + 16 * (k * 8 + p)));
     }
-    t.v = load_f32(at + 4 * (2 * DL_KEYS + col));
-    asm volatile("ld.shared.v4.f32 {%0, %1, %2, _}, [%3];" : "=f"(t.g), "=f"(t.beta), "=f"(t.kq) : "r"(at + 4 * (2 * DL_KEYS + DL_COLS)));
+    t.v = load_f32(at + 4 * (2 * KEYS + col));
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, _}, [%3];" : "=f"(t.g), "=f"(t.beta), "=f"(t.kq) : "r"(at + 4 * (2 * KEYS + DL_COLS)));
   };
   float x[8];                                              // this lane's share of the column's eight outputs
   auto take = [&](const Token& t, int r, Token& next, uint32_t next_at, bool more) {
     // a = S^T k over the old state: two chains of four pairs a lane
-    f2 a0 = mul2_first(s[0], t.k[0]), a1 = mul2_first(s[4], t.k[4]);
+    f2 a0 = mul2_first(s[0], t.k[0]), a1 = mul2_first(s[PAIRS / 2], t.k[PAIRS / 2]);
     if (more) load(next, next_at);
 #pragma unroll
-    for (int i = 1; i < 4; ++i) {
+    for (int i = 1; i < PAIRS / 2; ++i) {
       a0 = fma2(s[i], t.k[i], a0);
-      a1 = fma2(s[4 + i], t.k[4 + i], a1);
+      a1 = fma2(s[PAIRS / 2 + i], t.k[PAIRS / 2 + i], a1);
     }
     const float2 e0 = unpack2(a0), e1 = unpack2(a1);
     float a = (e0.x + e0.y) + (e1.x + e1.y);
@@ -488,24 +490,24 @@ delta_scan_rows_kernel(float* __restrict__ out, const float* __restrict__ ready,
     // (beside the shuffles: the read-out of the old state, the faded state)
     f2 c0 = pack2(0.f, 0.f), c1 = c0;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < PAIRS / 2; ++i) {
       c0 = fma2(s[i], t.q[i], c0);
-      c1 = fma2(s[4 + i], t.q[4 + i], c1);
+      c1 = fma2(s[PAIRS / 2 + i], t.q[PAIRS / 2 + i], c1);
     }
     a += __shfl_xor_sync(0xffffffffu, a, 2);
     const f2 g2 = pack2(t.g, t.g);
-    f2 gs[DL_ROWS / 2];
+    f2 gs[PAIRS];
 #pragma unroll
-    for (int i = 0; i < DL_ROWS / 2; ++i) gs[i] = fma2(g2, s[i], pack2(0.f, 0.f));
+    for (int i = 0; i < PAIRS; ++i) gs[i] = fma2(g2, s[i], pack2(0.f, 0.f));
     a += __shfl_xor_sync(0xffffffffu, a, 4);
     const float bg = t.beta * t.g, bv = t.beta * t.v;
     const float2 d0 = unpack2(c0), d1 = unpack2(c1);
     const float c = t.g * ((d0.x + d0.y) + (d1.x + d1.y));
     const float u = fmaf(-bg, a, bv);
-    const float ua = PAD && p * DL_ROWS >= D ? 0.f : u, ub = PAD && p * DL_ROWS + 8 >= D ? 0.f : u;
+    const float ua = PAD && p * ROWS >= D ? 0.f : u, ub = PAD && p * ROWS + ROWS / 2 >= D ? 0.f : u;
     const f2 u2[2] = {pack2(ua, ua), pack2(ub, ub)};
 #pragma unroll
-    for (int i = 0; i < DL_ROWS / 2; ++i) s[i] = fma2(t.k[i], u2[i / 4], gs[i]);
+    for (int i = 0; i < PAIRS; ++i) s[i] = fma2(t.k[i], u2[i / (PAIRS / 2)], gs[i]);
     x[r] = p == 0 ? fmaf(t.kq, u, c) : c;
   };
   int st = 0;
@@ -544,8 +546,8 @@ delta_scan_rows_kernel(float* __restrict__ out, const float* __restrict__ ready,
     }
   }
 #pragma unroll
-  for (int i = 0; i < DL_ROWS / 2; ++i) {
-    const int d = p * DL_ROWS + 2 * i;
+  for (int i = 0; i < PAIRS; ++i) {
+    const int d = p * ROWS + 2 * i;
     if (!live || d >= D) continue;
     const float2 v = unpack2(s[i]);
     S[(size_t)d * V] = v.x;
@@ -646,13 +648,15 @@ TS_API int ts_delta_scan(float* out, const float* ready, int ready_stride, const
   const int vec4 = D % 4 == 0 && W % 4 == 0 && (G * D) % 4 == 0 && !((uintptr_t)ready & 15);
   cudaStream_t s = (cudaStream_t)stream;
   if (max_q_len != 1 && vec4 && V % 4 == 0 && D <= DL_KEYS && g_delta_rows == 0) {
-    constexpr size_t bytes = sizeof(float) * DL_STAGES * DR_GROUP * (2 * DL_KEYS + DL_COLS + 4);
-    auto kernel = D < DL_KEYS ? delta_scan_rows_kernel<true> : delta_scan_rows_kernel<false>;
+    const bool narrow = D <= 64;
+    auto kernel = narrow ? (D < 64 ? delta_scan_rows_kernel<8, true> : delta_scan_rows_kernel<8, false>)
+                         : (D < DL_KEYS ? delta_scan_rows_kernel<16, true> : delta_scan_rows_kernel<16, false>);
+    const size_t bytes = dl_bytes(narrow ? 8 : 16);
     static bool ready_to_go = false;
     if (!ready_to_go) {
-      cudaError_t e = cudaFuncSetAttribute(delta_scan_rows_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-      if (e == cudaSuccess) e = cudaFuncSetAttribute(delta_scan_rows_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-      if (e != cudaSuccess) TS_REFUSE((int)e, "ts_delta_scan: shared memory %zu: %s", bytes, cudaGetErrorString(e));
+      cudaError_t e = cudaFuncSetAttribute(delta_scan_rows_kernel<16, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dl_bytes(16));
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(delta_scan_rows_kernel<16, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dl_bytes(16));
+      if (e != cudaSuccess) TS_REFUSE((int)e, "ts_delta_scan: shared memory %zu: %s", dl_bytes(16), cudaGetErrorString(e));
       ready_to_go = true;
     }
     const dim3 rows_grid(ceil_div(V, DL_COLS), H, B), rows_block((DL_WARPS + DL_LOAD_WARPS) * 32);
