@@ -88,3 +88,20 @@ def test_delta_rule_preparation(ops, H, G, lens):
     chosen, general = device_us(*(lambda w=room[k:k + C * taps].view(C, taps): ops.delta_prepare(
         ready, proj, w, a_log, dt, state, step, H, G, D, V, taps, 1e-6) for k in (0, 1)))
     assert chosen < 1.04 * general, (chosen, general)
+
+
+def test_many_short_requests_of_few_rows(ops, monkeypatch):
+    """The attention with options: more single tokens than SMs, 48 heads over one kv head, 140 keys each."""
+    B, H, D, page, keys = 256, 48, 128, 64, 140
+    per = -(-keys // page)
+    k, v = (torch.randn(B * per, 1, page, D, device=DEV).bfloat16() for _ in range(2))
+    tables = torch.arange(B * per, dtype=torch.int32, device=DEV).view(B, per)
+    step = SimpleNamespace(q_start=i32(list(range(B + 1))), seq_lens=i32([keys] * B), num_requests=B, num_decode=B, max_q_len=1, max_seq_len=keys)
+    q, out = torch.randn(B, H, D, device=DEV).bfloat16(), torch.empty(B, H, D, device=DEV).bfloat16()
+
+    def attend(least):
+        monkeypatch.setattr(ops, "biased_tc_keys", least)
+        ops.attention_biased(out, q, k, v, tables, step, 1, page, D ** -0.5, 0.0, None, None)
+
+    chosen, other = device_us(lambda: attend(128), lambda: attend(1 << 30))
+    assert chosen < 1.04 * other, (chosen, other)

@@ -889,7 +889,9 @@ class CudaOps:
     # (latent rows, one prompt: 64 tokens 24.5 against 18.4 us on mma.sync, 128 tokens 25 against 26.5, 256 tokens 31 against
     # 41; rows of 128: 16 tokens 14.3 against 12.3, 64 tokens 14.3 against 14.3, 256 tokens 16 against 25) and then takes a
     # third of the time a key (8 tokens behind 2,000: 92 against 238 and 39 against 121 us; 2 behind 500: 33 against 64 and 18
-    # against 39 us), whatever the number of rows.
+    # against 39 us), whatever the number of rows.  But a block of it fills an SM, with 128 rows: short requests of at most 64 rows that
+    # outnumber the SMs stay with the other (256 single tokens of 48 heads over one kv head of 128, 140 keys: 18.7 against 17.2 us;
+    # 600 keys: 29.3 against 47.9).
     biased_tc_keys = int(os.environ.get("TURINGSERVE_B200_BIASED_TC_KEYS", "128"))
     biased_decode_splits = int(os.environ.get("TURINGSERVE_B200_BIASED_DECODE_SPLITS", "0"))
 
@@ -951,7 +953,8 @@ class CudaOps:
 
             def portions(first: int, count: int) -> int:
                 """Requests whose keys are not cut: by tcgen05 from ``biased_tc_keys`` keys on."""
-                if self.use_tc_attention and reach >= self.biased_tc_keys and page_size % 16 == 0:
+                crowd = v_cache is not None and step.max_q_len * G <= 64 and count * KVH > self.num_sms and reach < 256
+                if self.use_tc_attention and reach >= self.biased_tc_keys and page_size % 16 == 0 and not crowd:
                     rc = self.lib.ts_attention_biased_tc(
                         _ptr(out), out.stride(0), out.stride(1), _ptr(q), q.stride(0), q.stride(1), _ptr(k_cache), _ptr(v_cache),
                         block_tables.data_ptr() + 4 * first * width, step.q_start.data_ptr() + 4 * first,
