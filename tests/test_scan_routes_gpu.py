@@ -105,3 +105,14 @@ def test_many_short_requests_of_few_rows(ops, monkeypatch):
 
     chosen, other = device_us(lambda: attend(128), lambda: attend(1 << 30))
     assert chosen < 1.04 * other, (chosen, other)
+
+
+@pytest.mark.parametrize("H,G,D,T", [(8, 1, 64, 8), (64, 8, 128, 8)])
+def test_turned_pairs(ops, H, G, D, T):
+    """Beside rows off their 16-byte boundary, which go to the kernel for any sizes."""
+    pos, freq = torch.arange(T, dtype=torch.int32, device=DEV), torch.rand(D // 2, device=DEV)
+    k, v = (torch.zeros(1, G, 64, D, device=DEV).bfloat16() for _ in range(2))
+    room = torch.randn(T * (H + 2 * G) * D + 1, device=DEV).bfloat16()
+    chosen, general = device_us(*(lambda p=room[i:i + T * (H + 2 * G) * D].view(T, -1): ops.rope_pairs_write(
+        p, H * D, (H + G) * D, pos, freq, 1.0, D, k, v, pos, H, G, D, D, 64) for i in (0, 1)))
+    assert chosen < 1.06 * general, (chosen, general)

@@ -1007,9 +1007,13 @@ TS_API int ts_rope_pairs_write(void* proj, int stride, int k_off, int v_off, con
   const int groups = ceil_div(H + G, RHN_WARPS);
   if (groups > 65535) TS_REFUSE(TS_ERR_LIMIT, "ts_rope_pairs_write: %d heads", H + G);
   cudaStream_t s = (cudaStream_t)stream;
-  if (dtype == TS_BF16 && D > 0 && D <= 4096 && ((stride | k_off | v_off | D | V | rot_dims) % 8) == 0 &&
+  // A block a token: too little for it to do in rows of fewer than 640 columns, too much in rows of over 6,000 of few tokens, which the
+  // other kernel spreads over several blocks (the same bits).  us, the other / this one: 9 heads of 64, 8 tokens 1.8 / 2.3, 512 tokens 2.8 /
+  // 2.6; 72 heads of 128, 8 tokens 3.6 / 4.1, 128 tokens 5.2 / 4.4.
+  const int vecs = (H + G) * (D / 8);
+  const bool by_vecs = vecs >= 80 ? (vecs <= 768 || T >= 128) : T >= 512;
+  if (dtype == TS_BF16 && by_vecs && D > 0 && D <= 4096 && ((stride | k_off | v_off | D | V | rot_dims) % 8) == 0 &&
       !(((uintptr_t)proj | (uintptr_t)k_cache | (uintptr_t)v_cache) & 15)) {
-    const int vecs = (H + G) * (D / 8);
     ts_launch(rope_pairs_write_vec_kernel, dim3(T), dim3(vecs > 128 ? 256 : 128), sizeof(float) * rot_dims, s, (bf16*)proj, stride,
               k_off, v_off, positions, freq, magnitude, rot_dims, (bf16*)k_cache, (bf16*)v_cache, slots, H, G, D, V, page);
     TS_LAUNCH_CHECK();
