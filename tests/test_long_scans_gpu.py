@@ -203,3 +203,28 @@ def test_infinite_values_in_narrow_states(ops, monkeypatch, kind, D):
     others = [c for c in range(V) if c != col]
     assert bool(out[:, others].isfinite().all()) and bool(out[:at, col].isfinite().all())
     assert bool((out[at:at + 1 if kind == "delta" else T, col] == inf).all())
+
+
+def test_delta_rule_single_tokens_beside_portions(ops):
+    """Steps in which every request brings one token sum a row in another order than portions do (four lanes of 32 rows, not
+    eight of 16): an uncut run and one with such steps agree to 32-bit roundings, outputs and states."""
+    H, G, D, V, taps, lens = 4, 2, 128, 64, 4, [150, 67]
+    C = 2 * G * D + H * V
+    width = C + 2 * H + G
+    g = torch.Generator(device=DEV).manual_seed(5)
+    rnd = lambda *s: torch.randn(*s, generator=g, device=DEV)
+    proj, conv_w, a_log, dt = rnd(sum(lens), C + H * V + 2 * H), rnd(C, taps) * 0.5, rnd(H) * 0.3, rnd(H) - 2.0
+    first = rnd(9, H * D * V + (taps - 1) * C)
+    results = []
+    for cuts in ((), (1, 2, 66), (64, 65, 100, 101)):
+        state, out = first.clone(), torch.full((sum(lens), H * V), float("nan"), device=DEV)
+        for rows, step in steps(lens, cuts):
+            p = proj[rows].contiguous()
+            ready = torch.empty_strided((len(rows), width), (width + -width % 4, 1), dtype=torch.float32, device=DEV)
+            ops.delta_prepare(ready, p, conv_w, a_log, dt, state, step, H, G, D, V, taps, 1e-6)
+            o = torch.empty(len(rows), H * V, device=DEV)
+            ops.delta_scan(o, ready, p, state, step, H, G, D, V, taps)
+            out[rows] = o
+        results.append((out, state))
+    for out, state in results[1:]:
+        assert close(out, results[0][0].double()) and close(state, results[0][1].double())

@@ -58,11 +58,10 @@ struct Plan {
   static constexpr uint32_t Q_BYTES = (KB - QT) * BLK_Q;
   static constexpr uint32_t S_COL = 0, O_COL = 2 * TK, Q_COL = O_COL + DV;
   static constexpr uint32_t COLS = Q_COL + QT * 32;
-  static constexpr uint32_t TMEM_COLS = COLS <= 256 ? 256 : 512;
-  static constexpr int PER_SM = TMEM_COLS == 256 ? 2 : 1;
+  static constexpr uint32_t TMEM_COLS = 512;               // (every instance needs more than 256: a block an SM)
   static constexpr int BARRIERS = 4 * STAGES + 2 + 2 + 3;
   static constexpr size_t SMEM = Q_BYTES + STAGES * (K_BYTES + V_BYTES) + (BARRIERS + 1) / 2 * 16 + 16 + 4 * TQ * sizeof(float);
-  static_assert(COLS <= 512 && SMEM <= 227 * 1024, "a block's tensor or shared memory");
+  static_assert(COLS > 256 && COLS <= 512 && SMEM <= 227 * 1024, "a block's tensor or shared memory");
 };
 
 struct Args {
@@ -127,7 +126,7 @@ __device__ __noinline__ void add_odd_values(T* dst, const bf16* values, const in
 __device__ __forceinline__ uint32_t below(int n) { return n <= 0 ? 0u : (n >= 32 ? 0xffffffffu : (1u << n) - 1u); }
 
 template <int DK, int DV, int TK, bool V_IN_K, int QT, bool MAPS = false>
-__global__ void __launch_bounds__(THREADS, Plan<DK, DV, TK, V_IN_K, QT, MAPS>::PER_SM)
+__global__ void __launch_bounds__(THREADS, 1)
 attention_biased_tc_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constant__ CUtensorMap v_map,
                            const __grid_constant__ CUtensorMap k_run_map, const __grid_constant__ CUtensorMap v_run_map,
                            const Args a) {
@@ -138,8 +137,8 @@ attention_biased_tc_kernel(const __grid_constant__ CUtensorMap k_map, const __gr
   pdl_launch_dependents();
   extern __shared__ __align__(1024) unsigned char smem[];
   unsigned char* q_s = smem;                               // [KB - QT][128][128 B]
-  unsigned char* k_s = q_s + PL::Q_BYTES;                  // [STAGES][KB][64][128 B]
-  unsigned char* v_s = k_s + STAGES * K_BYTES;             // [STAGES][VB][64][128 B] (absent when the values are in the key rows)
+  unsigned char* k_s = q_s + PL::Q_BYTES;                  // [STAGES][KB][TK][128 B]
+  unsigned char* v_s = k_s + STAGES * K_BYTES;             // [STAGES][VB][TK][128 B] (absent when the values are in the key rows)
   // (values in the key rows: the _k barriers are those of a tile's blocks that are no values here, the _v ones those of its values)
   uint64_t* full_k = reinterpret_cast<uint64_t*>(v_s + STAGES * V_BYTES);
   uint64_t* empty_k = full_k + STAGES;
