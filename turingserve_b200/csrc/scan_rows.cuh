@@ -108,6 +108,7 @@ __device__ __forceinline__ float tree_of(const float* p, int parts, int stride) 
 }
 template <bool FEW>
 __device__ __forceinline__ float tree_of_parts(const float* p, int parts, int stride) {
+  if (FEW && parts == 16) return tree_of<16>(p, 16, stride);               // (keys of 128 first)
   if (FEW && parts <= 4) return tree_of<4>(p, parts, stride);              // (absent parts add nothing)
   if (FEW && parts <= 8) return tree_of<8>(p, parts, stride);
   const float x = tree_of<16>(p, parts, stride);
