@@ -23,11 +23,12 @@ __device__ __forceinline__ float ts_activate(float z, int kind) {
 template <typename T> __device__ __forceinline__ float ts_activate_for(float z, int kind) { return ts_activate(z, kind); }
 // z Phi(z) in 32 bits without erff's branches, which cost the epilogue that applies this to a product's tile more than the
 // product itself.  |z| < 1.25: z / 2 + s (c + s R(s)), s = z^2, c = 1 / sqrt(2 pi), R the least-squares polynomial at Chebyshev
-// nodes; where z is below -1/2 the two terms cancel, and c enters with its low part.  Beyond, by erfc(x) = t exp(p(t) -
-// x^2), t = 1 / (1 + x / 2), x = |z| / sqrt(2) (the form in Numerical Recipes; the coefficients are fitted here), p the least-squares polynomial of log(erfcx(x) / t) at
-// Chebyshev nodes for x up to 10, off by 4e-8; the argument's rounding and the fast exponential make that 7e-7 of the result at
-// z = -2 and 2e-5 at -12.  Against 64 bits, with erff in brackets: root
-// mean square 2.8e-8 (3.9e-8) for z in [-0.5, 3], 5.9e-8 (8.7e-8) in [-1.25, -1], 1.8e-7 (3.5e-7) in [-2, -1.75], and nowhere more
+// nodes; where z is below -1/2 the two terms cancel, and c enters with its low part.  Beyond, by erfc(x) = t exp(p(t) - x^2),
+// t = 1 / (1 + x / 2), x = |z| / sqrt(2) (the form in Numerical Recipes; the coefficients are fitted here), p the least-squares
+// polynomial of log(erfcx(x) / t) at Chebyshev nodes for x up to 10, off by 4e-8; the argument's rounding and the fast
+// exponential make that 6e-7 of the result at z = -2 and 2e-5 at -12.  Error against 64 bits with an exact exponential and
+// quotient, erff's in brackets, root mean square: 2.8e-8 (3.9e-8) for z in [-0.5, 3], 8.0e-8 (8.7e-8) in [-1.25, -1], 1.2e-7
+// (3.5e-7) in [-2, -1.75].
 // Two values at a time, because the products and sums go two an instruction (fma.rn.f32x2: the same bits as two).
 __device__ __forceinline__ float2 ts_fma2(float2 a, float2 b, float2 c) {
   float2 d;

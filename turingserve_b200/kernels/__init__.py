@@ -687,9 +687,9 @@ class CudaOps:
                                               self._stream()), "kv_write_pair")
 
     # Portions (more than 16 query rows a kv head) that reach over at least this many keys go to the tcgen05 kernel and the one
-    # that joins its two maps.  The GPU is faster with them from 128 keys on (the whole mixer at width 1,536: 128 tokens 45.1
-    # against 45.5 us, 256 tokens 24.7 against 38.5, 512 tokens 30.8 against 59.3; 16 tokens behind 2,000: 47 against 169), but
-    # their launches and tensor maps cost the host 6 us more, and below 512 keys the host is what such a call waits for
+    # that joins its two maps.  The GPU is faster with them from 256 keys on at the latest (the whole mixer at width 1,536: 256 tokens 24.7
+    # against 38.5 us, 512 tokens 30.8 against 59.3; 16 tokens behind 2,000: 47 against 169; with weights of one term, two take the
+    # attention a fifth longer), but their launches and tensor maps cost the host 6 us more, and below 512 keys the host is what such a call waits for
     # (70 tokens behind 184: 79.6 against 73.2 us a call).
     diff_tc_keys = int(os.environ.get("TURINGSERVE_B200_DIFF_TC_KEYS", "512"))
 
