@@ -24,7 +24,7 @@
 // Order of the products: S(0) S(1) O(0) S(2) O(1) S(3) ...: a tile's softmax runs beside the O of the tile before and the
 // S of the tile behind.
 //
-// What bounds it (ncu and clock stamps): a tile's chain.  576: 36 + 8 products of 46 to 128 cycles a tile of 64 keys (64
+// What bounds it (clock stamps in the kernel): a tile's chain.  576: 36 + 8 products of 46 to 128 cycles a tile of 64 keys (64
 // rows of K give a product no fewer cycles than 128 would), 3,600 cycles a tile of about 4,300; 128: 2,900 cycles a tile of
 // 128 keys, of which the softmax is busy for 2,400.  Portion of 2,048 tokens, 12 heads (L2 flushed), against the mma.sync
 // kernel of attention_biased_mma.cu: latent rows 660 -> 164 us; 128 over 2 kv heads 149 -> 43 us, with cap and bias 174 ->
