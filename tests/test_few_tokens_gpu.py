@@ -1,0 +1,99 @@
+"""The few-token products whose weights pass through registers: every instance at ragged sizes (rows that are no multiple of
+a tile, K of 8 to a few thousand, 1 to 16 tokens) against the product in 64 bits, and what finishes itself against the
+product followed by the kernel that would.
+
+Bound: 32-bit sums of exact products of bfloat16 values; K roundings of partial sums of at most the sum of magnitudes:
+2^-24 sqrt(K) of it with chance signs, 4e-6 of an output's size for K of 5,000; 2e-5 with margin."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+PLANS = range(1, 8)
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from turingserve_b200 import kernels
+    return kernels.ops()
+
+
+def rnd(seed, *shape, std=1.0):
+    return (torch.randn(*shape, generator=torch.Generator(device=DEV).manual_seed(seed), device=DEV) * std).bfloat16()
+
+
+@pytest.mark.parametrize("plan", PLANS)
+@pytest.mark.parametrize("N,K", [(1, 8), (33, 40), (200, 72), (1001, 1000), (2400, 1536), (130, 4504), (19000, 264)])
+def test_plans_against_64_bits(ops, monkeypatch, plan, N, K):
+    monkeypatch.setattr(ops, "few_plan", plan)
+    w, b = rnd(1, N, K, std=0.05), rnd(2, N)
+    for M in (1, 7, 8, 9, 16):
+        x = rnd(M, M, K)
+        want = x.double() @ w.double().T
+        size = (x.double().abs() @ w.double().abs().T).clamp_min(1e-3)
+        out = torch.full((M, N), float("nan"), device=DEV)
+        assert ops._few(out, x, w, None, M, N, K, ops.FEW_FLOAT)
+        assert float(((out - want).abs() / size).max()) < 2e-5
+        out = torch.full((M * N + 1,), float("nan"), device=DEV)[1:].view(M, N)         # (off the boundary of two floats)
+        assert ops._few(out, x, w, b, M, N, K, ops.FEW_FLOAT)
+        assert float(((out - want - b.double()).abs() / (size + b.double().abs())).max()) < 2e-5
+        half = torch.full((M, N), float("nan"), device=DEV).bfloat16()
+        assert ops._few(half, x, w, b, M, N, K, ops.FEW_BF16)
+        assert torch.equal(half, out.bfloat16())
+        old = rnd(3, M, N)
+        resid = old.clone()
+        assert ops._few(resid, x, w, b, M, N, K, ops.FEW_RESID)
+        assert torch.equal(resid, (half.float() + old.float()).bfloat16())
+
+
+@pytest.mark.parametrize("plan", PLANS)
+@pytest.mark.parametrize("inter,K", [(64, 8), (448, 904), (2432, 264)])
+def test_gated(ops, monkeypatch, plan, inter, K):
+    monkeypatch.setattr(ops, "few_plan", plan)
+    w = rnd(1, 2 * inter, K, std=0.05)
+    for M in (1, 8, 13, 16):
+        x, act, two, gu = rnd(M, M, K), *(torch.full((M, n), float("nan"), device=DEV).bfloat16() for n in (inter, inter, 2 * inter))
+        assert ops._few(act, x, w, None, M, 2 * inter, K, ops.FEW_GATED) and ops._few(gu, x, w, None, M, 2 * inter, K, ops.FEW_BF16)
+        ops.silu_mul(two, gu, 64)
+        assert torch.equal(act, two)
+
+
+@pytest.mark.parametrize("plan", PLANS)
+@pytest.mark.parametrize("H,KVH,D,K", [(12, 2, 128, 1536), (3, 3, 64, 328), (5, 1, 64, 72)])
+def test_rotation_and_cache_write(ops, monkeypatch, plan, H, KVH, D, K):
+    N, page = (H + 2 * KVH) * D, 16
+    monkeypatch.setattr(ops, "pair_wins", lambda *a: False)       # (the many-row kernel sums in another order)
+    w, b = rnd(1, N, K, std=0.05), rnd(2, N)
+    cos, sin = (torch.rand(50, D // 2, device=DEV) for _ in range(2))
+    for M in (1, 8, 16):
+        x, slots = rnd(M, M, K), torch.randperm(60, device=DEV)[:M].int()
+        slots[M // 2] = -1
+        pos, got = torch.randint(0, 50, (M,), device=DEV).int(), []
+        for fused in (64, 0):
+            monkeypatch.setattr(ops, "few_plan", plan)
+            monkeypatch.setattr(ops, "fused_qkv_tokens", fused)
+            k, v = (torch.zeros(4, KVH, page, D, device=DEV).bfloat16() for _ in range(2))
+            q = torch.full((M, N), float("nan"), device=DEV).bfloat16()
+            q = ops.qkv_rope(q, x, w, b, pos, cos, sin, H, KVH, D, D, k, v, slots, page)
+            got.append((q.clone(), k, v))
+        assert all(torch.equal(a, c) for a, c in zip(*got))
+
+
+def test_infinite_values_stay_with_their_token_and_row(ops, monkeypatch):
+    for plan in PLANS:
+        monkeypatch.setattr(ops, "few_plan", plan)
+        x, w = rnd(1, 5, 200).abs(), rnd(2, 90, 200).abs()
+        x[3, 77], w[40, 10] = float("inf"), float("nan")
+        out = torch.empty(5, 90, device=DEV)
+        assert ops._few(out, x, w, None, 5, 90, 200, ops.FEW_FLOAT)
+        rows = [n for n in range(90) if n != 40]
+        assert bool(out[:, 40].isnan().all()) and bool((out[3, rows] == float("inf")).all())
+        assert bool(out[[0, 1, 2, 4]][:, rows].isfinite().all())
+
+
+def test_sizes_left_to_tcgen05(ops):
+    x, w, out = rnd(1, 3, 8968), rnd(2, 3584, 8968), torch.empty(3, 3584, device=DEV)
+    assert not ops._few(out, x, w, None, 3, 3584, 8968, ops.FEW_FLOAT)
+    ops.linear(out, x, w)
+    assert float((out - (x.double() @ w.double().T)).abs().max()) < 2e-5 * 8968

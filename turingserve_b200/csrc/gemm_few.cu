@@ -1,0 +1,444 @@
+// bfloat16 products of a decode step's few tokens (at most 16):
+//   out[M, N] = x[M, K] . w[N, K]^T (+ bias[N])          (turingserve/ops/reference.py:45-47)
+// The reference leaves them to cuBLAS (turingserve/ops/triton_ops.py:74-76).
+//
+// A step is a chain of such products, each bound by the weights' bytes or, where those are few, by its latency.  So
+// the weights go from global memory straight into the registers that mma.sync (m16n8k16) reads them from: no shared
+// memory, barrier or tensor memory on their way, and the first of them are fetched before the wait for the kernel
+// before.  The tokens are the product's 16 rows, eight weight rows its columns.  A lane's 16 bytes of weight row
+// lane / 4 are eight neighbouring columns of K, which stand for columns 2t, 2t+1, 2t+8, 2t+9 of two products; the
+// same permutation on the tokens' side leaves the sum as it is.
+//
+// Two forms.  DIRECT: the warps of a block cut K between them, a block has one tile of 8 R weight rows, and as every
+// token's column is read by one warp only, tokens come from L2 to registers too (N up to a few thousand).
+// Otherwise the tokens stand in shared memory and a warp takes tiles one after the other (the gate/up product, the
+// output head).  RING: what does not fit the registers at once goes through a ring of cp.async copies in which every
+// lane has 16 bytes of its own per slot and waits for nobody else.  Sums over K are in the order of the warps, whatever finishes the product, so that a product that
+// finishes itself (activation, rotation and cache write, residual add) has the bits of the product followed by the
+// kernel that would do it.
+#include "common.cuh"
+#include "mma_utils.cuh"
+
+namespace {
+
+enum FewMode : int { FEW_BF16 = 0, FEW_FLOAT = 1, FEW_GATED = 2, FEW_ROPE = 3, FEW_RESID = 4 };
+
+struct FewArgs {
+  const bf16* x;          // [M, K]
+  const bf16* w;          // [N, K]
+  const bf16* bias;       // [N] or null
+  void* out;              // [M, N] bf16 / float; [M, N / 2] (gated); the residual rows [M, N] (added to in place)
+  int M, N, K;
+  int tiles;              // of 8 R weight rows
+  int mode;
+  int pairs;              // two neighbouring outputs may be read and written together: N even, out on their boundary
+  // FEW_ROPE
+  const int* positions;
+  const float* cos_t;     // [positions][D / 2]
+  const float* sin_t;
+  const int* slots;
+  bf16* k_cache;
+  bf16* v_cache;
+  int page, H, KVH, D;
+};
+
+__device__ __forceinline__ uint4 ld_weights(const bf16* p) {
+  uint4 v;
+  asm volatile("ld.global.nc.L1::no_allocate.L2::128B.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+
+// A lane's own copy to shared memory and the wait for it: no barrier stands between them and the lane's reads, so these
+// (unlike cp_async_16 and cp_async_wait) keep the compiler from moving a read across.
+__device__ __forceinline__ void own_copy(void* smem, const void* gmem, bool valid) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(gmem), "r"(valid ? 16 : 0) : "memory");
+}
+template <int N> __device__ __forceinline__ void own_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// Weight row behind column `n` (0..7) of tile `tile`: neighbours, or, where the columns are pairs (gate and up, the two
+// halves a rotation joins), columns 2i and 2i + 1 are the two of a pair.
+__device__ __forceinline__ int few_row(const FewArgs& a, int tile, int n) {
+  int row = tile * 8 + n;
+  if (a.mode == FEW_GATED) {
+    const int j = tile * 4 + (n >> 1);
+    row = (j >> 6) * 128 + (j & 63) + (n & 1) * 64;
+  } else if (a.mode == FEW_ROPE) {
+    const int half = a.D >> 1, q = tile * 4 + (n >> 1), head = q / half;
+    row = head * a.D + (q - head * half) + (n & 1) * half;
+  }
+  return min(row, a.N - 1);
+}
+
+// What finishes two neighbouring columns (pair q = 4 tile + t) of a token: b0, b1 their bias, old the residual's two.
+__device__ __forceinline__ void few_finish(const FewArgs& a, int m, int q, float v0, float v1, float b0, float b1, float2 old) {
+  if (m >= a.M) return;
+  if (a.mode == FEW_GATED) {
+    if (2 * q >= a.N) return;
+    const float gate = round_to<bf16>(v0), up = round_to<bf16>(v1);
+    const float s = round_to<bf16>(silu_for<bf16>(gate));
+    reinterpret_cast<bf16*>(a.out)[(size_t)m * (a.N >> 1) + q] = __float2bfloat16_rn(s * up);
+    return;
+  }
+  if (a.mode == FEW_ROPE) {
+    const int half = a.D >> 1, head = q / half, p = q - head * half;
+    if (head >= a.H + 2 * a.KVH) return;
+    const float x1 = round_to<bf16>(v0 + b0), x2 = round_to<bf16>(v1 + b1);
+    float o1 = x1, o2 = x2;
+    if (head < a.H + a.KVH) {
+      const int pos = a.positions[m];
+      const float cs = round_to<bf16>(a.cos_t[(size_t)pos * half + p]), sn = round_to<bf16>(a.sin_t[(size_t)pos * half + p]);
+      o1 = x1 * cs - x2 * sn;
+      o2 = x2 * cs + x1 * sn;
+    }
+    const bf16 w1 = __float2bfloat16_rn(o1), w2 = __float2bfloat16_rn(o2);
+    bf16* qkv = reinterpret_cast<bf16*>(a.out) + (size_t)m * a.N + head * a.D + p;
+    qkv[0] = w1;
+    qkv[half] = w2;
+    if (head >= a.H && a.k_cache != nullptr) {
+      const int slot = a.slots[m];
+      if (slot >= 0) {
+        const bool is_k = head < a.H + a.KVH;
+        bf16* dst = (is_k ? a.k_cache : a.v_cache) + ((size_t)(slot / a.page) * a.KVH * a.page + (size_t)(slot % a.page)) * a.D +
+                    (size_t)(head - a.H - (is_k ? 0 : a.KVH)) * a.page * a.D;
+        dst[p] = w1;
+        dst[p + half] = w2;
+      }
+    }
+    return;
+  }
+  const int n = 2 * q;
+  if (n >= a.N) return;
+  v0 += b0;
+  v1 += b1;
+  const size_t at = (size_t)m * a.N + n;
+  const bool both = n + 1 < a.N, together = a.pairs;
+  if (a.mode == FEW_FLOAT) {
+    float* o = reinterpret_cast<float*>(a.out) + at;
+    if (together) *reinterpret_cast<float2*>(o) = make_float2(v0, v1);
+    else {
+      o[0] = v0;
+      if (both) o[1] = v1;
+    }
+    return;
+  }
+  if (a.mode == FEW_RESID) {
+    v0 = round_to<bf16>(v0) + old.x;
+    v1 = round_to<bf16>(v1) + old.y;
+  }
+  bf16* o = reinterpret_cast<bf16*>(a.out) + at;
+  if (together) *reinterpret_cast<__nv_bfloat162*>(o) = __floats2bfloat162_rn(v0, v1);
+  else {
+    o[0] = __float2bfloat16_rn(v0);
+    if (both) o[1] = __float2bfloat16_rn(v1);
+  }
+}
+
+__device__ __forceinline__ float2 few_bias(const FewArgs& a, int q) {
+  float2 b = make_float2(0.f, 0.f);
+  if (a.bias == nullptr) return b;
+  int n0 = 2 * q, n1 = 2 * q + 1;
+  if (a.mode == FEW_ROPE) {
+    const int half = a.D >> 1, head = q / half;
+    n0 = head * a.D + (q - head * half);
+    n1 = n0 + half;
+  }
+  if (n0 < a.N) b.x = to_f(a.bias[n0]);
+  if (n1 < a.N) b.y = to_f(a.bias[n1]);
+  return b;
+}
+
+__device__ __forceinline__ float2 few_old(const FewArgs& a, int m, int q) {
+  const int n = 2 * q;
+  if (a.mode != FEW_RESID || m >= a.M || n >= a.N) return make_float2(0.f, 0.f);
+  const bf16* r = reinterpret_cast<const bf16*>(a.out) + (size_t)m * a.N + n;
+  if (a.pairs) return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(r));
+  return make_float2(to_f(r[0]), n + 1 < a.N ? to_f(r[1]) : 0.f);
+}
+
+__host__ __device__ constexpr int few_ldx(int K) { return (K + 31) / 32 * 32 + ((K + 31) / 32 % 2 == 0 ? 32 : 0); }   // (rows an odd number of 64 bytes: no bank conflicts)
+
+// TT: 8 TT tokens at most.  R: tiles of eight weight rows a warp works on at a time.  WK warps cut K, WN take other
+// rows.  U: 16-byte loads of weights a lane keeps under way, times R; with RING in shared memory.
+template <int TT, int R, int WK, int WN, bool DIRECT, int U, bool RING>
+__global__ void __launch_bounds__(WK * WN * 32, 1) few_kernel(const FewArgs a) {
+  pdl_launch_dependents();
+  static_assert(!DIRECT || WN == 1, "tokens in registers: one tile a block");
+  constexpr int THREADS = WK * WN * 32, ITEMS = WN * R * TT * 32;
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+  const int wk = warp % WK, wn = warp / WK;
+  const int steps = (a.K + 31) >> 5, per = (steps + WK - 1) / WK;
+  const int s0 = wk * per, ns = max(0, min(steps, s0 + per) - s0);
+  const int tile0 = blockIdx.x * WN + wn, stride = gridDim.x * WN;
+  const int nt = tile0 < a.tiles ? (WK > 1 ? 1 : (a.tiles - 1 - tile0) / stride + 1) : 0;
+  const int total = nt * ns;
+  const int ldx = few_ldx(a.K);
+
+  constexpr int SLOT = (R + (DIRECT ? TT : 0)) * 512;
+  unsigned char* ring = smem + (size_t)warp * U * SLOT + lane * 16;          // RING: this lane's own 16 bytes of every 512
+  uint4 wb[RING ? 1 : U][R];
+  const bf16* wp[R];
+  int l_tile = tile0, l_step = 0, l_i = 0;
+  auto rows = [&](int tile) {
+#pragma unroll
+    for (int r = 0; r < R; ++r) wp[r] = a.w + (size_t)few_row(a, tile * R + r, g) * a.K + s0 * 32 + 8 * t;
+  };
+  auto fetch = [&](int u) {
+    if (l_i < total) {
+      const bool in = (s0 + l_step) * 32 + 8 * t < a.K;
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        if constexpr (RING) own_copy(ring + u * SLOT + r * 512, in ? wp[r] + l_step * 32 : a.w, in);
+        else wb[u][r] = in ? ld_weights(wp[r] + l_step * 32) : make_uint4(0u, 0u, 0u, 0u);
+      }
+      ++l_i;
+      if (++l_step == ns) {
+        l_step = 0;
+        l_tile += stride;
+        if (WK == 1 && l_i < total) rows(l_tile);
+      }
+    }
+  };
+  rows(min(tile0, a.tiles - 1));
+#pragma unroll
+  for (int u = 0; u < U; ++u) fetch(u);
+  if constexpr (RING) cp_async_commit();
+  if (WK > 1 && nt > 0) {
+    // the rest of this warp's weights start towards L2
+    for (int off = U * 32 + t * 64; off < ns * 32; off += 256)
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+        if (s0 * 32 + 8 * t + off < a.K) asm volatile("prefetch.global.L2 [%0];" ::"l"(wp[r] + off));
+  }
+  // the two columns that this thread finishes, where the warps' sums meet in shared memory
+  const int it = threadIdx.x, i_t = it & 3, i_m = (it >> 2) % (8 * TT), i_r = it / (32 * TT) % R, i_wn = it / (32 * TT * R);
+  const int i_q = ((blockIdx.x * WN + i_wn) * R + i_r) * 4 + i_t;
+  float2 bias2 = make_float2(0.f, 0.f), old2 = make_float2(0.f, 0.f);
+  if (WK > 1 && it < ITEMS) bias2 = few_bias(a, i_q);
+  pdl_wait();
+  if (WK > 1 && it < ITEMS) old2 = few_old(a, i_m, i_q);
+
+  bf16* xs = reinterpret_cast<bf16*>(smem + (RING ? WK * WN * U * SLOT : 0));
+  uint4 xb[DIRECT && !RING ? U : 1][TT];
+  auto fetch_x = [&](int i, int u) {
+    const int k = (s0 + i) * 32 + 8 * t;
+#pragma unroll
+    for (int h = 0; h < TT; ++h) {
+      const bool in = k < a.K && g + 8 * h < a.M;
+      const bf16* from = a.x + (in ? (size_t)(g + 8 * h) * a.K + k : 0);
+      if constexpr (RING) own_copy(ring + u * SLOT + (R + h) * 512, from, in);
+      else xb[u][h] = in ? __ldcg(reinterpret_cast<const uint4*>(from)) : make_uint4(0u, 0u, 0u, 0u);
+    }
+  };
+  if constexpr (DIRECT) {
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+    {
+      if (u < total) fetch_x(u, u);
+      if constexpr (RING) cp_async_commit();
+    }
+  } else {
+    const int chunks = ldx / 8;
+    for (int i = threadIdx.x; i < TT * 8 * chunks; i += THREADS) {
+      const int m = i / chunks, c = i - m * chunks;
+      const bool in = m < a.M && c * 8 < a.K;
+      cp_async_16(xs + (size_t)m * ldx + c * 8, a.x + (in ? (size_t)m * a.K + c * 8 : 0), in);
+    }
+    cp_async_commit();
+    if constexpr (RING) {
+#pragma unroll
+      for (int u = 0; u < U - 1; ++u) cp_async_commit();
+      cp_async_wait<U - 1>();
+    } else {
+      cp_async_wait<0>();
+    }
+    __syncthreads();
+  }
+
+  float acc[R][2][4];
+  auto clear = [&] {
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[r][0][e] = acc[r][1][e] = 0.f;
+  };
+  clear();
+  int c_tile = tile0, c_step = 0;
+  const bf16* xrow = xs + (size_t)g * ldx + s0 * 32 + 8 * t;
+  for (int i = 0; i < total; i += U) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (i + u < total) {
+        const int o = RING ? 0 : u;
+        if constexpr (RING) {
+          own_wait<U - 1>();
+#pragma unroll
+          for (int r = 0; r < R; ++r) wb[0][r] = *reinterpret_cast<const uint4*>(ring + u * SLOT + r * 512);
+        }
+        uint4 x0, x1 = make_uint4(0u, 0u, 0u, 0u);
+        if constexpr (DIRECT && RING) {
+          x0 = *reinterpret_cast<const uint4*>(ring + u * SLOT + R * 512);
+          if constexpr (TT == 2) x1 = *reinterpret_cast<const uint4*>(ring + u * SLOT + (R + 1) * 512);
+        } else if constexpr (DIRECT) {
+          x0 = xb[u][0];
+          if constexpr (TT == 2) x1 = xb[u][1];
+        } else {
+          x0 = *reinterpret_cast<const uint4*>(xrow + c_step * 32);
+          if constexpr (TT == 2) x1 = *reinterpret_cast<const uint4*>(xrow + 8 * ldx + c_step * 32);
+        }
+        const unsigned a0[4] = {x0.x, x1.x, x0.y, x1.y}, a1[4] = {x0.z, x1.z, x0.w, x1.w};
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          mma_bf16(acc[r][0], a0, wb[o][r].x, wb[o][r].y);
+          mma_bf16(acc[r][1], a1, wb[o][r].z, wb[o][r].w);
+        }
+        fetch(u);
+        if constexpr (DIRECT) {
+          if (i + u + U < total) fetch_x(i + u + U, u);
+        }
+        if constexpr (RING) cp_async_commit();
+        if (++c_step == ns && WK == 1) {
+#pragma unroll
+          for (int r = 0; r < R; ++r) {
+            const int q = (c_tile * R + r) * 4 + t;
+            const float2 b = few_bias(a, q);
+            few_finish(a, g, q, acc[r][0][0] + acc[r][1][0], acc[r][0][1] + acc[r][1][1], b.x, b.y, few_old(a, g, q));
+            if constexpr (TT == 2)
+              few_finish(a, g + 8, q, acc[r][0][2] + acc[r][1][2], acc[r][0][3] + acc[r][1][3], b.x, b.y, few_old(a, g + 8, q));
+          }
+          clear();
+          c_step = 0;
+          c_tile += stride;
+        }
+      }
+    }
+  }
+  if constexpr (WK > 1) {
+    // [wn][r][wk][token][4] pairs of columns
+    float2* red = reinterpret_cast<float2*>(smem + (RING ? WK * WN * U * SLOT : 0) + (DIRECT ? 0 : (size_t)TT * 8 * ldx * 2));
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+      for (int h = 0; h < TT; ++h)
+        red[(((wn * R + r) * WK + wk) * TT + h) * 32 + lane] =
+            make_float2(acc[r][0][2 * h] + acc[r][1][2 * h], acc[r][0][2 * h + 1] + acc[r][1][2 * h + 1]);
+    __syncthreads();
+    if (it < ITEMS) {
+      const float2* p = red + (size_t)((i_wn * R + i_r) * WK) * TT * 32 + i_m * 4 + i_t;
+      float v0 = 0.f, v1 = 0.f;
+#pragma unroll
+      for (int k = 0; k < WK; ++k) {
+        const float2 v = p[k * TT * 32];
+        v0 += v.x;
+        v1 += v.y;
+      }
+      if (blockIdx.x * WN + i_wn < a.tiles) few_finish(a, i_m, i_q, v0, v1, bias2.x, bias2.y, old2);
+    }
+  }
+}
+
+template <int TT, int R, int WK, int WN, bool DIRECT, int U, bool RING = false>
+int launch(FewArgs& a, cudaStream_t s) {
+  static_assert(WK == 1 || WN * R * TT * 32 <= WK * WN * 32, "a thread finishes one pair of columns");
+  a.tiles = ceil_div(a.N, 8 * R);
+  const size_t smem = (RING ? (size_t)WK * WN * U * (R + (DIRECT ? TT : 0)) * 512 : 0) + (DIRECT ? 0 : (size_t)TT * 8 * few_ldx(a.K) * 2) + (WK > 1 ? (size_t)WN * R * WK * TT * 32 * 8 : 0);
+  static size_t allowed = 48 * 1024;
+  if (smem > 220 * 1024) TS_REFUSE(TS_ERR_UNSUPPORTED, "ts_linear_few: %zu bytes of shared memory", smem);
+  auto kernel = few_kernel<TT, R, WK, WN, DIRECT, U, RING>;
+  if (smem > allowed) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) TS_REFUSE((int)e, "ts_linear_few: shared memory %zu: %s", smem, cudaGetErrorString(e));
+    allowed = smem;
+  }
+  int blocks = ceil_div(a.tiles, WN);
+  if (WK == 1 && blocks > ts_sm_count()) blocks = ts_sm_count();
+  ts_launch(kernel, dim3(blocks), dim3(WK * WN * 32), smem, s, a);
+  TS_LAUNCH_CHECK();
+}
+
+// The instances by number (tests ask for one; callers leave it to few_plan).
+template <int TT> int launch_plan(FewArgs& a, int plan, cudaStream_t s) {
+  switch (plan) {
+    case 1: return launch<TT, 2, 16, 1, true, 3>(a, s);
+    case 2: return launch<TT, 2, 8, 1, true, TT == 1 ? 6 : 4>(a, s);
+    case 3: return launch<TT, 2, 16, 1, true, 6, true>(a, s);
+    case 4: return launch<TT, 2, 8, 1, true, TT == 1 ? 8 : 5, true>(a, s);
+    case 5: return launch<TT, 1, 4, 4, false, TT == 1 ? 8 : 6, true>(a, s);
+    case 6: return launch<TT, 1, 2, 8, false, TT == 1 ? 8 : 6, true>(a, s);
+    case 7: return launch<TT, 1, 1, 16, false, 8, true>(a, s);
+  }
+  TS_REFUSE(TS_ERR_SHAPE, "ts_linear_few: no plan %d", plan);
+}
+
+// Which instance, by the sizes alone (so a product's bits do not depend on what finishes it).  Times of a product
+// with residual add at 8 tokens, weights from DRAM, in us, against the tcgen05 kernel's:
+//  * tiles of 16 rows for at most one block an SM: 16 warps cut K; all of a warp's weights in registers at once while
+//    they are few (1,536 x 1,536: 2.3 / 4.6; 2,048 x 1,536: 2.6 / 5.0), else a ring in shared memory (896 x 4,864:
+//    3.7 / 5.2; 1,536 x 8,960: 7.3 / 9.2; registers 10.8 there: their waits share six scoreboards);
+//  * for two blocks an SM: the same with 8 warps (4,632 x 1,536: 4.1 / 6.7; 3,584 x 3,584: 6.4 / 9.3).  Beyond that, and
+//    where K is long, blocks of one tile no longer divide the chip evenly: 3,584 x 18,944 33 / 30, left to tcgen05;
+//  * more rows: tokens in shared memory, 4, 2 or 1 warps a tile so that about 16 warps an SM have a tile (8,192 x 1,536:
+//    6.4 / 8.8; 9,728 x 896 gated: 5.6 / 6.9; 17,920 x 1,536 gated: 11.1 / 12.7; 151,936 x 1,536: 82 / 86), but for
+//    long rows of tokens, which leave room for one block only (6,144 x 3,584: 12.2 by the second rule, 14.9 / 12.6; 9 to 16
+//    tokens: 6,144 x 2,304 11.9 / 10.0, 12,288 x 1,536 12.0 / 11.2).
+int few_plan(int M, int N, int K) {
+  const int tiles16 = ceil_div(N, 16), sms = ts_sm_count();
+  if (tiles16 <= sms) return K <= 2048 ? 1 : 3;
+  if (tiles16 <= 2 * sms) return K <= 1536 ? 2 : (K <= 8192 ? 4 : 0);
+  if (M > 8 && tiles16 <= 7 * sms && (K > 1900 || tiles16 > 5 * sms)) return 0;
+  if (K > 2560 && tiles16 <= 6 * sms) return K <= 8192 ? 4 : 0;
+  if (few_ldx(K) > 4600) return 0;                 // (16 tokens and the ring: 220 KB)
+  return tiles16 <= 4 * sms ? 5 : (tiles16 <= 7 * sms ? 6 : 7);
+}
+
+int run(FewArgs& a, int plan, cudaStream_t s) {
+  if (a.M > 16 || a.K % 8 != 0 || a.K <= 0)
+    TS_REFUSE(TS_ERR_UNSUPPORTED, "ts_linear_few: M=%d N=%d K=%d is not taken by this kernel", a.M, a.N, a.K);
+  if (((uintptr_t)a.x | (uintptr_t)a.w) & 15) TS_REFUSE(TS_ERR_ALIGN, "ts_linear_few: operands must be 16-byte aligned");
+  a.pairs = a.N % 2 == 0 && ((uintptr_t)a.out & (a.mode == FEW_FLOAT ? 7 : 3)) == 0;
+  if (plan == 0) {
+    plan = few_plan(a.M, a.N, a.K);
+    if (plan == 0) TS_REFUSE(TS_ERR_UNSUPPORTED, "ts_linear_few: N=%d K=%d is faster on tcgen05", a.N, a.K);
+  }
+  return a.M <= 8 ? launch_plan<1>(a, plan, s) : launch_plan<2>(a, plan, s);
+}
+
+}  // namespace
+
+// At most 16 tokens, K a multiple of 8, operands on 16-byte boundaries.  kind: 0 out is bfloat16, 1 float32,
+// 2 out[M, N / 2] = silu(g) * u (rows of w in blocks of 64 gates and their 64 ups, N a multiple of 128, no bias),
+// 4 out[M, N] += the product, both rounded to bfloat16.  plan: 0 = by the sizes (TS_ERR_UNSUPPORTED where the tcgen05
+// kernel is the faster one).
+TS_API int ts_linear_few(void* out, const void* x, const void* w, const void* bias, int M, int N, int K, int kind, int plan,
+                         void* stream) {
+  if (M <= 0 || N <= 0) return 0;
+  if (kind < 0 || kind > 4 || kind == FEW_ROPE) TS_REFUSE(TS_ERR_SHAPE, "ts_linear_few: no kind %d", kind);
+  if (kind == FEW_GATED && (N % 128 != 0 || bias != nullptr))
+    TS_REFUSE(TS_ERR_UNSUPPORTED, "ts_linear_few: gated N=%d is not taken by this kernel", N);
+  FewArgs a = {};
+  a.x = (const bf16*)x; a.w = (const bf16*)w; a.bias = (const bf16*)bias; a.out = out;
+  a.M = M; a.N = N; a.K = K;
+  a.mode = kind;
+  return run(a, plan, (cudaStream_t)stream);
+}
+
+// The q/k/v product of at most 16 tokens that rotates and writes the cache itself: arguments as ts_linear_tc_qkv_rope.
+TS_API int ts_linear_few_qkv_rope(void* qkv, const void* x, const void* w, const void* bias, const int* positions,
+                                  const float* cos_t, const float* sin_t, const int* slots, void* k_cache, void* v_cache, int M,
+                                  int H, int KVH, int D, int page, int K, int plan, void* stream) {
+  if (M <= 0) return 0;
+  if (H <= 0 || KVH <= 0 || (D != 64 && D != 128))
+    TS_REFUSE(TS_ERR_UNSUPPORTED, "ts_linear_few_qkv_rope: heads %d, %d of %d are not taken by this kernel", H, KVH, D);
+  if (positions == nullptr || cos_t == nullptr || sin_t == nullptr)
+    TS_REFUSE(TS_ERR_SHAPE, "ts_linear_few_qkv_rope: positions and tables are needed");
+  if (k_cache != nullptr && (v_cache == nullptr || slots == nullptr || page <= 0))
+    TS_REFUSE(TS_ERR_SHAPE, "ts_linear_few_qkv_rope: the cache write needs both caches, slots and the page size");
+  FewArgs a = {};
+  a.x = (const bf16*)x; a.w = (const bf16*)w; a.bias = (const bf16*)bias; a.out = qkv;
+  a.M = M; a.N = (H + 2 * KVH) * D; a.K = K;
+  a.mode = FEW_ROPE;
+  a.positions = positions; a.cos_t = cos_t; a.sin_t = sin_t; a.slots = slots;
+  a.k_cache = (bf16*)k_cache; a.v_cache = (bf16*)v_cache;
+  a.page = page; a.H = H; a.KVH = KVH; a.D = D;
+  return run(a, plan, (cudaStream_t)stream);
+}

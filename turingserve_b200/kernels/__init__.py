@@ -68,7 +68,7 @@ class LazyProduct:
 class CudaOps:
     """ctypes front of ``libturingserve_b200.so``."""
 
-    ABI = 23
+    ABI = 24
     UNSUPPORTED = -4            # a kernel's refusal of a shape or layout another kernel takes
 
     def __init__(self, lib_path: str) -> None:
@@ -86,6 +86,8 @@ class CudaOps:
             "ts_silu_mul_ex": [P, P, I, I, I, I, P],
             "ts_linear_tc_gated": [P, P, P, I, I, I, P],
             "ts_linear_tc_resid": [P, P, P, P, I, I, I, I, P],
+            "ts_linear_few": [P, P, P, P, I, I, I, I, I, P],
+            "ts_linear_few_qkv_rope": [P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, P],
             "ts_linear_pair": [P, P, P, P, I, I, I, I, P],
             "ts_linear_pair_qkv": [P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, P],
             "ts_linear_tc_qkv_rope": [P, P, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, P],
@@ -341,6 +343,8 @@ class CudaOps:
         K = p.w.shape[1]
         if not (residual.dtype == torch.bfloat16 and residual.is_contiguous() and tuple(residual.shape) == (M, N)):
             return False
+        if self._few(residual, p.x, p.w, p.bias, M, N, K, self.FEW_RESID):
+            return True
         splits = min(self.tc_splits(M, N, K), 8)
         if M <= 16 and M > 4 * splits:
             # up to 16 tokens a block of the cluster sums its tokens one after the other: with few splits that
@@ -384,6 +388,9 @@ class CudaOps:
         kernel, the activation in the product's epilogue; otherwise product, then activation."""
         T, inter = out.shape
         K = w.shape[1]
+        if (bias is None and group == self.GATE_GROUP and T <= self.fused_gate_tokens
+                and self._few(out, x, w, None, T, 2 * inter, K, self.FEW_GATED)):
+            return
         use_tc = self.gemm_mode == "tc" or (self.gemm_mode == "auto" and T <= 128)
         if (x.dtype == torch.bfloat16 and use_tc and bias is None and group == self.GATE_GROUP and T <= self.fused_gate_tokens
                 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0):
@@ -436,6 +443,13 @@ class CudaOps:
         if (x.dtype == torch.bfloat16 and use_tc and T <= self.fused_qkv_tokens and D in (64, 128) and rotary_dim == D
                 and cos is not None and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
                 and self.lib.ts_linear_tc_supported(T, (H + 2 * KVH) * D, K)):
+            if self.takes_few(T, x, w):
+                rc = self.lib.ts_linear_few_qkv_rope(
+                    _ptr(out), _ptr(x), _ptr(w), _ptr(bias), _ptr(positions), _ptr(cos), _ptr(sin), _ptr(slots), _ptr(k_cache),
+                    _ptr(v_cache), T, H, KVH, D, page_size, K, self.few_plan, self._stream())
+                if rc != self.UNSUPPORTED:
+                    self._check(rc, "linear_few_qkv_rope")
+                    return out
             splits = self.tc_splits(T, (H + 2 * KVH) * D, K)
             need = self.lib.ts_linear_tc_qkv_rope_scratch_floats(T, -(-(H + 2 * KVH) * D // 128), splits)
             qkv_part = self._buffer("qkv_part", need, torch.float32, x.device, floor=1 << 18)
@@ -550,6 +564,26 @@ class CudaOps:
             step.q_start.data_ptr() + 4 * nd, step.seq_lens.data_ptr() + 4 * nd, B - nd, width,
             step.max_q_len, H, KVH, D, page_size, float(scale), w, code, self._stream()), "attention")
 
+    FEW_BF16, FEW_FLOAT, FEW_GATED, FEW_RESID = 0, 1, 2, 4
+    # up to this many tokens a product goes to the kernel whose weights pass through registers (it takes 16; 0: to tcgen05)
+    few_tokens = int(os.environ.get("TURINGSERVE_B200_FEW_TOKENS", "16"))
+    few_plan = 0         # its instance; 0: by the sizes
+
+    def takes_few(self, M: int, x, w) -> bool:
+        """Whether the product is one for the kernel for a decode step's few tokens."""
+        return (0 < M <= self.few_tokens and self.gemm_mode == "auto" and x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16
+                and w.shape[1] % 8 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
+
+    def _few(self, out, x, w, bias, M: int, N: int, K: int, kind: int) -> bool:
+        """A few-token product on that kernel; False where it leaves the sizes to the tcgen05 kernel."""
+        if not self.takes_few(M, x, w):
+            return False
+        rc = self.lib.ts_linear_few(_ptr(out), _ptr(x), _ptr(w), _ptr(bias), M, N, K, kind, self.few_plan, self._stream())
+        if rc == self.UNSUPPORTED:
+            return False
+        self._check(rc, "linear_few")
+        return True
+
     def linear(self, out, x, w, bias=None, rows=None, may_defer: bool = False, lazy: bool = True):
         """out[M, N] = x[rows or all, :] @ w[N, K]^T + bias.  Returns ``out``; or, when ``may_defer``
         and the few-token tensor-core kernel takes the product, a ``LazyProduct`` (not launched yet:
@@ -567,6 +601,13 @@ class CudaOps:
             xg = torch.empty((M, K), dtype=x.dtype, device=x.device)
             self.gather_rows(xg, x, rows)
             x, rows = xg, None
+        if rows is None and self.takes_few(M, x, w):
+            if may_defer and N % 8 == 0 and out.dtype == torch.bfloat16:
+                part = self.partial_scratch(M * N, x.device)
+                if self._few(part, x, w, None, M, N, K, self.FEW_FLOAT):
+                    return Deferred(part.view(-1)[: M * N].view(1, M, N), 1, (M, N), out.dtype, bias, out)
+            elif self._few(out, x, w, bias, M, N, K, self.FEW_FLOAT if out.dtype == torch.float32 else self.FEW_BF16):
+                return out
         if (x.dtype == torch.bfloat16 and use_tc and self.lib.ts_linear_tc_supported(M, N, K)
                 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0):
             splits = self.tc_splits(M, N, K)
