@@ -71,15 +71,16 @@ class StepInputs:
     host_ids: np.ndarray | None = None
 
 
-# From about this many keys under the decode rows of a step (requests x longest context), reading them
-# takes longer than the fixed chain of a decode-attention launch, and the kernel built for streaming wins
-# (measured at 12 heads over 2 kv heads of 128: 4 x 16,384 keys 23 against 26 us for the short-chain kernel,
-# 8 x 16,384 keys 38 against 32 us).  The kernels' front adds its own rule for many requests.
+# From about this many keys under the decode rows of a step (requests x longest context), or a third of them in one
+# request, the kernel that cuts a request's keys over as many blocks as the chip has takes the decode attention, below
+# the one whose blocks of a (request, kv head) are one cluster (12 heads over 2 kv heads of 128, us a launch: 1 x 16,000
+# keys 15.7 / 12.4, 1 x 32,000 19.3 / 20.8, 1 x 64,000 24.6 / 38.1, 8 x 32,000 50.5 / 53.0).  The kernels' front adds
+# its own rule for many requests.
 STREAMING_DECODE_KEYS = 98304
 
 
 def streaming_decode(num_decode: int, longest_context: int) -> bool:
-    return num_decode * longest_context >= STREAMING_DECODE_KEYS
+    return max(num_decode, min(num_decode, 1) * 3) * longest_context >= STREAMING_DECODE_KEYS
 
 
 def _align(n: int, a: int = 4) -> int:

@@ -86,6 +86,7 @@ class CudaOps:
             "ts_silu_mul_ex": [P, P, I, I, I, I, P],
             "ts_linear_tc_gated": [P, P, P, I, I, I, P],
             "ts_linear_tc_resid": [P, P, P, P, I, I, I, I, P],
+            "ts_attention_single": [P, I, I, P, I, I, P, P, P, P, P, I, I, I, I, I, I, I, I, F, F, P, I, I, P, I, P, P, I, I, P],
             "ts_linear_few": [P, P, P, P, I, I, I, I, I, P],
             "ts_linear_few_qkv_rope": [P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, P],
             "ts_linear_pair": [P, P, P, P, I, I, I, I, P],
@@ -513,16 +514,18 @@ class CudaOps:
         code = _code(qkv.dtype)
         B, nd = step.num_requests, 0
         width = block_tables.shape[1]
+        # long contexts: the streaming kernel cuts a request's keys over as many blocks as there are
+        long = getattr(step, "streaming_decode", None)
+        if long is None:
+            long = max(step.num_decode, 3) * step.max_seq_len >= 98304
         streaming = self.decode_kernel == "tma"
         if self.decode_kernel == "auto":
-            streaming = getattr(step, "streaming_decode", None)
-            if streaming is None:
-                streaming = step.num_decode * step.max_seq_len >= 98304
-            # The other kernel is the faster one only while its blocks of 8 warps fit one per SM, eight to
-            # a (request, kv head): from ten requests with two kv heads on, the streaming kernel wins at
-            # every context (batch 12 x 2,048 keys: 12.3 against 18.7 us; batch 16 x 256 keys: 9.5 against 12.8)
-            streaming = streaming or step.num_decode * KVH * 8 > self.num_sms
-        if (self.use_fast_attention and streaming and step.num_decode > 0
+            streaming = long or step.num_decode * KVH * 8 > self.num_sms
+        if (self.use_fast_attention and step.num_decode > 0 and qkv.dtype == torch.bfloat16 and self.single_wins(step, KVH, long)
+                and self._attention_single(out.view(out.shape[0], H, D), qkv[:, :H * D].view(qkv.shape[0], H, D), k_cache, v_cache,
+                                           block_tables, step, KVH, page_size, scale, 0.0, None, w, 0, None, 0, None, None, False)):
+            nd = step.num_decode
+        if (nd == 0 and self.use_fast_attention and streaming and step.num_decode > 0
                 and self.lib.ts_attention_decode_tma_supported(H, KVH, D, page_size, code)):
             nd = step.num_decode
             nsplit = self.decode_splits_tma(nd, KVH, D, step.max_seq_len)
@@ -563,6 +566,31 @@ class CudaOps:
             _ptr(out), _ptr(qkv), _ptr(k_cache), _ptr(v_cache), block_tables.data_ptr() + 4 * nd * width,
             step.q_start.data_ptr() + 4 * nd, step.seq_lens.data_ptr() + 4 * nd, B - nd, width,
             step.max_q_len, H, KVH, D, page_size, float(scale), w, code, self._stream()), "attention")
+
+    # single tokens on the kernel whose blocks of a (request, kv head) are one cluster (0: never)
+    single_mode = int(os.environ.get("TURINGSERVE_B200_SINGLE", "1"))
+
+    def single_wins(self, step, KVH: int, streaming: bool) -> bool:
+        return self.single_mode == 2 or (self.single_mode == 1 and self.decode_kernel == "auto" and not streaming
+                                         and step.num_decode * KVH <= self.num_sms)
+
+    def _attention_single(self, out, q, k_cache, v_cache, block_tables, step, KVH: int, page_size: int, scale: float, softcap: float,
+                          slopes, window: int, block_of: int, sinks, keep: int, out_freq, gate, two_terms: bool) -> bool:
+        """The first ``step.num_decode`` requests, one token each, on the kernel whose blocks of a (request, kv head) are one
+        cluster; False where it does not take the shape."""
+        H, Dk = q.shape[1], q.shape[2]
+        reach = min(step.max_seq_len, window + keep) if window else step.max_seq_len
+        if block_of:
+            reach = min(reach, block_of)
+        rc = self.lib.ts_attention_single(
+            _ptr(out), out.stride(0), out.stride(1), _ptr(q), q.stride(0), q.stride(1), _ptr(k_cache), _ptr(v_cache), _ptr(block_tables),
+            _ptr(step.q_start), _ptr(step.seq_lens), step.num_decode, block_tables.shape[1], reach, H, KVH, Dk, out.shape[2], page_size,
+            float(scale), float(softcap), _ptr(slopes), window, block_of, _ptr(sinks), keep, _ptr(out_freq), _ptr(gate),
+            0 if gate is None else gate.stride(0), 1 if two_terms else 0, self._stream())
+        if rc == self.UNSUPPORTED:
+            return False
+        self._check(rc, "attention_single")
+        return True
 
     FEW_BF16, FEW_FLOAT, FEW_GATED, FEW_RESID = 0, 1, 2, 4
     # up to this many tokens a product goes to the kernel whose weights pass through registers (it takes 16; 0: to tcgen05)
@@ -1006,6 +1034,14 @@ class CudaOps:
                         return rc
                 return launch(first, count, step.max_q_len, 1, 0)
 
+            # (16 heads over one kv head of 128, 256 requests of 600 keys: 40 us, 36 with the launch below; 8 heads or latent
+            # rows win at every count)
+            if (spread and self.single_mode and (G <= 8 or v_in_k or nd * KVH <= self.num_sms)
+                    and self._attention_single(out, q, k_cache, v_cache, block_tables, step, KVH, page_size, scale, softcap, slopes, w,
+                                               c, sinks, keep, out_freq, gate, True)):
+                if nd < B:
+                    self._check(portions(nd, B - nd), "attention_biased")
+                return
             if spread:
                 rc = launch(0, nd, 1, ms, 1)
                 if rc == 0 and nd < B:
