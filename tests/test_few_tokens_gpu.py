@@ -10,7 +10,7 @@ import torch
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
-PLANS = range(1, 8)
+PLANS = range(1, 10)
 
 
 @pytest.fixture(scope="module")
@@ -78,6 +78,26 @@ def test_rotation_and_cache_write(ops, monkeypatch, plan, H, KVH, D, K):
             q = ops.qkv_rope(q, x, w, b, pos, cos, sin, H, KVH, D, D, k, v, slots, page)
             got.append((q.clone(), k, v))
         assert all(torch.equal(a, c) for a, c in zip(*got))
+
+
+@pytest.mark.parametrize("plan", PLANS)
+@pytest.mark.parametrize("N,K", [(40, 8), (130, 200), (2051, 1536), (9728, 896)])
+def test_stream_and_activation(ops, monkeypatch, plan, N, K):
+    """Sums into 32-bit rows and activations: the bits of product, then kernel."""
+    monkeypatch.setattr(ops, "few_plan", plan)
+    w, b = rnd(1, N, K, std=0.05), rnd(2, N)
+    for M in (1, 8, 13, 16):
+        x, half = rnd(M, M, K), torch.empty(M, N, device=DEV).bfloat16()
+        assert ops._few(half, x, w, b, M, N, K, ops.FEW_BF16)
+        old = rnd(3, M, N).float() * 1.1
+        stream = old.clone()
+        assert ops._few(stream, x, w, b, M, N, K, ops.FEW_STREAM)
+        assert torch.equal(stream, old + half.float())
+        for code in (1, 2, 3, 4):
+            got, want, part = torch.empty_like(half), torch.empty_like(half), torch.empty(1, M, N, device=DEV)
+            assert ops._few(got, x, w, b, M, N, K, ops.FEW_ACT, code) and ops._few(part, x, w, None, M, N, K, ops.FEW_FLOAT)
+            ops._check(ops.lib.ts_activation_parts(want.data_ptr(), part.data_ptr(), 1, b.data_ptr(), M, N, code, 1, ops._stream()), "activation_parts")
+            assert torch.equal(got, want)
 
 
 def test_infinite_values_stay_with_their_token_and_row(ops, monkeypatch):

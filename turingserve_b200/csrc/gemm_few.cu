@@ -9,25 +9,27 @@
 // lane / 4 are eight neighbouring columns of K, which stand for columns 2t, 2t+1, 2t+8, 2t+9 of two products; the
 // same permutation on the tokens' side leaves the sum as it is.
 //
-// Two forms.  DIRECT: the warps of a block cut K between them, a block has one tile of 8 R weight rows, and as every
-// token's column is read by one warp only, tokens come from L2 to registers too (N up to a few thousand).
-// Otherwise the tokens stand in shared memory and a warp takes tiles one after the other (the gate/up product, the
-// output head).  RING: what does not fit the registers at once goes through a ring of cp.async copies in which every
-// lane has 16 bytes of its own per slot and waits for nobody else.  Sums over K are in the order of the warps, whatever finishes the product, so that a product that
-// finishes itself (activation, rotation and cache write, residual add) has the bits of the product followed by the
-// kernel that would do it.
+// Two forms.  few_kernel: the warps of a block cut K between them, a block has one tile of 8 R weight rows, and as every
+// token's column is read by one warp only, tokens come from L2 to the warp too (N up to a few thousand).  few_rows_kernel:
+// the tokens stand in shared memory and a block of 16 warps an SM takes tiles one after the other (the gate/up product, the
+// output head).  What does not fit the registers at once goes through a ring of cp.async copies in which every
+// lane has 16 bytes of its own per slot and waits for nobody else.  Sums over K are in the order of the warps, whatever
+// finishes the product, so that a product that finishes itself (activation, rotation and cache write, residual add) has
+// the bits of the product followed by the kernel that would do it.
+#include "activations.cuh"
 #include "common.cuh"
 #include "mma_utils.cuh"
 
 namespace {
 
-enum FewMode : int { FEW_BF16 = 0, FEW_FLOAT = 1, FEW_GATED = 2, FEW_ROPE = 3, FEW_RESID = 4 };
+enum FewMode : int { FEW_BF16 = 0, FEW_FLOAT = 1, FEW_GATED = 2, FEW_ROPE = 3, FEW_RESID = 4, FEW_STREAM = 5, FEW_ACT = 6 };
 
 struct FewArgs {
   const bf16* x;          // [M, K]
   const bf16* w;          // [N, K]
   const bf16* bias;       // [N] or null
-  void* out;              // [M, N] bf16 / float; [M, N / 2] (gated); the residual rows [M, N] (added to in place)
+  void* out;              // [M, N] bf16 / float; [M, N / 2] (gated); the residual rows [M, N], bf16 or 32-bit (added to in place)
+  int act;                // FEW_ACT: which activation
   int M, N, K;
   int tiles;              // of 8 R weight rows
   int mode;
@@ -121,9 +123,23 @@ __device__ __forceinline__ void few_finish(const FewArgs& a, int m, int q, float
     }
     return;
   }
+  if (a.mode == FEW_STREAM) {
+    float* o = reinterpret_cast<float*>(a.out) + at;
+    v0 = old.x + round_to<bf16>(v0);
+    v1 = old.y + round_to<bf16>(v1);
+    if (together) *reinterpret_cast<float2*>(o) = make_float2(v0, v1);
+    else {
+      o[0] = v0;
+      if (both) o[1] = v1;
+    }
+    return;
+  }
   if (a.mode == FEW_RESID) {
     v0 = round_to<bf16>(v0) + old.x;
     v1 = round_to<bf16>(v1) + old.y;
+  } else if (a.mode == FEW_ACT) {
+    v0 = ts_activate(round_to<bf16>(v0), a.act);
+    v1 = ts_activate(round_to<bf16>(v1), a.act);
   }
   bf16* o = reinterpret_cast<bf16*>(a.out) + at;
   if (together) *reinterpret_cast<__nv_bfloat162*>(o) = __floats2bfloat162_rn(v0, v1);
@@ -149,223 +165,286 @@ __device__ __forceinline__ float2 few_bias(const FewArgs& a, int q) {
 
 __device__ __forceinline__ float2 few_old(const FewArgs& a, int m, int q) {
   const int n = 2 * q;
-  if (a.mode != FEW_RESID || m >= a.M || n >= a.N) return make_float2(0.f, 0.f);
+  if ((a.mode != FEW_RESID && a.mode != FEW_STREAM) || m >= a.M || n >= a.N) return make_float2(0.f, 0.f);
+  if (a.mode == FEW_STREAM) {
+    const float* r = reinterpret_cast<const float*>(a.out) + (size_t)m * a.N + n;
+    if (a.pairs) return *reinterpret_cast<const float2*>(r);
+    return make_float2(r[0], n + 1 < a.N ? r[1] : 0.f);
+  }
   const bf16* r = reinterpret_cast<const bf16*>(a.out) + (size_t)m * a.N + n;
   if (a.pairs) return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(r));
   return make_float2(to_f(r[0]), n + 1 < a.N ? to_f(r[1]) : 0.f);
 }
 
+// Bias, residual and finish of two columns, out of line: inside the unrolled ring every place would hold a copy of all kinds.
+__device__ __noinline__ void few_store(const FewArgs& a, int m, int q, float v0, float v1) {
+  const float2 b = few_bias(a, q);
+  few_finish(a, m, q, v0, v1, b.x, b.y, few_old(a, m, q));
+}
+
 __host__ __device__ constexpr int few_ldx(int K) { return (K + 31) / 32 * 32 + ((K + 31) / 32 % 2 == 0 ? 32 : 0); }   // (rows an odd number of 64 bytes: no bank conflicts)
 
-// TT: 8 TT tokens at most.  R: tiles of eight weight rows a warp works on at a time.  WK warps cut K, WN take other
-// rows.  U: 16-byte loads of weights a lane keeps under way, times R; with RING in shared memory.
-template <int TT, int R, int WK, int WN, bool DIRECT, int U, bool RING>
-__global__ void __launch_bounds__(WK * WN * 32, 1) few_kernel(const FewArgs a) {
+// TT: 8 TT tokens at most.  R: tiles of eight weight rows a warp works on at a time.  WK warps cut K.  U: 16-byte loads of
+// weights a lane keeps under way, times R; with RING in shared memory.
+template <int TT, int R, int WK, int U, bool RING>
+__global__ void __launch_bounds__(WK * 32, 1) few_kernel(const __grid_constant__ FewArgs a) {
   pdl_launch_dependents();
-  static_assert(!DIRECT || WN == 1, "tokens in registers: one tile a block");
-  constexpr int THREADS = WK * WN * 32, ITEMS = WN * R * TT * 32;
+  constexpr int ITEMS = R * TT * 32;
+  static_assert(ITEMS <= WK * 32, "a thread finishes one pair of columns");
   extern __shared__ __align__(16) unsigned char smem[];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
-  const int wk = warp % WK, wn = warp / WK;
+  const int lane = threadIdx.x & 31, wk = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
   const int steps = (a.K + 31) >> 5, per = (steps + WK - 1) / WK;
   const int s0 = wk * per, ns = max(0, min(steps, s0 + per) - s0);
-  const int tile0 = blockIdx.x * WN + wn, stride = gridDim.x * WN;
-  const int nt = tile0 < a.tiles ? (WK > 1 ? 1 : (a.tiles - 1 - tile0) / stride + 1) : 0;
-  const int total = nt * ns;
-  const int ldx = few_ldx(a.K);
 
-  constexpr int SLOT = (R + (DIRECT ? TT : 0)) * 512;
-  unsigned char* ring = smem + (size_t)warp * U * SLOT + lane * 16;          // RING: this lane's own 16 bytes of every 512
-  uint4 wb[RING ? 1 : U][R];
+  constexpr int SLOT = (R + TT) * 512;
+  unsigned char* ring = smem + (size_t)wk * U * SLOT + lane * 16;          // RING: this lane's own 16 bytes of every 512
+  uint4 wb[RING ? 1 : U][R], xb[RING ? 1 : U][TT];
   const bf16* wp[R];
-  int l_tile = tile0, l_step = 0, l_i = 0;
-  auto rows = [&](int tile) {
 #pragma unroll
-    for (int r = 0; r < R; ++r) wp[r] = a.w + (size_t)few_row(a, tile * R + r, g) * a.K + s0 * 32 + 8 * t;
-  };
-  auto fetch = [&](int u) {
-    if (l_i < total) {
-      const bool in = (s0 + l_step) * 32 + 8 * t < a.K;
+  for (int r = 0; r < R; ++r) wp[r] = a.w + (size_t)few_row(a, blockIdx.x * R + r, g) * a.K + s0 * 32 + 8 * t;
+  auto fetch = [&](int i, int u) {
+    if (i < ns) {
+      const bool in = (s0 + i) * 32 + 8 * t < a.K;
 #pragma unroll
       for (int r = 0; r < R; ++r) {
-        if constexpr (RING) own_copy(ring + u * SLOT + r * 512, in ? wp[r] + l_step * 32 : a.w, in);
-        else wb[u][r] = in ? ld_weights(wp[r] + l_step * 32) : make_uint4(0u, 0u, 0u, 0u);
-      }
-      ++l_i;
-      if (++l_step == ns) {
-        l_step = 0;
-        l_tile += stride;
-        if (WK == 1 && l_i < total) rows(l_tile);
+        if constexpr (RING) own_copy(ring + u * SLOT + r * 512, in ? wp[r] + i * 32 : a.w, in);
+        else wb[u][r] = in ? ld_weights(wp[r] + i * 32) : make_uint4(0u, 0u, 0u, 0u);
       }
     }
   };
-  rows(min(tile0, a.tiles - 1));
-#pragma unroll
-  for (int u = 0; u < U; ++u) fetch(u);
-  if constexpr (RING) cp_async_commit();
-  if (WK > 1 && nt > 0) {
-    // the rest of this warp's weights start towards L2
-    for (int off = U * 32 + t * 64; off < ns * 32; off += 256)
-#pragma unroll
-      for (int r = 0; r < R; ++r)
-        if (s0 * 32 + 8 * t + off < a.K) asm volatile("prefetch.global.L2 [%0];" ::"l"(wp[r] + off));
-  }
-  // the two columns that this thread finishes, where the warps' sums meet in shared memory
-  const int it = threadIdx.x, i_t = it & 3, i_m = (it >> 2) % (8 * TT), i_r = it / (32 * TT) % R, i_wn = it / (32 * TT * R);
-  const int i_q = ((blockIdx.x * WN + i_wn) * R + i_r) * 4 + i_t;
-  float2 bias2 = make_float2(0.f, 0.f), old2 = make_float2(0.f, 0.f);
-  if (WK > 1 && it < ITEMS) bias2 = few_bias(a, i_q);
-  pdl_wait();
-  if (WK > 1 && it < ITEMS) old2 = few_old(a, i_m, i_q);
-
-  bf16* xs = reinterpret_cast<bf16*>(smem + (RING ? WK * WN * U * SLOT : 0));
-  uint4 xb[DIRECT && !RING ? U : 1][TT];
   auto fetch_x = [&](int i, int u) {
-    const int k = (s0 + i) * 32 + 8 * t;
+    if (i < ns) {
+      const int k = (s0 + i) * 32 + 8 * t;
 #pragma unroll
-    for (int h = 0; h < TT; ++h) {
-      const bool in = k < a.K && g + 8 * h < a.M;
-      const bf16* from = a.x + (in ? (size_t)(g + 8 * h) * a.K + k : 0);
-      if constexpr (RING) own_copy(ring + u * SLOT + (R + h) * 512, from, in);
-      else xb[u][h] = in ? __ldcg(reinterpret_cast<const uint4*>(from)) : make_uint4(0u, 0u, 0u, 0u);
+      for (int h = 0; h < TT; ++h) {
+        const bool in = k < a.K && g + 8 * h < a.M;
+        const bf16* from = a.x + (in ? (size_t)(g + 8 * h) * a.K + k : 0);
+        if constexpr (RING) own_copy(ring + u * SLOT + (R + h) * 512, from, in);
+        else xb[u][h] = in ? __ldcg(reinterpret_cast<const uint4*>(from)) : make_uint4(0u, 0u, 0u, 0u);
+      }
     }
   };
-  if constexpr (DIRECT) {
 #pragma unroll
-    for (int u = 0; u < U; ++u)
-    {
-      if (u < total) fetch_x(u, u);
-      if constexpr (RING) cp_async_commit();
-    }
-  } else {
-    const int chunks = ldx / 8;
-    for (int i = threadIdx.x; i < TT * 8 * chunks; i += THREADS) {
-      const int m = i / chunks, c = i - m * chunks;
-      const bool in = m < a.M && c * 8 < a.K;
-      cp_async_16(xs + (size_t)m * ldx + c * 8, a.x + (in ? (size_t)m * a.K + c * 8 : 0), in);
-    }
-    cp_async_commit();
-    if constexpr (RING) {
+  for (int u = 0; u < U; ++u) fetch(u, u);
+  if constexpr (RING) cp_async_commit();
+  // the rest of this warp's weights start towards L2
+  for (int off = U * 32 + t * 64; off < ns * 32; off += 256)
 #pragma unroll
-      for (int u = 0; u < U - 1; ++u) cp_async_commit();
-      cp_async_wait<U - 1>();
-    } else {
-      cp_async_wait<0>();
-    }
-    __syncthreads();
+    for (int r = 0; r < R; ++r)
+      if (s0 * 32 + 8 * t + off < a.K) asm volatile("prefetch.global.L2 [%0];" ::"l"(wp[r] + off));
+  // the two columns that this thread finishes, where the warps' sums meet in shared memory
+  const int it = threadIdx.x, i_t = it & 3, i_m = (it >> 2) % (8 * TT), i_r = it / (32 * TT);
+  const int i_q = (blockIdx.x * R + i_r) * 4 + i_t;
+  float2 bias2 = make_float2(0.f, 0.f), old2 = make_float2(0.f, 0.f);
+  if (it < ITEMS) bias2 = few_bias(a, i_q);
+  pdl_wait();
+  if (it < ITEMS) old2 = few_old(a, i_m, i_q);
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    fetch_x(u, u);
+    if constexpr (RING) cp_async_commit();
   }
 
   float acc[R][2][4];
-  auto clear = [&] {
 #pragma unroll
-    for (int r = 0; r < R; ++r)
+  for (int r = 0; r < R; ++r)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) acc[r][0][e] = acc[r][1][e] = 0.f;
-  };
-  clear();
-  int c_tile = tile0, c_step = 0;
-  const bf16* xrow = xs + (size_t)g * ldx + s0 * 32 + 8 * t;
-  for (int i = 0; i < total; i += U) {
+    for (int e = 0; e < 4; ++e) acc[r][0][e] = acc[r][1][e] = 0.f;
+  for (int i = 0; i < ns; i += U) {
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      if (i + u < total) {
-        const int o = RING ? 0 : u;
+      if (i + u < ns) {
+        constexpr int Z = 0;
+        const int o = RING ? Z : u;
         if constexpr (RING) {
           own_wait<U - 1>();
 #pragma unroll
           for (int r = 0; r < R; ++r) wb[0][r] = *reinterpret_cast<const uint4*>(ring + u * SLOT + r * 512);
+#pragma unroll
+          for (int h = 0; h < TT; ++h) xb[0][h] = *reinterpret_cast<const uint4*>(ring + u * SLOT + (R + h) * 512);
         }
-        uint4 x0, x1 = make_uint4(0u, 0u, 0u, 0u);
-        if constexpr (DIRECT && RING) {
-          x0 = *reinterpret_cast<const uint4*>(ring + u * SLOT + R * 512);
-          if constexpr (TT == 2) x1 = *reinterpret_cast<const uint4*>(ring + u * SLOT + (R + 1) * 512);
-        } else if constexpr (DIRECT) {
-          x0 = xb[u][0];
-          if constexpr (TT == 2) x1 = xb[u][1];
-        } else {
-          x0 = *reinterpret_cast<const uint4*>(xrow + c_step * 32);
-          if constexpr (TT == 2) x1 = *reinterpret_cast<const uint4*>(xrow + 8 * ldx + c_step * 32);
-        }
+        const uint4 x0 = xb[o][0], x1 = TT == 2 ? xb[o][TT - 1] : make_uint4(0u, 0u, 0u, 0u);
         const unsigned a0[4] = {x0.x, x1.x, x0.y, x1.y}, a1[4] = {x0.z, x1.z, x0.w, x1.w};
 #pragma unroll
         for (int r = 0; r < R; ++r) {
           mma_bf16(acc[r][0], a0, wb[o][r].x, wb[o][r].y);
           mma_bf16(acc[r][1], a1, wb[o][r].z, wb[o][r].w);
         }
-        fetch(u);
-        if constexpr (DIRECT) {
-          if (i + u + U < total) fetch_x(i + u + U, u);
-        }
+        fetch(i + u + U, u);
+        fetch_x(i + u + U, u);
         if constexpr (RING) cp_async_commit();
-        if (++c_step == ns && WK == 1) {
-#pragma unroll
-          for (int r = 0; r < R; ++r) {
-            const int q = (c_tile * R + r) * 4 + t;
-            const float2 b = few_bias(a, q);
-            few_finish(a, g, q, acc[r][0][0] + acc[r][1][0], acc[r][0][1] + acc[r][1][1], b.x, b.y, few_old(a, g, q));
-            if constexpr (TT == 2)
-              few_finish(a, g + 8, q, acc[r][0][2] + acc[r][1][2], acc[r][0][3] + acc[r][1][3], b.x, b.y, few_old(a, g + 8, q));
-          }
-          clear();
-          c_step = 0;
-          c_tile += stride;
-        }
       }
     }
   }
-  if constexpr (WK > 1) {
-    // [wn][r][wk][token][4] pairs of columns
-    float2* red = reinterpret_cast<float2*>(smem + (RING ? WK * WN * U * SLOT : 0) + (DIRECT ? 0 : (size_t)TT * 8 * ldx * 2));
+  // [r][wk][token][4] pairs of columns
+  float2* red = reinterpret_cast<float2*>(smem + (RING ? WK * U * SLOT : 0));
 #pragma unroll
-    for (int r = 0; r < R; ++r)
+  for (int r = 0; r < R; ++r)
 #pragma unroll
-      for (int h = 0; h < TT; ++h)
-        red[(((wn * R + r) * WK + wk) * TT + h) * 32 + lane] =
-            make_float2(acc[r][0][2 * h] + acc[r][1][2 * h], acc[r][0][2 * h + 1] + acc[r][1][2 * h + 1]);
-    __syncthreads();
-    if (it < ITEMS) {
-      const float2* p = red + (size_t)((i_wn * R + i_r) * WK) * TT * 32 + i_m * 4 + i_t;
-      float v0 = 0.f, v1 = 0.f;
+    for (int h = 0; h < TT; ++h)
+      red[((r * WK + wk) * TT + h) * 32 + lane] =
+          make_float2(acc[r][0][2 * h] + acc[r][1][2 * h], acc[r][0][2 * h + 1] + acc[r][1][2 * h + 1]);
+  __syncthreads();
+  if (it < ITEMS) {
+    const float2* p = red + (size_t)(i_r * WK) * TT * 32 + i_m * 4 + i_t;
+    float v0 = 0.f, v1 = 0.f;
 #pragma unroll
-      for (int k = 0; k < WK; ++k) {
-        const float2 v = p[k * TT * 32];
-        v0 += v.x;
-        v1 += v.y;
-      }
-      if (blockIdx.x * WN + i_wn < a.tiles) few_finish(a, i_m, i_q, v0, v1, bias2.x, bias2.y, old2);
+    for (int k = 0; k < WK; ++k) {
+      const float2 v = p[k * TT * 32];
+      v0 += v.x;
+      v1 += v.y;
     }
+    few_finish(a, i_m, i_q, v0, v1, bias2.x, bias2.y, old2);
   }
 }
 
-template <int TT, int R, int WK, int WN, bool DIRECT, int U, bool RING = false>
-int launch(FewArgs& a, cudaStream_t s) {
-  static_assert(WK == 1 || WN * R * TT * 32 <= WK * WN * 32, "a thread finishes one pair of columns");
-  a.tiles = ceil_div(a.N, 8 * R);
-  const size_t smem = (RING ? (size_t)WK * WN * U * (R + (DIRECT ? TT : 0)) * 512 : 0) + (DIRECT ? 0 : (size_t)TT * 8 * few_ldx(a.K) * 2) + (WK > 1 ? (size_t)WN * R * WK * TT * 32 * 8 : 0);
-  static size_t allowed = 48 * 1024;
-  if (smem > 220 * 1024) TS_REFUSE(TS_ERR_UNSUPPORTED, "ts_linear_few: %zu bytes of shared memory", smem);
-  auto kernel = few_kernel<TT, R, WK, WN, DIRECT, U, RING>;
-  if (smem > allowed) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) TS_REFUSE((int)e, "ts_linear_few: shared memory %zu: %s", smem, cudaGetErrorString(e));
-    allowed = smem;
+// Many rows: the tokens in shared memory, one block of 16 warps an SM (two: where one round each leaves SMs without).  WK warps cut K of a tile of eight weight rows, 16 / WK tiles
+// make a round; a block takes rounds blockIdx.x, + gridDim.x, ... while its rings of U copies a lane run on across them.
+constexpr int ROWS_WARPS = 16;
+constexpr size_t ROWS_ALONE = 116 * 1024;      // no two of such blocks on an SM
+
+template <int TT, int WK, int U, int PER_SM>
+__global__ void __launch_bounds__(ROWS_WARPS * 32, PER_SM) few_rows_kernel(const __grid_constant__ FewArgs a) {
+  pdl_launch_dependents();
+  constexpr int WN = ROWS_WARPS / WK, THREADS = ROWS_WARPS * 32, ITEMS = WN * TT * 32;
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ float2 red[WK > 1 ? 2 : 1][WK > 1 ? ROWS_WARPS * TT * 32 : 1];                  // by turns: [wn][wk][token][4] pairs of columns
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3, wk = warp % WK, wn = warp / WK;
+  const int steps = (a.K + 31) >> 5, per = (steps + WK - 1) / WK;
+  const int s0 = wk * per, ns = max(0, min(steps, s0 + per) - s0);
+  const int rounds = (a.tiles + WN - 1) / WN;
+  const int mine = (int)blockIdx.x < rounds ? (rounds - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+  const int ldx = few_ldx(a.K);
+  unsigned char* ring = smem + (size_t)warp * U * 512 + lane * 16;                           // this lane's own 16 bytes of every 512
+  bf16* xs = reinterpret_cast<bf16*>(smem + (size_t)ROWS_WARPS * U * 512);
+
+  // (a tile past the last is the last again, and finishes nothing)
+  auto row_at = [&](int round) { return a.w + (size_t)few_row(a, min(round * WN + wn, a.tiles - 1), g) * a.K + s0 * 32 + 8 * t; };
+  int l_round = blockIdx.x, l_step = 0, l_left = mine * ns, l_slot = 0;
+  const bf16* wp = row_at(l_round);
+  auto fetch = [&] {
+    if (l_left > 0) {
+      const bool in = (s0 + l_step) * 32 + 8 * t < a.K;
+      own_copy(ring + l_slot * 512, in ? wp + l_step * 32 : a.w, in);
+      --l_left;
+      if (++l_step == ns) {
+        l_step = 0;
+        l_round += gridDim.x;
+        if (l_left > 0) wp = row_at(l_round);
+      }
+    }
+    cp_async_commit();
+    l_slot = l_slot + 1 == U ? 0 : l_slot + 1;
+  };
+  for (int u = 0; u < U; ++u) fetch();
+  pdl_wait();
+  {
+    const int chunks = ldx / 8;
+    for (int i = threadIdx.x; i < TT * 8 * chunks; i += THREADS) {
+      const int m = i / chunks, c = i - m * chunks;
+      const bool in = m < a.M && c * 8 < a.K;
+      *reinterpret_cast<uint4*>(xs + (size_t)m * ldx + c * 8) =
+          in ? __ldcg(reinterpret_cast<const uint4*>(a.x + (size_t)m * a.K + c * 8)) : make_uint4(0u, 0u, 0u, 0u);
+    }
   }
-  int blocks = ceil_div(a.tiles, WN);
-  if (WK == 1 && blocks > ts_sm_count()) blocks = ts_sm_count();
-  ts_launch(kernel, dim3(blocks), dim3(WK * WN * 32), smem, s, a);
+  __syncthreads();
+
+  const bf16* xrow = xs + (size_t)g * ldx + s0 * 32 + 8 * t;
+  int slot = 0;
+  for (int k = 0; k < mine; ++k) {
+    const int round = blockIdx.x + k * gridDim.x;
+    float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+#pragma unroll 4
+    for (int i = 0; i < ns; ++i) {
+      own_wait<U - 1>();
+      const uint4 w = *reinterpret_cast<const uint4*>(ring + slot * 512);
+      const uint4 x0 = *reinterpret_cast<const uint4*>(xrow + i * 32);
+      const uint4 x1 = TT == 2 ? *reinterpret_cast<const uint4*>(xrow + 8 * ldx + i * 32) : make_uint4(0u, 0u, 0u, 0u);
+      const unsigned a0[4] = {x0.x, x1.x, x0.y, x1.y}, a1[4] = {x0.z, x1.z, x0.w, x1.w};
+      mma_bf16(acc[0], a0, w.x, w.y);
+      mma_bf16(acc[1], a1, w.z, w.w);
+      fetch();
+      slot = slot + 1 == U ? 0 : slot + 1;
+    }
+    if constexpr (WK == 1) {
+      const int q = (round * WN + wn) * 4 + t;
+      if (round * WN + wn < a.tiles) {
+        few_store(a, g, q, acc[0][0] + acc[1][0], acc[0][1] + acc[1][1]);
+        if constexpr (TT == 2) few_store(a, g + 8, q, acc[0][2] + acc[1][2], acc[0][3] + acc[1][3]);
+      }
+    } else {
+#pragma unroll
+      for (int h = 0; h < TT; ++h)
+        red[k & 1][(warp * TT + h) * 32 + lane] = make_float2(acc[0][2 * h] + acc[1][2 * h], acc[0][2 * h + 1] + acc[1][2 * h + 1]);
+      __syncthreads();
+      if ((int)threadIdx.x < ITEMS) {
+        const int i_n = threadIdx.x / (TT * 32), at = threadIdx.x % (TT * 32);                // (the first warps finish; one barrier a round)
+        const float2* p = red[k & 1] + (size_t)i_n * WK * TT * 32 + at;
+        float v0 = 0.f, v1 = 0.f;
+#pragma unroll
+        for (int j = 0; j < WK; ++j) {
+          const float2 v = p[j * TT * 32];
+          v0 += v.x;
+          v1 += v.y;
+        }
+        if (round * WN + i_n < a.tiles) few_store(a, at >> 2, (round * WN + i_n) * 4 + (at & 3), v0, v1);
+      }
+    }
+  }
+  cp_async_wait<0>();
+}
+
+template <typename K> int allow_smem(K kernel, size_t smem, size_t* allowed) {
+  if (smem <= *allowed) return 0;
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    TS_REFUSE((int)e, "ts_linear_few: shared memory %zu: %s", smem, cudaGetErrorString(e));
+  }
+  *allowed = smem;
+  return 0;
+}
+
+template <int TT, int R, int WK, int U, bool RING = false>
+int launch(FewArgs& a, cudaStream_t s) {
+  a.tiles = ceil_div(a.N, 8 * R);
+  constexpr size_t smem = (RING ? (size_t)WK * U * (R + TT) * 512 : 0) + (size_t)R * WK * TT * 32 * 8;
+  static size_t allowed = 48 * 1024;
+  const int rc = allow_smem(few_kernel<TT, R, WK, U, RING>, smem, &allowed);
+  if (rc != 0) return rc;
+  ts_launch(few_kernel<TT, R, WK, U, RING>, dim3(a.tiles), dim3(WK * 32), smem, s, a);
+  TS_LAUNCH_CHECK();
+}
+
+template <int TT, int WK, bool TWO = false> int launch_rows(FewArgs& a, cudaStream_t s) {
+  constexpr int U = TT == 1 && !TWO ? 12 : (TT == 2 && TWO ? 6 : 8);
+  auto kernel = few_rows_kernel<TT, WK, U, TWO ? 2 : 1>;
+  a.tiles = ceil_div(a.N, 8);
+  size_t smem = (size_t)ROWS_WARPS * U * 512 + (size_t)TT * 8 * few_ldx(a.K) * 2;
+  if (smem > 210 * 1024) TS_REFUSE(TS_ERR_UNSUPPORTED, "ts_linear_few: %zu bytes of shared memory", smem);
+  // (launched while the kernel before still holds some SMs, two blocks would land on those that are free and stay there: an
+  // output head of 151,936 x 1,536 took 114 us as a step's last link, 82 with one an SM)
+  if (!TWO && smem < ROWS_ALONE) smem = ROWS_ALONE;
+  static size_t allowed = 48 * 1024;
+  const int rc = allow_smem(kernel, smem, &allowed);
+  if (rc != 0) return rc;
+  const int rounds = ceil_div(a.tiles, ROWS_WARPS / WK), most = (TWO ? 2 : 1) * ts_sm_count();
+  ts_launch(kernel, dim3(rounds < most ? rounds : most), dim3(ROWS_WARPS * 32), smem, s, a);
   TS_LAUNCH_CHECK();
 }
 
 // The instances by number (tests ask for one; callers leave it to few_plan).
 template <int TT> int launch_plan(FewArgs& a, int plan, cudaStream_t s) {
   switch (plan) {
-    case 1: return launch<TT, 2, 16, 1, true, 3>(a, s);
-    case 2: return launch<TT, 2, 8, 1, true, TT == 1 ? 6 : 4>(a, s);
-    case 3: return launch<TT, 2, 16, 1, true, 6, true>(a, s);
-    case 4: return launch<TT, 2, 8, 1, true, TT == 1 ? 8 : 5, true>(a, s);
-    case 5: return launch<TT, 1, 4, 4, false, TT == 1 ? 8 : 6, true>(a, s);
-    case 6: return launch<TT, 1, 2, 8, false, TT == 1 ? 8 : 6, true>(a, s);
-    case 7: return launch<TT, 1, 1, 16, false, 8, true>(a, s);
+    case 1: return launch<TT, 2, 16, 3>(a, s);
+    case 2: return launch<TT, 2, 8, TT == 1 ? 6 : 4>(a, s);
+    case 3: return launch<TT, 2, 16, 6, true>(a, s);
+    case 4: return launch<TT, 2, 8, TT == 1 ? 8 : 5, true>(a, s);
+    case 5: return launch_rows<TT, 8>(a, s);
+    case 6: return launch_rows<TT, 4>(a, s);
+    case 7: return launch_rows<TT, 2>(a, s);
+    case 8: return launch_rows<TT, 1>(a, s);
+    case 9: return launch_rows<TT, 4, true>(a, s);
   }
   TS_REFUSE(TS_ERR_SHAPE, "ts_linear_few: no plan %d", plan);
 }
@@ -377,10 +456,12 @@ template <int TT> int launch_plan(FewArgs& a, int plan, cudaStream_t s) {
 //    3.7 / 5.2; 1,536 x 8,960: 7.3 / 9.2; registers 10.8 there: their waits share six scoreboards);
 //  * for two blocks an SM: the same with 8 warps (4,632 x 1,536: 4.1 / 6.7; 3,584 x 3,584: 6.4 / 9.3).  Beyond that, and
 //    where K is long, blocks of one tile no longer divide the chip evenly: 3,584 x 18,944 33 / 30, left to tcgen05;
-//  * more rows: tokens in shared memory, 4, 2 or 1 warps a tile so that about 16 warps an SM have a tile (8,192 x 1,536:
-//    6.4 / 8.8; 9,728 x 896 gated: 5.6 / 6.9; 17,920 x 1,536 gated: 11.1 / 12.7; 151,936 x 1,536: 82 / 86), but for
-//    long rows of tokens, which leave room for one block only (6,144 x 3,584: 12.2 by the second rule, 14.9 / 12.6; 9 to 16
-//    tokens: 6,144 x 2,304 11.9 / 10.0, 12,288 x 1,536 12.0 / 11.2).
+//  * more rows: tokens in shared memory.  Few columns: two blocks of 16 warps an SM, 4 warps a tile (9,728 x 896 5.8 / 6.9, 8,192
+//    x 1,536 7.1 / 8.8, 20,480 x 1,024 10.8 / 15.5).  Else one block an SM, 1, 2, 4 or 8 warps a tile, whichever deals the tiles
+//    out most evenly (17,920 x 1,536 gated, 1 warp: 11.6 / 12.6; 151,936 x 1,536, 1 and 2 warps: 79 and 78 / 86; 13,440 x 1,536, 1, 2
+//    and 4 warps: 10.4, 11.3 and 11.3 / 11.1; 37,888 x 3,584 48 / 54).  Long rows of tokens leave too little room: 6,144 x 3,584
+//    12.2 by the second rule, 12.6 by tcgen05; 9 to 16 tokens, 6,144 x 2,304 11.9 / 10.0, 12,288 x 1,536 12.0 / 11.2.
+// Clusters that share K further (1,536 x 8,960 over 3 blocks each) lose: 10.5 us against 7.0.
 int few_plan(int M, int N, int K) {
   const int tiles16 = ceil_div(N, 16), sms = ts_sm_count();
   if (tiles16 <= sms) return K <= 2048 ? 1 : 3;
@@ -388,14 +469,23 @@ int few_plan(int M, int N, int K) {
   if (M > 8 && tiles16 <= 7 * sms && (K > 1900 || tiles16 > 5 * sms)) return 0;
   if (K > 2560 && tiles16 <= 6 * sms) return K <= 8192 ? 4 : 0;
   if (few_ldx(K) > 4600) return 0;                 // (16 tokens and the ring: 220 KB)
-  return tiles16 <= 4 * sms ? 5 : (tiles16 <= 7 * sms ? 6 : 7);
+  if (few_ldx(K) <= 1600 && (tiles16 <= 5 * sms || K <= 1100)) return 9;
+  // rounds of the busiest SM x (four times the steps of a round + what its end costs)
+  const int tiles = ceil_div(N, 8), steps = ceil_div(K, 32);
+  int best = 0, best_cost = 0;
+  for (int wk = 1, plan = 8; wk <= 8; wk *= 2, --plan) {
+    const int end = wk == 1 ? 8 : (wk == 2 ? 9 : 5 * wk);
+    const int cost = ceil_div(ceil_div(tiles, ROWS_WARPS / wk), sms) * (4 * ceil_div(steps, wk) + end);
+    if (best == 0 || cost < best_cost) best = plan, best_cost = cost;
+  }
+  return best;
 }
 
 int run(FewArgs& a, int plan, cudaStream_t s) {
   if (a.M > 16 || a.K % 8 != 0 || a.K <= 0)
     TS_REFUSE(TS_ERR_UNSUPPORTED, "ts_linear_few: M=%d N=%d K=%d is not taken by this kernel", a.M, a.N, a.K);
   if (((uintptr_t)a.x | (uintptr_t)a.w) & 15) TS_REFUSE(TS_ERR_ALIGN, "ts_linear_few: operands must be 16-byte aligned");
-  a.pairs = a.N % 2 == 0 && ((uintptr_t)a.out & (a.mode == FEW_FLOAT ? 7 : 3)) == 0;
+  a.pairs = a.N % 2 == 0 && ((uintptr_t)a.out & (a.mode == FEW_FLOAT || a.mode == FEW_STREAM ? 7 : 3)) == 0;
   if (plan == 0) {
     plan = few_plan(a.M, a.N, a.K);
     if (plan == 0) TS_REFUSE(TS_ERR_UNSUPPORTED, "ts_linear_few: N=%d K=%d is faster on tcgen05", a.N, a.K);
@@ -407,18 +497,20 @@ int run(FewArgs& a, int plan, cudaStream_t s) {
 
 // At most 16 tokens, K a multiple of 8, operands on 16-byte boundaries.  kind: 0 out is bfloat16, 1 float32,
 // 2 out[M, N / 2] = silu(g) * u (rows of w in blocks of 64 gates and their 64 ups, N a multiple of 128, no bias),
-// 4 out[M, N] += the product, both rounded to bfloat16.  plan: 0 = by the sizes (TS_ERR_UNSUPPORTED where the tcgen05
-// kernel is the faster one).
-TS_API int ts_linear_few(void* out, const void* x, const void* w, const void* bias, int M, int N, int K, int kind, int plan,
-                         void* stream) {
+// 4 out[M, N] += the product, both rounded to bfloat16, 5 the same for 32-bit rows (the product rounded to bfloat16),
+// 6 out = act(product rounded to bfloat16), `act` as ts_activation's kind.  plan: 0 = by the sizes (TS_ERR_UNSUPPORTED where
+// the tcgen05 kernel is the faster one).
+TS_API int ts_linear_few(void* out, const void* x, const void* w, const void* bias, int M, int N, int K, int kind, int act,
+                         int plan, void* stream) {
   if (M <= 0 || N <= 0) return 0;
-  if (kind < 0 || kind > 4 || kind == FEW_ROPE) TS_REFUSE(TS_ERR_SHAPE, "ts_linear_few: no kind %d", kind);
+  if (kind < 0 || kind > 6 || kind == FEW_ROPE) TS_REFUSE(TS_ERR_SHAPE, "ts_linear_few: no kind %d", kind);
   if (kind == FEW_GATED && (N % 128 != 0 || bias != nullptr))
     TS_REFUSE(TS_ERR_UNSUPPORTED, "ts_linear_few: gated N=%d is not taken by this kernel", N);
+  if (kind == FEW_ACT && (act < 1 || act > TS_ACT_LAST)) TS_REFUSE(TS_ERR_UNSUPPORTED, "ts_linear_few: activation %d", act);
   FewArgs a = {};
   a.x = (const bf16*)x; a.w = (const bf16*)w; a.bias = (const bf16*)bias; a.out = out;
   a.M = M; a.N = N; a.K = K;
-  a.mode = kind;
+  a.mode = kind; a.act = act;
   return run(a, plan, (cudaStream_t)stream);
 }
 

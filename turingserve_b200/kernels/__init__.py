@@ -68,7 +68,7 @@ class LazyProduct:
 class CudaOps:
     """ctypes front of ``libturingserve_b200.so``."""
 
-    ABI = 24
+    ABI = 25
     UNSUPPORTED = -4            # a kernel's refusal of a shape or layout another kernel takes
 
     def __init__(self, lib_path: str) -> None:
@@ -87,7 +87,7 @@ class CudaOps:
             "ts_linear_tc_gated": [P, P, P, I, I, I, P],
             "ts_linear_tc_resid": [P, P, P, P, I, I, I, I, P],
             "ts_attention_single": [P, I, I, P, I, I, P, P, P, P, P, I, I, I, I, I, I, I, I, F, F, P, I, I, P, I, P, P, I, I, P],
-            "ts_linear_few": [P, P, P, P, I, I, I, I, I, P],
+            "ts_linear_few": [P, P, P, P, I, I, I, I, I, I, P],
             "ts_linear_few_qkv_rope": [P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, P],
             "ts_linear_pair": [P, P, P, P, I, I, I, I, P],
             "ts_linear_pair_qkv": [P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, P],
@@ -592,7 +592,7 @@ class CudaOps:
         self._check(rc, "attention_single")
         return True
 
-    FEW_BF16, FEW_FLOAT, FEW_GATED, FEW_RESID = 0, 1, 2, 4
+    FEW_BF16, FEW_FLOAT, FEW_GATED, FEW_RESID, FEW_STREAM, FEW_ACT = 0, 1, 2, 4, 5, 6
     # up to this many tokens a product goes to the kernel whose weights pass through registers (it takes 16; 0: to tcgen05)
     few_tokens = int(os.environ.get("TURINGSERVE_B200_FEW_TOKENS", "16"))
     few_plan = 0         # its instance; 0: by the sizes
@@ -602,11 +602,11 @@ class CudaOps:
         return (0 < M <= self.few_tokens and self.gemm_mode == "auto" and x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16
                 and w.shape[1] % 8 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
 
-    def _few(self, out, x, w, bias, M: int, N: int, K: int, kind: int) -> bool:
+    def _few(self, out, x, w, bias, M: int, N: int, K: int, kind: int, act: int = 0) -> bool:
         """A few-token product on that kernel; False where it leaves the sizes to the tcgen05 kernel."""
         if not self.takes_few(M, x, w):
             return False
-        rc = self.lib.ts_linear_few(_ptr(out), _ptr(x), _ptr(w), _ptr(bias), M, N, K, kind, self.few_plan, self._stream())
+        rc = self.lib.ts_linear_few(_ptr(out), _ptr(x), _ptr(w), _ptr(bias), M, N, K, kind, act, self.few_plan, self._stream())
         if rc == self.UNSUPPORTED:
             return False
         self._check(rc, "linear_few")
@@ -676,6 +676,15 @@ class CudaOps:
         (stream - mean) / sqrt(variance + eps) * weight + norm_bias; 32-bit, rounded once.  ``out`` None: only the sum."""
         T, h = stream.shape
         part, splits, bias = None, 0, None
+        if (isinstance(add1, LazyProduct) and add2 is None and alpha == 1.0 and not first and stream.is_contiguous() and add1.shape == (T, h)
+                and self._few(stream, add1.x, add1.w, add1.bias, T, h, add1.w.shape[1], self.FEW_STREAM)):
+            if out is None and row is None:
+                return
+            dt, add1 = add1.dtype, None                  # (the product has added itself to the stream)
+            self._check(self.lib.ts_rmsnorm_wide(_ptr(out), _ptr(stream), None, None, _ptr(weight), float(eps), T, h, 0, _code(dt),
+                                                 _code(weight.dtype), None, 0, None, 1.0, _ptr(row), _ptr(norm_bias), self._stream()),
+                        "rmsnorm_stream")
+            return
         if isinstance(add1, (LazyProduct, Deferred)) and self.lib.ts_rmsnorm_wide_takes_parts(h):
             # a few-token product that was put off: its partial sums are summed here, no kernel of their own
             add1 = self._settle(add1)
@@ -706,6 +715,9 @@ class CudaOps:
     def activation(self, out, x, kind: str) -> None:
         """out = act(x) elementwise (32-bit arithmetic, one rounding); out may be x.  ``x`` may be a product that
         was put off: its partial sums are summed on the way."""
+        if (isinstance(x, LazyProduct) and out.dtype == torch.bfloat16 and out.is_contiguous() and tuple(out.shape) == x.shape
+                and self._few(out, x.x, x.w, x.bias, *x.shape, x.w.shape[1], self.FEW_ACT, self.ACTIVATIONS[kind])):
+            return
         x = self._settle(x)
         if isinstance(x, Deferred):
             rows, cols = x.shape
