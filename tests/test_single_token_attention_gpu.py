@@ -167,3 +167,32 @@ def test_the_new_row_is_read_after_the_kernel_before(ops):
         c.q = qkv[:, : H * D].reshape(4, H, D).clone()
         want, size = c.want(D ** -0.5)
         assert bool(((out.view(want.shape).double() - want).abs() <= 2.0 ** -8 * want.abs() + (2.0 ** -8 + 1e-4) * size).all())
+
+
+@pytest.mark.parametrize("H,KVH,D,V,page", [(12, 2, 128, 128, 16), (6, 1, 64, 64, 16), (12, 1, 576, 512, 64), (28, 1, 576, 512, 16)])
+def test_unsettled_steps_wait_for_every_row_and_array(ops, monkeypatch, H, KVH, D, V, page):
+    """All rows of the cache and the lengths, written by kernels of the same chain just before (behind one that runs a while), are
+    the ones that count with options and with latent rows."""
+    c = Case([33, 1, 160, 700], H, KVH, D, V, page, latent=D == 576)
+    caches = [t for t in (c.k, c.v) if t is not None]
+    sources = [t.clone() for t in caches]
+    rows = torch.arange(caches[0].numel() // D, device=DEV).int()
+    x, w = (torch.zeros(n, 4096, device=DEV).bfloat16() for n in (64, 16384))
+    product, lens, places = torch.empty(64, 16384, device=DEV).bfloat16(), c.step.seq_lens.clone(), i32([0, 1, 2, 3])
+    scale = 192 ** -0.5 if D == 576 else D ** -0.5
+    want, size = c.want(scale, cap=30.0, window=500)
+    calls = launched(ops, monkeypatch)
+    for _ in range(20):
+        for t in caches:
+            t.zero_()
+        c.step.seq_lens.fill_(1)
+        out = torch.full((4, H, V), float("nan"), device=DEV).bfloat16()
+        torch.cuda.synchronize()
+        ops.linear(product, x, w)
+        ops.feed_tokens(c.step.seq_lens, places, places, lens, 1 << 20)
+        for t, s in zip(caches, sources):
+            ops.gather_rows(t.view(-1, t.shape[-1]), s.view(-1, t.shape[-1]), rows)
+        ops.attention_biased(out, c.q, c.k, c.v, c.tables, c.step, KVH, page, scale, 30.0, None, 500)
+        err = (out.double() - want).abs()
+        assert bool((err <= 2.0 ** -8 * want.abs() + 1e-4 * size).all())
+    assert calls == [True] * 20

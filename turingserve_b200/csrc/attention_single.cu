@@ -7,7 +7,9 @@
 // The keys of a pair are cut over the blocks of one thread-block cluster, as large a cluster as lets all pairs run at
 // once.  What such a launch costs is a chain of latencies (with 2,048 keys a request all there is to read is 2.6 us at 8
 // requests), so: the first keys and values, up to 320 a block, are in shared memory before the wait for the kernel before is
-// over, all but the new token's row; no barrier stands between a warp and its keys (64 and 128 columns); and the blocks' sums
+// over, all but the new token's row, where the caller vouches that nothing queued before the step still writes what is read then
+// (`early`: the wait for one kernel is not a wait for those before it, as every kernel releases its successor at its start);
+// no barrier stands between a warp and its keys (64 and 128 columns); and the blocks' sums
 // cross the cluster once, pushed to the block that finishes a share of the output, as a read of a peer's shared memory costs a
 // round trip of 0.5 us and more.  The weights enter the second product as one bfloat16 term (P2 false: plain attention, as in
 // the reference) or as two.
@@ -45,6 +47,7 @@ struct SingleArgs {
   int window, block_of, keep;
   const float* sinks;
   AttnFinish fin;
+  int early;              // nothing before this step's kernels still writes its arrays or older rows: they are read before the wait
 };
 
 __device__ __forceinline__ void st_peer_v4(unsigned addr, float4 v) {
@@ -92,6 +95,7 @@ struct Shape {
 template <int DK, int DV, bool V_IN_K, int MT, int STAGE, int NKP, int WARPS, int CW, bool P2>
 __global__ void __launch_bounds__(WARPS * 32, 1) attention_single_kernel(const SingleArgs a) {
   pdl_launch_dependents();
+  if (!a.early) pdl_wait();
   using S = Shape<DK, DV, V_IN_K, MT, STAGE, NKP, WARPS, CW>;
   constexpr int THREADS = WARPS * 32, CHK = DK / 8, CHV = DV / 8, NTW = CW / 8, PVW = DV / CW;
   extern __shared__ __align__(128) unsigned char smem[];
@@ -401,6 +405,7 @@ template <int D, int HT, bool P2>
 __global__ void __launch_bounds__(SG_WARPS * 32, HT == 1 ? 2 : 1) attention_single_tiles_kernel(const SingleArgs a) {
   pdl_launch_dependents();
   if (gridDim.x > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // (this block runs: its shared memory may be written)
+  if (!a.early) pdl_wait();
   using S = Tiles<D, HT>;
   constexpr int THREADS = SG_WARPS * 32, CH = D / 8, KS = D / 16, MD = D / 16;
   extern __shared__ __align__(128) unsigned char smem[];
@@ -718,13 +723,15 @@ TS_API int ts_attention_single_supported(int H, int KVH, int Dk, int Dv, int v_i
 }
 
 // Arguments as ts_attention_biased_mma's for requests of one token each.  reach: the most keys any of them sees.  two_terms:
-// the weights enter the second product as two bfloat16 terms.  TS_ERR_UNSUPPORTED: shapes, or strides off their boundaries, or
+// the weights enter the second product as two bfloat16 terms.  early: block_tables, q_start, seq_lens and the cache rows before
+// each request's last were written by work that the stream has finished before the step's first kernel starts (a copy from the
+// host stands between, say), so they are read before the wait for the kernel before; 0: after it.  TS_ERR_UNSUPPORTED: shapes, or strides off their boundaries, or
 // clusters switched off.
 TS_API int ts_attention_single(void* out, int out_ts, int out_hs, const void* q, int q_ts, int q_hs, const void* k_cache,
                                const void* v_cache, const int* block_tables, const int* q_start, const int* seq_lens, int B,
                                int table_width, int reach, int H, int KVH, int Dk, int Dv, int page, float scale, float softcap,
                                const float* slopes, int window, int block_of, const float* sinks, int keep, const float* out_freq,
-                               const void* gate, int gate_ts, int two_terms, void* stream) {
+                               const void* gate, int gate_ts, int two_terms, int early, void* stream) {
   if (B <= 0) return 0;
   const int v_in_k = v_cache == nullptr;
   if (!ts_attention_single_supported(H, KVH, Dk, Dv, v_in_k, TS_BF16) || !ts_clusters_enabled())
@@ -743,6 +750,7 @@ TS_API int ts_attention_single(void* out, int out_ts, int out_hs, const void* q,
   a.scale = scale; a.softcap = softcap; a.slopes = slopes;
   a.window = window; a.block_of = block_of; a.keep = keep; a.sinks = sinks;
   a.fin.out_freq = out_freq; a.fin.gate = gate; a.fin.gate_ts = gate_ts;
+  a.early = early;
   cudaStream_t s = (cudaStream_t)stream;
   if (v_in_k && out_freq != nullptr) TS_REFUSE(TS_ERR_UNSUPPORTED, "ts_attention_single: the pairs of latent values are not turned");
   if (v_in_k && H / KVH <= 16) return launch<576, 512, true, 1, 80, 3, 16, 32, true>(a, B, reach, s);

@@ -69,6 +69,10 @@ class StepInputs:
     all_rows_sampled: bool = False
     # the step's token ids on the host, where it knows them all (None: some are fed back on the device)
     host_ids: np.ndarray | None = None
+    # Whoever runs the step vouches that its arrays and the cache rows of earlier steps are in place before its first
+    # kernel starts (a copy from the host stands between them and the step): attention may read them while the
+    # step's kernels before it still run.  A step that is built ahead, behind others that still run, is not settled.
+    settled: bool = False
 
 
 # From about this many keys under the decode rows of a step (requests x longest context), or a third of them in one

@@ -68,7 +68,8 @@ class ModelRunner:
         if shape is not None:
             logits = self._replay(shape, entries, prev_tokens)
         else:
-            step = self.builder.build(entries)
+            # (the arrays' copy from the host has just been queued: it ends after the step before, and before this one begins)
+            step = dataclasses.replace(self.builder.build(entries), settled=True)
             self._feed(step, prev_tokens)
             logits = self.forward(step)
         for e in entries:
@@ -178,8 +179,9 @@ class _StepGraph:
         n_dec = sum(1 for e in entries if len(e.tokens) == 1)
         step = r.builder.build(entries, fixed_width=r.max_pages, pad_requests=self.size - n_dec, arena=self.arena)
         # launch geometry must not depend on this step's lengths: size it for the longest context
+        # (settled: a replay begins when the copy of its arrays, and so the step before it, has ended)
         return dataclasses.replace(step, sample_rows=self.rows, max_seq_len=r.max_model_len,
-                                   streaming_decode=self.streaming, all_rows_sampled=self.portion == 0)
+                                   streaming_decode=self.streaming, all_rows_sampled=self.portion == 0, settled=True)
 
     def _wanted(self, entries: list[StepEntry]) -> torch.Tensor | None:
         """The caller's rows (order of ``entries`` and of their ``want``) out of the static logits."""

@@ -68,7 +68,7 @@ class LazyProduct:
 class CudaOps:
     """ctypes front of ``libturingserve_b200.so``."""
 
-    ABI = 25
+    ABI = 26
     UNSUPPORTED = -4            # a kernel's refusal of a shape or layout another kernel takes
 
     def __init__(self, lib_path: str) -> None:
@@ -86,7 +86,7 @@ class CudaOps:
             "ts_silu_mul_ex": [P, P, I, I, I, I, P],
             "ts_linear_tc_gated": [P, P, P, I, I, I, P],
             "ts_linear_tc_resid": [P, P, P, P, I, I, I, I, P],
-            "ts_attention_single": [P, I, I, P, I, I, P, P, P, P, P, I, I, I, I, I, I, I, I, F, F, P, I, I, P, I, P, P, I, I, P],
+            "ts_attention_single": [P, I, I, P, I, I, P, P, P, P, P, I, I, I, I, I, I, I, I, F, F, P, I, I, P, I, P, P, I, I, I, P],
             "ts_linear_few": [P, P, P, P, I, I, I, I, I, I, P],
             "ts_linear_few_qkv_rope": [P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, P],
             "ts_linear_pair": [P, P, P, P, I, I, I, I, P],
@@ -509,7 +509,9 @@ class CudaOps:
     def attention(self, out, qkv, k_cache, v_cache, block_tables, step, H, KVH, D, page_size, scale,
                   window) -> None:
         """Rows of requests with one token (the first ``step.num_decode`` requests) go to a
-        split-key decode kernel when one takes the shape; the rest to the chunk kernels."""
+        split-key decode kernel when one takes the shape; the rest to the chunk kernels.  The decode kernels read the
+        step's arrays and all cache rows but each request's last while kernels queued before still run: those must
+        not be written by kernels of this library without a copy, an event or another kernel between."""
         w = 0 if window is None else int(window)
         code = _code(qkv.dtype)
         B, nd = step.num_requests, 0
@@ -523,7 +525,7 @@ class CudaOps:
             streaming = long or step.num_decode * KVH * 8 > self.num_sms
         if (self.use_fast_attention and step.num_decode > 0 and qkv.dtype == torch.bfloat16 and self.single_wins(step, KVH, long)
                 and self._attention_single(out.view(out.shape[0], H, D), qkv[:, :H * D].view(qkv.shape[0], H, D), k_cache, v_cache,
-                                           block_tables, step, KVH, page_size, scale, 0.0, None, w, 0, None, 0, None, None, False)):
+                                           block_tables, step, KVH, page_size, scale, 0.0, None, w, 0, None, 0, None, None, False, True)):
             nd = step.num_decode
         if (nd == 0 and self.use_fast_attention and streaming and step.num_decode > 0
                 and self.lib.ts_attention_decode_tma_supported(H, KVH, D, page_size, code)):
@@ -575,9 +577,10 @@ class CudaOps:
                                          and step.num_decode * KVH <= self.num_sms)
 
     def _attention_single(self, out, q, k_cache, v_cache, block_tables, step, KVH: int, page_size: int, scale: float, softcap: float,
-                          slopes, window: int, block_of: int, sinks, keep: int, out_freq, gate, two_terms: bool) -> bool:
+                          slopes, window: int, block_of: int, sinks, keep: int, out_freq, gate, two_terms: bool, early: bool) -> bool:
         """The first ``step.num_decode`` requests, one token each, on the kernel whose blocks of a (request, kv head) are one
-        cluster; False where it does not take the shape."""
+        cluster; False where it does not take the shape.  ``early``: the step's arrays and the cache rows before each request's
+        last are read before the wait for the kernel before."""
         H, Dk = q.shape[1], q.shape[2]
         reach = min(step.max_seq_len, window + keep) if window else step.max_seq_len
         if block_of:
@@ -586,7 +589,7 @@ class CudaOps:
             _ptr(out), out.stride(0), out.stride(1), _ptr(q), q.stride(0), q.stride(1), _ptr(k_cache), _ptr(v_cache), _ptr(block_tables),
             _ptr(step.q_start), _ptr(step.seq_lens), step.num_decode, block_tables.shape[1], reach, H, KVH, Dk, out.shape[2], page_size,
             float(scale), float(softcap), _ptr(slopes), window, block_of, _ptr(sinks), keep, _ptr(out_freq), _ptr(gate),
-            0 if gate is None else gate.stride(0), 1 if two_terms else 0, self._stream())
+            0 if gate is None else gate.stride(0), 1 if two_terms else 0, 1 if early else 0, self._stream())
         if rc == self.UNSUPPORTED:
             return False
         self._check(rc, "attention_single")
@@ -1050,7 +1053,7 @@ class CudaOps:
             # rows win at every count)
             if (spread and self.single_mode and (G <= 8 or v_in_k or nd * KVH <= self.num_sms)
                     and self._attention_single(out, q, k_cache, v_cache, block_tables, step, KVH, page_size, scale, softcap, slopes, w,
-                                               c, sinks, keep, out_freq, gate, True)):
+                                               c, sinks, keep, out_freq, gate, True, getattr(step, "settled", False))):
                 if nd < B:
                     self._check(portions(nd, B - nd), "attention_biased")
                 return
