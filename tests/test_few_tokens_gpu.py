@@ -117,3 +117,17 @@ def test_sizes_left_to_tcgen05(ops):
     assert not ops._few(out, x, w, None, 3, 3584, 8968, ops.FEW_FLOAT)
     ops.linear(out, x, w)
     assert float((out - (x.double() @ w.double().T)).abs().max()) < 2e-5 * 8968
+
+
+# (which kernel is the faster one was measured with the residual add and norm, the rotation and plainly; the sizes lie on both
+# sides of each line of the rule)
+@pytest.mark.parametrize("M,N,K,taken", [(1, 2048, 18432, True), (16, 1536, 20480, False), (8, 256, 28416, False), (16, 1536, 16384, True), (12, 2432, 8192, False), (8, 2432, 8192, True),
+                                         (8, 2816, 7168, True), (12, 2816, 7168, False), (12, 2560, 7168, True), (12, 3072, 7168, True), (1, 2816, 8192, False),
+                                         (1, 4736, 5120, True), (1, 4752, 5120, False), (8, 5120, 3584, True), (1, 5120, 4352, False), (8, 5120, 5120, False), (9, 5120, 1536, True),
+                                         (9, 5120, 2048, False), (1, 5632, 7168, False), (8, 6144, 6144, True), (8, 6144, 8192, False), (8, 7168, 8192, True)])
+def test_which_sizes_are_left_to_tcgen05(ops, M, N, K, taken):
+    x, w, out = rnd(1, M, K), rnd(2, N, K, std=0.05), torch.empty(M, N, device=DEV)
+    assert ops._few(out, x, w, None, M, N, K, ops.FEW_FLOAT) == taken
+    ops.linear(out, x, w)
+    size = (x.double().abs() @ w.double().abs().T).clamp_min(1e-3)
+    assert float(((out - x.double() @ w.double().T).abs() / size).max()) < 2e-5

@@ -453,9 +453,17 @@ template <int TT> int launch_plan(FewArgs& a, int plan, cudaStream_t s) {
 // with residual add at 8 tokens, weights from DRAM, in us, against the tcgen05 kernel's:
 //  * tiles of 16 rows for at most one block an SM: 16 warps cut K; all of a warp's weights in registers at once while
 //    they are few (1,536 x 1,536: 2.3 / 4.6; 2,048 x 1,536: 2.6 / 5.0), else a ring in shared memory (896 x 4,864:
-//    3.7 / 5.2; 1,536 x 8,960: 7.3 / 9.2; registers 10.8 there: their waits share six scoreboards);
-//  * for two blocks an SM: the same with 8 warps (4,632 x 1,536: 4.1 / 6.7; 3,584 x 3,584: 6.4 / 9.3).  Beyond that, and
-//    where K is long, blocks of one tile no longer divide the chip evenly: 3,584 x 18,944 33 / 30, left to tcgen05;
+//    3.7 / 5.2; 1,536 x 8,960: 7.3 / 9.2; registers 10.8 there: their waits share six scoreboards).  Very long rows have the
+//    bytes to keep tcgen05's bulk copies busy (16 tokens: 1,536 x 18,432 16.9 / 15.7; with the norm behind, 1,536 x 28,416
+//    26.6 / 24.2, 256 x 20,480 14.9 / 14.3);
+//  * for two blocks an SM: the same with 8 warps (4,632 x 1,536: 4.1 / 6.7; 3,584 x 3,584: 6.4 / 9.3).  Where K is long too,
+//    blocks of one tile no longer divide the chip evenly: 3,584 x 18,944 33 / 30, left to tcgen05, and sooner where few SMs
+//    have a second block (12 tokens: 2,432 x 8,192 13.4 / 12.0; with the norm, 2,816 x 7,168 13.5 / 12.4, but 2,560 x 7,168
+//    13.6 / 14.1);
+//  * up to two and a half blocks an SM: still that, while a third round costs less than the rows' kernel below (one token, with the
+//    norm: 5,120 x 2,560 9.6 / 9.4, 10.9 by rows; q/k/v 5,120 x 2,304 8.4 / 8.4, 9.1 by rows; 9 tokens, 5,120 x 1,536 8.7 / 8.6,
+//    9.9 by rows); above, tcgen05 (5,120 x 4,352 14.0 / 12.4, 5,120 x 5,120 15.2 / 14.0), and up to two and
+//    three quarters once K is long (without a norm, 6,144 x 7,168 19.7 / 18.8, 6,144 x 8,192 23.6 / 20.9);
 //  * more rows: tokens in shared memory.  Few columns: two blocks of 16 warps an SM, 4 warps a tile (9,728 x 896 5.8 / 6.9, 8,192
 //    x 1,536 7.1 / 8.8, 20,480 x 1,024 10.8 / 15.5).  Else one block an SM, 1, 2, 4 or 8 warps a tile, whichever deals the tiles
 //    out most evenly (17,920 x 1,536 gated, 1 warp: 11.6 / 12.6; 151,936 x 1,536, 1 and 2 warps: 79 and 78 / 86; 13,440 x 1,536, 1, 2
@@ -464,8 +472,16 @@ template <int TT> int launch_plan(FewArgs& a, int plan, cudaStream_t s) {
 // Clusters that share K further (1,536 x 8,960 over 3 blocks each) lose: 10.5 us against 7.0.
 int few_plan(int M, int N, int K) {
   const int tiles16 = ceil_div(N, 16), sms = ts_sm_count();
-  if (tiles16 <= sms) return K <= 2048 ? 1 : 3;
-  if (tiles16 <= 2 * sms) return K <= 1536 ? 2 : (K <= 8192 ? 4 : 0);
+  if (tiles16 <= sms) return K <= 2048 ? 1 : (K <= (M > 8 ? 16384 : 18432) ? 3 : 0);
+  if (tiles16 <= 2 * sms) {
+    if (4 * tiles16 < 5 * sms && K > (8 * tiles16 <= 9 * sms ? (M > 8 ? 7168 : 8192) : (M > 8 ? 5120 : 7168))) return 0;
+    return K <= 1536 ? 2 : (K <= 8192 ? 4 : 0);
+  }
+  if (2 * tiles16 <= 5 * sms && K > 1100) {
+    if (K <= (M > 8 ? 1900 : 3584)) return 4;
+    return 0;
+  }
+  if (4 * tiles16 <= 11 * sms && K > 6144) return 0;
   if (M > 8 && tiles16 <= 7 * sms && (K > 1900 || tiles16 > 5 * sms)) return 0;
   if (K > 2560 && tiles16 <= 6 * sms) return K <= 8192 ? 4 : 0;
   if (few_ldx(K) > 4600) return 0;                 // (16 tokens and the ring: 220 KB)
