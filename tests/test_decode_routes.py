@@ -46,7 +46,7 @@ def front(**answers) -> CudaOps:
     ops = CudaOps.__new__(CudaOps)
     ops.lib = Library(**answers)
     ops.num_sms, ops.launches, ops.decode_stages = 148, 0, 3
-    ops.decode_kernel, ops.use_fast_attention, ops.use_tc_attention = "auto", True, True
+    ops.decode_kernel, ops.use_fast_attention, ops.use_tc_attention, ops.use_tma_decode = "auto", True, True, True
     ops.single_mode, ops.biased_decode_splits = 1, 0
     ops._buffers, ops._outgrown, ops._decode_slots = {}, [], {}
     ops._stream = lambda: 0
@@ -64,6 +64,13 @@ def biased(ops, step, H=12, KVH=2, D=128, V=128, latent=False, page=16):
     k = torch.zeros(B + 1, KVH, page, D).bfloat16()
     ops.attention_biased(torch.zeros(B, H, V).bfloat16(), torch.zeros(B, H, D).bfloat16(), k, None if latent else k,
                          torch.zeros(B, 4, dtype=torch.int32), step, KVH, page, 0.1, 30.0, None, None)
+
+
+def plain(ops, step, H=12, KVH=2, D=128, page=16):
+    B = step.num_requests
+    k = torch.zeros(B + 1, KVH, page, D).bfloat16()
+    ops.attention(torch.zeros(B, H * D).bfloat16(), torch.zeros(B, (H + 2 * KVH) * D).bfloat16(), k, k, torch.zeros(B, 4, dtype=torch.int32),
+                  step, H, KVH, D, page, 0.1, None)
 
 
 EARLY = -2                     # the argument's place in ts_attention_single
@@ -100,3 +107,22 @@ def test_the_runner_settles_its_steps_and_the_builder_does_not(tmp_path):
         assert _StepGraph(runner, 1, 0, False)._build([StepEntry(rc, [1], [0])]).settled
     finally:
         kernels.use(None)
+
+
+def test_a_fault_of_the_streaming_kernel_takes_only_that_kernel_off():
+    """Single tokens stay on the kernel that has no bounded wait; what the streaming kernel took goes to the older one."""
+    ops = front()
+    ops.fault_reported([0, 0, 7, 0])
+    ops.lib.calls.clear()
+    plain(ops, step_of([40, 7]))
+    assert ops.lib.launched() == ["ts_attention_single"]
+    ops.lib.calls.clear()
+    plain(ops, step_of([40] * 100))                    # more (request, kv head) pairs than SMs
+    assert ops.lib.launched() == ["ts_attention_decode"]
+    for kernel in ("tma", "cp"):
+        ops = front()
+        ops.decode_kernel = kernel
+        ops.fault_reported([0, 0, 7, 0])
+        ops.lib.calls.clear()
+        plain(ops, step_of([40, 7]))
+        assert ops.lib.launched() == ["ts_attention_decode"]

@@ -264,6 +264,7 @@ class CudaOps:
         self._outgrown: list[torch.Tensor] = []
         self._decode_slots: dict = {}
         self.use_fast_attention = True
+        self.use_tma_decode = True          # (off after a fault of that kernel)
         self.use_fused_step = True          # a whole decode step as one kernel where the model allows it
         self.use_library_gemm = True
         self.max_splits = 10        # (the fused reduce kernels load up to 16 partial sums in one go)
@@ -527,7 +528,7 @@ class CudaOps:
                 and self._attention_single(out.view(out.shape[0], H, D), qkv[:, :H * D].view(qkv.shape[0], H, D), k_cache, v_cache,
                                            block_tables, step, KVH, page_size, scale, 0.0, None, w, 0, None, 0, None, None, False, True)):
             nd = step.num_decode
-        if (nd == 0 and self.use_fast_attention and streaming and step.num_decode > 0
+        if (nd == 0 and self.use_fast_attention and streaming and self.use_tma_decode and step.num_decode > 0
                 and self.lib.ts_attention_decode_tma_supported(H, KVH, D, page_size, code)):
             nd = step.num_decode
             nsplit = self.decode_splits_tma(nd, KVH, D, step.max_seq_len)
@@ -1501,7 +1502,7 @@ class CudaOps:
         if int(status[1]):
             self.use_tc_attention = False
         if int(status[2]):
-            self.decode_kernel = "cp"
+            self.use_tma_decode = False
         if int(status[3]):
             self.use_fused_step = False
         self.lib.ts_clear_status(self._stream())
