@@ -126,3 +126,13 @@ def test_a_fault_of_the_streaming_kernel_takes_only_that_kernel_off():
         ops.lib.calls.clear()
         plain(ops, step_of([40, 7]))
         assert ops.lib.launched() == ["ts_attention_decode"]
+
+
+@pytest.mark.parametrize("shape", [dict(), dict(H=12, KVH=1, D=576, V=512, latent=True)], ids=["options", "latent"])
+def test_a_number_of_splits_is_for_the_kernel_that_splits(shape):
+    for splits, name in ((0, "ts_attention_single"), (1, "ts_attention_biased_mma"), (3, "ts_attention_biased_mma")):
+        ops = front()
+        ops._buffer = lambda *a, **k: None
+        ops.biased_decode_splits = splits
+        biased(ops, step_of([700, 7]), **shape)
+        assert ops.lib.launched() == [name]

@@ -196,3 +196,21 @@ def test_unsettled_steps_wait_for_every_row_and_array(ops, monkeypatch, H, KVH, 
         err = (out.double() - want).abs()
         assert bool((err <= 2.0 ** -8 * want.abs() + 1e-4 * size).all())
     assert calls == [True] * 20
+
+
+@pytest.mark.parametrize("splits", [1, 3])
+@pytest.mark.parametrize("H,KVH,D,V,page", [(12, 2, 128, 128, 64), (16, 1, 64, 64, 16), (12, 1, 576, 512, 64), (28, 1, 576, 512, 16)])
+def test_a_number_of_splits_runs_the_kernel_that_splits(ops, monkeypatch, splits, H, KVH, D, V, page):
+    c = Case([1, 64, 333, 2100, 700], H, KVH, D, V, page, latent=D == 576)
+    monkeypatch.setattr(ops, "biased_decode_splits", splits)
+    calls, took = launched(ops, monkeypatch), []
+    real = ops.lib.ts_attention_biased_mma
+    monkeypatch.setattr(ops.lib, "ts_attention_biased_mma", lambda *a: took.append(a[23]) or real(*a))
+    sinks, gate = torch.rand(H, device=DEV), torch.randn(5, H, device=DEV).bfloat16()
+    scale = 192 ** -0.5 if D == 576 else D ** -0.5
+    for window, keep in ((None, 0), (500, 40)):
+        out = torch.full((5, H, V), float("nan"), device=DEV).bfloat16()
+        ops.attention_biased(out, c.q, c.k, c.v, c.tables, c.step, KVH, page, scale, 20.0, None, window, None, sinks, keep, None, gate)
+        want, size = c.want(scale, cap=20.0, window=window, sinks=sinks, keep=keep, gate=gate)
+        assert bool(((out.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-4 * size).all())
+    assert calls == [] and took == [splits, splits]

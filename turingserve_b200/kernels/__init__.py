@@ -978,6 +978,7 @@ class CudaOps:
     # outnumber the SMs stay with the other (256 single tokens of 48 heads over one kv head of 128, 140 keys: 18.7 against 17.2 us;
     # 600 keys: 29.3 against 47.9).
     biased_tc_keys = int(os.environ.get("TURINGSERVE_B200_BIASED_TC_KEYS", "128"))
+    # pieces the keys of single tokens are cut into by the kernels of attention_biased*.cu (above 0: those take them, whatever the size)
     biased_decode_splits = int(os.environ.get("TURINGSERVE_B200_BIASED_DECODE_SPLITS", "0"))
 
     def attention_biased(self, out, q, k_cache, v_cache, block_tables, step, KVH: int, page_size: int, scale: float,
@@ -1052,7 +1053,7 @@ class CudaOps:
 
             # (16 heads over one kv head of 128, 256 requests of 600 keys: 40 us, 36 with the launch below; 8 heads or latent
             # rows win at every count)
-            if (spread and self.single_mode and (G <= 8 or v_in_k or nd * KVH <= self.num_sms)
+            if (spread and self.single_mode and splits <= 0 and (G <= 8 or v_in_k or nd * KVH <= self.num_sms)
                     and self._attention_single(out, q, k_cache, v_cache, block_tables, step, KVH, page_size, scale, softcap, slopes, w,
                                                c, sinks, keep, out_freq, gate, True, getattr(step, "settled", False))):
                 if nd < B:
