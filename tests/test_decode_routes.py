@@ -136,3 +136,27 @@ def test_a_number_of_splits_is_for_the_kernel_that_splits(shape):
         ops.biased_decode_splits = splits
         biased(ops, step_of([700, 7]), **shape)
         assert ops.lib.launched() == [name]
+
+
+def test_long_contexts_that_the_streaming_kernel_does_not_take():
+    """Pages that are no multiple of 16, caches that no tensor map spans: clusters, or the older kernel for a pair or two."""
+    single, tma, older = "ts_attention_single", "ts_attention_decode_tma", "ts_attention_decode"
+    for lens, KVH, page, answer, want in (
+            ([16000] * 8, 2, 16, 0, [tma]), ([16000] * 8, 2, 24, 0, [single]), ([16000] * 8, 2, 16, CudaOps.UNSUPPORTED, [tma, single]),
+            ([64000], 2, 16, 0, [tma]), ([64000], 2, 24, 0, [older]), ([64000], 2, 16, CudaOps.UNSUPPORTED, [tma, older]),
+            ([64000], 4, 24, 0, [single]), ([300] * 8, 2, 24, 0, [single]),
+            ([300] * 100, 2, 24, 0, [older]), ([300] * 100, 2, 16, CudaOps.UNSUPPORTED, [tma, older])):
+        ops = front(ts_attention_decode_tma=answer)
+        ops._buffer = lambda *a, **k: None
+        plain(ops, step_of(lens), KVH=KVH, page=page)
+        assert ops.lib.launched() == want, (lens, KVH, page, answer)
+
+
+def test_the_front_and_the_steps_share_the_threshold(monkeypatch):
+    from turingserve_b200.engine import batch
+    for keys, want in ((1000, "ts_attention_single"), (120, "ts_attention_decode_tma")):
+        monkeypatch.setattr(batch, "STREAMING_DECODE_KEYS", keys)
+        ops = front()
+        ops._buffer = lambda *a, **k: None
+        plain(ops, step_of([40, 40, 40]))
+        assert ops.lib.launched() == [want]

@@ -214,3 +214,16 @@ def test_a_number_of_splits_runs_the_kernel_that_splits(ops, monkeypatch, splits
         want, size = c.want(scale, cap=20.0, window=window, sinks=sinks, keep=keep, gate=gate)
         assert bool(((out.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-4 * size).all())
     assert calls == [] and took == [splits, splits]
+
+
+@pytest.mark.parametrize("H,KVH,D,page,lens,cluster", [(12, 2, 128, 24, [40000, 33000], True), (14, 2, 64, 24, [50000, 7], True),
+                                                       (12, 2, 128, 24, [40000], False), (28, 4, 128, 24, [34001], True)])
+def test_long_contexts_on_pages_that_the_streaming_kernel_does_not_take(ops, monkeypatch, H, KVH, D, page, lens, cluster):
+    c = Case(lens, H, KVH, D, D, page)
+    calls = launched(ops, monkeypatch)
+    qkv = torch.cat([c.q.flatten(1), torch.zeros(len(lens), 2 * KVH * D, device=DEV).bfloat16()], 1)
+    out = torch.full((len(lens), H * D), float("nan"), device=DEV).bfloat16()
+    ops.attention(out, qkv, c.k, c.v, c.tables, c.step, H, KVH, D, page, D ** -0.5, None)
+    assert calls == ([True] if cluster else [])
+    want, size = c.want(D ** -0.5)
+    assert bool(((out.view(want.shape).double() - want).abs() <= 2.0 ** -8 * want.abs() + (2.0 ** -8 + 1e-4) * size).all())

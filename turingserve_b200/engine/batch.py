@@ -78,8 +78,9 @@ class StepInputs:
 # From about this many keys under the decode rows of a step (requests x longest context), or a third of them in one
 # request, the kernel that cuts a request's keys over as many blocks as the chip has takes the decode attention, below
 # the one whose blocks of a (request, kv head) are one cluster (12 heads over 2 kv heads of 128, us a launch: 1 x 16,000
-# keys 15.7 / 12.4, 1 x 32,000 19.3 / 20.8, 1 x 64,000 24.6 / 38.1, 8 x 32,000 50.5 / 53.0).  The kernels' front adds
-# its own rule for many requests.
+# keys 15.7 / 12.4, 1 x 32,000 19.3 / 20.8, 1 x 64,000 24.6 / 38.1, 8 x 32,000 50.5 / 53.0; where clusters are switched off, the
+# third costs nothing against the older kernel: 1 x 32,000 18.9 / 18.8, heads of 64 14.5 / 18.4).  The kernels' front adds its
+# own rules for many requests and for caches that the streaming kernel does not take.
 STREAMING_DECODE_KEYS = 98304
 
 

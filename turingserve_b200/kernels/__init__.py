@@ -520,16 +520,28 @@ class CudaOps:
         # long contexts: the streaming kernel cuts a request's keys over as many blocks as there are
         long = getattr(step, "streaming_decode", None)
         if long is None:
-            long = max(step.num_decode, 3) * step.max_seq_len >= 98304
+            from turingserve_b200.engine.batch import streaming_decode
+            long = streaming_decode(step.num_decode, step.max_seq_len)
         streaming = self.decode_kernel == "tma"
         if self.decode_kernel == "auto":
             streaming = long or step.num_decode * KVH * 8 > self.num_sms
-        if (self.use_fast_attention and step.num_decode > 0 and qkv.dtype == torch.bfloat16 and self.single_wins(step, KVH, long)
-                and self._attention_single(out.view(out.shape[0], H, D), qkv[:, :H * D].view(qkv.shape[0], H, D), k_cache, v_cache,
-                                           block_tables, step, KVH, page_size, scale, 0.0, None, w, 0, None, 0, None, None, False, True)):
+        tma = (streaming and self.use_tma_decode and step.num_decode > 0
+               and bool(self.lib.ts_attention_decode_tma_supported(H, KVH, D, page_size, code)))
+        # Without the streaming kernel (pages or caches that it does not take, a fault) long contexts leave the clusters only for
+        # a few pairs, which the older kernel cuts over more blocks (12 heads over 2 of 128: 1 x 48,000 keys 29.6 us on a cluster /
+        # 21.4; 2 x 48,000 30.8 / 32.5; 8 x 16,000 27.9 / 36.1; 28 over 4, 1 x 48,000 30.7 / 33.6)
+        few_pairs = step.num_decode * KVH < 4
+
+        def single(barred: bool) -> bool:
+            return (self.use_fast_attention and step.num_decode > 0 and qkv.dtype == torch.bfloat16
+                    and self.single_wins(step, KVH, barred)
+                    and self._attention_single(out.view(out.shape[0], H, D), qkv[:, :H * D].view(qkv.shape[0], H, D), k_cache,
+                                               v_cache, block_tables, step, KVH, page_size, scale, 0.0, None, w, 0, None, 0, None,
+                                               None, False, True))
+
+        if single(long and (tma or few_pairs)):
             nd = step.num_decode
-        if (nd == 0 and self.use_fast_attention and streaming and self.use_tma_decode and step.num_decode > 0
-                and self.lib.ts_attention_decode_tma_supported(H, KVH, D, page_size, code)):
+        if nd == 0 and self.use_fast_attention and tma:
             nd = step.num_decode
             nsplit = self.decode_splits_tma(nd, KVH, D, step.max_seq_len)
             scratch, counters = self._decode_scratch(nd, H, KVH, D, nsplit, qkv.device)
@@ -538,7 +550,7 @@ class CudaOps:
                 _ptr(step.q_start), _ptr(step.seq_lens), nd, width, H, KVH, D, page_size, k_cache.shape[0],
                 float(scale), w, nsplit, self.decode_stages, self._stream())
             if rc == self.UNSUPPORTED:          # e.g. key and value caches that no one tensor map spans
-                nd = 0
+                nd = step.num_decode if long and single(few_pairs) else 0
             else:
                 self._check(rc, "attention_decode_tma")
         if nd == 0 and self.use_fast_attention and step.num_decode > 0 and self.lib.ts_attention_decode_supported(H, KVH, D, code):
@@ -573,8 +585,12 @@ class CudaOps:
     # single tokens on the kernel whose blocks of a (request, kv head) are one cluster (0: never)
     single_mode = int(os.environ.get("TURINGSERVE_B200_SINGLE", "1"))
 
-    def single_wins(self, step, KVH: int, streaming: bool) -> bool:
-        return self.single_mode == 2 or (self.single_mode == 1 and self.decode_kernel == "auto" and not streaming
+    def single_wins(self, step, KVH: int, barred: bool) -> bool:
+        """Whether plain single tokens go to that kernel; ``barred``: contexts too long for one cluster."""
+        # (up to one block a pair it is the faster one even with half of the SMs empty; 12 heads over 2 of 128 against the
+        # streaming kernel, us: 48 requests of 300 / 1,000 keys 5.7 / 8.7 and 12.8 / 16.1, 74 of them 7.1 / 10.1 and 15.2 / 19.2;
+        # 16 over 1, 100 of 300 keys 8.2 / 10.7)
+        return self.single_mode == 2 or (self.single_mode == 1 and self.decode_kernel == "auto" and not barred
                                          and step.num_decode * KVH <= self.num_sms)
 
     def _attention_single(self, out, q, k_cache, v_cache, block_tables, step, KVH: int, page_size: int, scale: float, softcap: float,
