@@ -131,3 +131,63 @@ def test_which_sizes_are_left_to_tcgen05(ops, M, N, K, taken):
     ops.linear(out, x, w)
     size = (x.double().abs() @ w.double().abs().T).clamp_min(1e-3)
     assert float(((out - x.double() @ w.double().T).abs() / size).max()) < 2e-5
+
+
+# (N, K): on both sides of the rule's lines, and whether the rule takes them at up to 8 and up to 16 tokens
+FRONT = [(1536, 1536, True, True), (896, 4864, True, True), (136, 200, True, True), (264, 18944, False, False), (2816, 7168, True, False),
+         (5120, 1536, True, True), (5120, 2048, True, False), (5120, 5120, False, False), (7168, 2048, True, False)]
+
+
+def put_off(ops, M, N, K, few, monkeypatch):
+    """(a product of few tokens not launched yet, its 64-bit value, the sum of magnitudes, whether few-token calls took it)."""
+    from turingserve_b200.kernels import LazyProduct
+    monkeypatch.setattr(ops, "few_tokens", few)
+    x, w, b = rnd(1, M, K), rnd(2, N, K, std=0.05), rnd(3, N)
+    p = ops.linear(torch.full((M, N), float("nan"), device=DEV).bfloat16(), x, w, b, may_defer=True)
+    assert isinstance(p, LazyProduct)
+    took, real = [], type(ops)._few
+    monkeypatch.setattr(type(ops), "_few", lambda self, *a: took.append(real(self, *a)) or took[-1])
+    return p, x.double() @ w.double().T + b.double(), x.double().abs() @ w.double().abs().T + b.double().abs(), took
+
+
+@pytest.mark.parametrize("few", [16, 0])
+@pytest.mark.parametrize("M", [1, 8, 9, 16])
+@pytest.mark.parametrize("N,K,to8,to16", FRONT)
+@pytest.mark.parametrize("form", ["norm", "layer_norm", "row", "row_layer_norm", "sum", "row_sum"])
+def test_norm_of_a_stream_that_gets_a_product(ops, monkeypatch, few, M, N, K, to8, to16, form):
+    """stream += product (rounded to bfloat16) + row, then its norm: the route by size, and either kernel's result against 64 bits."""
+    p, want, size, took = put_off(ops, M, N, K, few, monkeypatch)
+    old = torch.randn(M, N, device=DEV) * 3
+    row = torch.randn(N, device=DEV) if "row" in form else None
+    weight, bias = torch.rand(N, device=DEV) + 0.5, torch.randn(N, device=DEV) if "layer_norm" in form else None
+    out = None if "sum" in form else torch.full((M, N), float("nan"), device=DEV).bfloat16()
+    stream = old.clone()
+    ops.rmsnorm_stream(out, stream, p, None, weight, 1e-6, row=row, norm_bias=bias)
+    fused = [few > 0 and (to8 if M <= 8 else to16)]
+    assert any(took) == fused[0]
+    total = old.double() + want + (0 if row is None else row.double())
+    # (the product's rounding to bfloat16, its 32-bit sum, and two sums in 32 bits)
+    assert bool(((stream - total).abs() <= 2.0 ** -8 * want.abs() + 2e-5 * size + 2.0 ** -22 * (old.double().abs() + total.abs())).all())
+    if out is None:
+        return
+    s = stream.double()
+    mean = s.mean(-1, keepdim=True) if bias is not None else 0.0
+    y = (s - mean) / torch.sqrt((s - mean).pow(2).mean(-1, keepdim=True) + 1e-6) * weight.double() + (0.0 if bias is None else bias.double())
+    assert bool(((out.double() - y).abs() <= 2.0 ** -8 * y.abs() + 1e-5 * (weight * 4 + 1)).all())
+
+
+@pytest.mark.parametrize("few", [16, 0])
+@pytest.mark.parametrize("M", [1, 8, 9, 16])
+@pytest.mark.parametrize("N,K,to8,to16", FRONT)
+@pytest.mark.parametrize("kind", ["gelu_tanh", "relu2", "silu", "gelu"])
+def test_activation_that_gets_a_product(ops, monkeypatch, few, M, N, K, to8, to16, kind):
+    p, want, size, took = put_off(ops, M, N, K, few, monkeypatch)
+    ops.activation(p.out, p, kind)
+    assert any(took) == (few > 0 and (to8 if M <= 8 else to16))
+    act = {"gelu_tanh": lambda v: torch.nn.functional.gelu(v, approximate="tanh"), "relu2": lambda v: v.relu() ** 2,
+           "silu": torch.nn.functional.silu, "gelu": torch.nn.functional.gelu}[kind]
+    # what a difference of the product makes of the activation: its slope is at most 1.13, relu2's 2 |v|
+    off = 2.0 ** -8 * want.abs() + 2e-5 * size
+    slope = 2 * want.abs() + off if kind == "relu2" else 1.13
+    y = act(want)
+    assert bool(((p.out.double() - y).abs() <= 2.0 ** -8 * (y.abs() + slope * off) + slope * off + 1e-6).all())
