@@ -228,7 +228,7 @@ def timeline(a) -> None:
     step = sorted(evs[firsts[2]:firsts[3]], key=lambda e: e.time_range.end)
 
     def short(name: str) -> str:
-        m = re.search(r"(gemm_tc_kernel<[^>]*>|attention_\w+_kernel|reduce_rmsnorm_kernel|rope_kv_write\w*|rmsnorm\w*|"
+        m = re.search(r"(gemm_tc_kernel<[^>]*>|few_\w*kernel<[^>]*>|attention_\w+_kernel|reduce_rmsnorm_kernel|rope_kv_write\w*|rmsnorm\w*|"
                       r"silu_mul\w*|embedding_kernel|gather_rows_kernel|feed_tokens_kernel|sample\w*|splitk_reduce_kernel|"
                       r"Memcpy \w+|nvjet\w*)", name)
         return m.group(1) if m else name[:50]

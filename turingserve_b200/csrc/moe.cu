@@ -830,6 +830,16 @@ TS_API int ts_moe_gather(void* xs, const void* x, const int* order, const float*
 
 namespace {
 
+// The streaming kernel's warps read the same input rows over and over from L1, and it needs no shared memory.  Started while a
+// kernel with 100 KB and more of it still holds the SMs, it would run with what that one has left of L1 unless it says what it
+// prefers (8 tokens of width 3,584, 8 experts of 4,736 and top 4, behind few-token products and attention of single tokens, us:
+// gate/up 124 -> 84, down 77 -> 52; behind the products on tcgen05 they took 85 and 54).
+template <typename K> bool prefer_l1(K kernel) {
+  const bool ok = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxL1) == cudaSuccess;
+  if (!ok) cudaGetLastError();                                          // (a preference: it runs without, too)
+  return ok;
+}
+
 template <bool GLU>
 int launch_grouped(void* out, const void* x, const void* w, const int* order, const float* row_scale, const int* offsets,
                    const int* tiles, int P, int E, int top, int N, int K, int act, TsGlu glu, int dtype, int out_dtype,
@@ -838,6 +848,8 @@ int launch_grouped(void* out, const void* x, const void* w, const int* order, co
   if (grid.y > 65535) TS_REFUSE(TS_ERR_LIMIT, "ts_grouped_linear: %d rows too many for one launch", P);
   if (dtype == TS_BF16 && K % 8 == 0 && !(((uintptr_t)x | (uintptr_t)w) & 15) && P <= GV_STREAM_ROWS) {
     dim3 sgrid(ceil_div(N, GV_WARPS * 8), ceil_div(P, GL_BM) + E);
+    static const bool l1 = prefer_l1(grouped_linear_stream_kernel<bf16, GLU>) & prefer_l1(grouped_linear_stream_kernel<float, GLU>);
+    (void)l1;
     if (out_dtype == TS_BF16)
       ts_launch(grouped_linear_stream_kernel<bf16, GLU>, dim3(sgrid), dim3(GV_WARPS * 32), 0, s, (bf16*)out, (const bf16*)x,
                 (const bf16*)w, order, row_scale, offsets, tiles, top, N, K, act, glu);
