@@ -25,7 +25,9 @@
 // S of the tile behind.
 //
 // What bounds it (clock stamps in the kernel): a tile's chain.  576: 36 + 8 products of 46 to 128 cycles a tile of 64 keys (64
-// rows of K give a product no fewer cycles than 128 would), 3,600 cycles a tile of about 4,300; 128: 2,900 cycles a tile of
+// rows of K give a product no fewer cycles than 128 would), 3,600 cycles from issue to completion of about 4,450 a tile (148
+// blocks, 592 tokens of 16 heads behind 2,048 and 6,144: 2.27 us a tile more; by its counter the tensor pipe is active for 2,300
+// of them), and some 20 us a launch for the blocks' start, masked tiles and end; 128: 2,900 cycles a tile of
 // 128 keys, of which the softmax is busy for 2,400.  Portion of 2,048 tokens, 12 heads (L2 flushed), against the mma.sync
 // kernel of attention_biased_mma.cu: latent rows 660 -> 164 us; 128 over 2 kv heads 149 -> 43 us, with cap and bias 174 ->
 // 59 us; 64 over 2: 115 -> 39 us.  512 tokens behind 3,000, 28 heads: latent 1,456 -> 266 us, 128 over 4: 254 -> 61 us.

@@ -17,7 +17,8 @@
 // Measured (captured, keys from DRAM, us a launch; against the kernels that took these calls before): 12 heads over 2 of 128,
 // 8 requests of 300 / 1,000 / 2,048 / 6,000 keys 4.0 / 5.8 / 7.6 / 13.3, before 6.6 / 8.6 / 10.5 / 18.4; 1 request of 2,048
 // 5.0 / 8.6; 32 requests of 2,048 14.3 / 17.0; 14 heads over 2 of 64, 1 request of 1,000 3.2 / 5.7; with cap, bias and window
-// of 1,024, 8 requests 6.4 / 14.9; latent rows: see below.
+// of 1,024, 8 requests 6.4 / 14.9; latent rows: see below.  Not `early`: 0.2 to 1.5 us more (capped, 8 x 2,048 6.6 -> 7.6;
+// latent 16.3 -> 17.6).
 #include "common.cuh"
 #include "mma_utils.cuh"
 

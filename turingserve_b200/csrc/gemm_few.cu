@@ -2,9 +2,10 @@
 //   out[M, N] = x[M, K] . w[N, K]^T (+ bias[N])          (turingserve/ops/reference.py:45-47)
 // The reference leaves them to cuBLAS (turingserve/ops/triton_ops.py:74-76).
 //
-// A step is a chain of such products, each bound by the weights' bytes or, where those are few, by its latency.  So
-// the weights go from global memory straight into the registers that mma.sync (m16n8k16) reads them from: no shared
-// memory, barrier or tensor memory on their way, and the first of them are fetched before the wait for the kernel
+// A step is a chain of such products, each bound by the weights' bytes or, where those are few, by its latency.  So every
+// lane fetches the 16 bytes of weights that it hands to mma.sync (m16n8k16) itself: no layout change, block-wide barrier or
+// tensor memory on their way, and none of shared memory either where a warp's share fits its registers (plans 1 and 2; the
+// others pass them through a ring of the lane's own).  The first of them are fetched before the wait for the kernel
 // before.  The tokens are the product's 16 rows, eight weight rows its columns.  A lane's 16 bytes of weight row
 // lane / 4 are eight neighbouring columns of K, which stand for columns 2t, 2t+1, 2t+8, 2t+9 of two products; the
 // same permutation on the tokens' side leaves the sum as it is.
