@@ -191,3 +191,23 @@ def test_activation_that_gets_a_product(ops, monkeypatch, few, M, N, K, to8, to1
     slope = 2 * want.abs() + off if kind == "relu2" else 1.13
     y = act(want)
     assert bool(((p.out.double() - y).abs() <= 2.0 ** -8 * (y.abs() + slope * off) + slope * off + 1e-6).all())
+
+
+@pytest.mark.parametrize("plan", PLANS)
+def test_tokens_bias_and_residual_are_read_after_the_kernels_before(ops, monkeypatch, plan):
+    """What kernels of the same chain have just written (behind one that runs a while) is what counts; the weights alone are fetched early."""
+    M, N, K = 8, 2048, 1024
+    monkeypatch.setattr(ops, "few_plan", plan)
+    w, new = rnd(1, N, K, std=0.05), [rnd(2, M, K), rnd(3, 1, N), rnd(4, M, N)]
+    long_x, long_w, long_out = (torch.zeros(*s, device=DEV).bfloat16() for s in ((64, 4096), (16384, 4096), (64, 16384)))
+    rows = torch.arange(M, device=DEV).int()
+    half = (new[0].double() @ w.double().T + new[1].double()).float().bfloat16().float()
+    for _ in range(10):
+        x, b, resid = (torch.zeros_like(t) for t in new)
+        torch.cuda.synchronize()
+        ops.linear(long_out, long_x, long_w)
+        for to, t in zip((x, b, resid), new):
+            ops.gather_rows(to, t, rows[: t.shape[0]])
+        assert ops._few(resid, x, w, b.view(-1), M, N, K, ops.FEW_RESID)
+        err = (resid.float() - half - new[2].float()).abs()
+        assert bool((err <= 2.0 ** -7 * (half.abs() + new[2].float().abs()) + 1e-3).all())
